@@ -120,8 +120,9 @@ mcg_status mcg_destroy(mcg_context *ctx) {
     cudaFree(ctx->icp_pose);
     cudaFree(ctx->icp_inlier);
     cudaFree(ctx->depth_scaled);
-    cudaFree(ctx->integ_rows);
-    cudaFree(ctx->integ_zmax);
+    cudaFree(ctx->integ_blocks);
+    cudaFree(ctx->integ_tiles);
+    cudaFree(ctx->integ_count);
     for (const auto &r : ctx->ray_x) cudaFree(r.d);
     cudaFree(ctx->tr_text);
     cudaFree(ctx->tr_tok);

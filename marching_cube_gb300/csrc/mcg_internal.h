@@ -187,10 +187,12 @@ struct mcg_context {
     // integrate scratch
     float *depth_scaled = nullptr;
     size_t depth_scaled_cap = 0;
-    int2 *integ_rows = nullptr;  // per voxel row: the candidate x interval of the frame
-    size_t integ_rows_cap = 0;
-    unsigned int *integ_zmax = nullptr;  // the frame's largest ray-length depth (float bits)
-    size_t integ_zmax_cap = 0;
+    unsigned int *integ_blocks = nullptr;  // blocks of 8^3 voxels that the frame can update
+    size_t integ_blocks_cap = 0;
+    float *integ_tiles = nullptr;  // largest valid ray-length depth per tile of pixels
+    size_t integ_tiles_cap = 0;
+    unsigned int *integ_count = nullptr;  // blocks listed
+    size_t integ_count_cap = 0;
     // x coordinates of the voxel centres as the reference accumulates them
     // (p.x += grid_s per voxel), one device table per (nx, grid_s) seen on
     // this context, built once and never rewritten, so the calls on several

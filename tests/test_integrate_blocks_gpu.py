@@ -1,0 +1,60 @@
+"""Integrate's block list (blocks of 8^3 voxels that the frame can update)
+at the sizes where it can go wrong: volumes with ragged blocks, images
+with ragged depth tiles and images too small to hold a pixel, every option,
+the pose on the host and on the device.  The oracle tests every voxel, so
+the volumes have to be equal bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _look_at(eye, at):
+    f = (at - eye) / np.linalg.norm(at - eye)
+    r = np.cross([0.0, 1.0, 0.1], f)
+    r /= np.linalg.norm(r)
+    return np.stack([r, np.cross(f, r), f], axis=1)
+
+
+@pytest.mark.parametrize("vtype", [torch.int16, torch.float32])
+@pytest.mark.parametrize("dims,image", [((8, 8, 8), (64, 48)), ((9, 7, 17), (33, 25)), ((41, 30, 23), (47, 31)),
+                                        ((36, 24, 40), (16, 8)), ((20, 20, 20), (2, 40)), ((20, 20, 20), (3, 3))])
+def test_blocks_keep_every_update(mcg, orc, dims, image, vtype):
+    rng = np.random.default_rng(sum(dims) + image[0])
+    (nx, ny, nz), (w, h) = dims, image
+    gs = 1.0 / max(dims)
+    trunc = 2.5 * gs
+    f = 0.9 * w
+    k, ko = mcg.intrinsic(f, f, (w - 1) / 2.0, (h - 1) / 2.0), orc.intrinsic(f, f, (w - 1) / 2.0, (h - 1) / 2.0)
+    v = mcg.voxel_new(dims, trunc, trunc, gs, dtype=vtype)
+    ref = v.data.cpu().numpy().copy()
+    middle = np.array(dims) * gs / 2
+    for i in range(8):
+        # outside, inside, and next to a face of the volume
+        eye = middle + rng.uniform(-1, 1, 3) * (1.2, 0.3, 0.55)[i % 3]
+        R = _look_at(eye, middle + rng.uniform(-0.2, 0.2, 3))
+        m = rng.uniform(0.1, 1.6, (h, w)).astype(np.float32)
+        m[rng.random((h, w)) < 0.3] = 0.0
+        if i == 7:
+            m[0, 0], m[h // 2, w // 2] = np.inf, np.nan
+        n = rng.standard_normal((h, w, 3)).astype(np.float32)
+        n[..., 2] = -np.abs(n[..., 2]) - 0.5
+        n /= np.linalg.norm(n, axis=-1, keepdims=True)
+        n = n if i % 2 else None
+        nd = None if n is None else torch.from_numpy(n).cuda()
+        if i % 4 < 2:
+            mcg.volumetric_integration(v, k, mcg.extrinsic(R, eye), torch.from_numpy(m).cuda(), nd, is_dynamic=i > 3)
+        else:
+            mcg.volumetric_integration_device_pose(v, k, mcg.extrinsic_tensor(R, eye), torch.from_numpy(m).cuda(), nd,
+                                                   is_dynamic=i > 3)
+        orc.integrate(ref, trunc, trunc, gs, ko, orc.extrinsic(R, eye), m, n, is_dynamic=i > 3)
+    got = v.data.cpu().numpy()
+    # an infinite depth has weight 0 and gives an empty float voxel 0 / 0,
+    # a NaN whose bits no arithmetic fixes; everything else is equal in bits
+    none = np.isnan(ref) if vtype == torch.float32 else np.zeros(ref.shape, bool)
+    assert np.array_equal(np.isnan(got) if vtype == torch.float32 else none, none)
+    bits = np.uint32 if vtype == torch.float32 else np.uint16
+    assert np.array_equal(got.view(bits)[~none], ref.view(bits)[~none])
+    if w > 2:
+        assert (ref[..., 1] != 0).any()
