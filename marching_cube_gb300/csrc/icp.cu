@@ -4,21 +4,15 @@
 // The reference runs, per ICP iteration, a correspondence kernel, a kernel
 // writing the 6 columns of A and b, then 27 pairs of nppsMul_32f +
 // thrust::inclusive_scan for the normal equations, copies them to the host
-// and solves there.  Here one iteration is two launches on the stream and
-// no host round trip:
-//   icp_reduce  per pixel: the correspondence (nearest pixel, step 1, or
-//               bilinear, step 4), the row of A and b (step 2), the inlier
-//               flag (step 3); the 27 products A_i A_j and A_i b are formed
-//               in binary32 as nppsMul_32f forms them and summed in binary64
-//               per CTA (fixed order);
-//   icp_solve   one warp: the per-CTA sums in a fixed order, then Cholesky,
-//               the determinant and 1-norm condition tests, the increment,
-//               its bounds, exp([w]x) (Rodrigues), compose and the stopping
-//               rule of kf.cu:1177-1262, and the loop state on the device.
-// All it_max iterations are enqueued at once; once the loop has ended the
-// remaining launches return at their first instruction.  The host reads the
-// loop state once, after the last launch.  Per-pixel arithmetic is the
-// reference's binary32 in source order (--fmad=false).
+// and solves there.  Here one cooperative launch (icp_loop) runs all
+// iterations of a level: per pixel the correspondence (nearest pixel, step 1,
+// or bilinear, step 4), the row of A and b (step 2) and the inlier flag (step
+// 3); the 27 products A_i A_j and A_i b are formed in binary32 as nppsMul_32f
+// forms them and summed in binary64 in a fixed order; then Cholesky, the
+// determinant and 1-norm condition tests, the increment, its bounds, exp([w]x)
+// (Rodrigues), compose and the stopping rule of kf.cu:1177-1262.  The host
+// reads the outcome once.  Per-pixel arithmetic is the reference's binary32 in
+// source order (--fmad=false).
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -31,13 +25,13 @@ namespace {
 
 constexpr int IC_THREADS = 256;
 
+// the outcome of a loop
 struct IcpState {
     float r[9], t[3];  // pose_rel: rotation column-major, translation
-    double md;         // mahalanobis distance of the last step
-    int it;            // iterations left (the reference's `it`)
-    int rt;            // result so far
-    int done;          // the loop has ended
+    int rt;            // succeeded
     int iters;         // iterations run
+    int late;          // a wait at the grid barrier ran out
+    unsigned int arrived;  // the barrier's counter
 };
 
 struct IcpArgs {
@@ -154,167 +148,299 @@ __global__ void __launch_bounds__(IC_THREADS) icp_correspond_kernel(IcpArgs a, c
     }
 }
 
-// the 27 sums of one iteration: 21 of A_i A_j (i <= j, row-major upper
-// triangle), 6 of A_i b
-template <bool BILINEAR>
-__global__ void __launch_bounds__(IC_THREADS) icp_reduce(IcpArgs a, const IcpState *__restrict__ st,
-                                                         double *__restrict__ partial, uint8_t *__restrict__ inl) {
-    __shared__ double s_red[IC_THREADS / 32][27];
-    __shared__ float s_pose[12];
-    if (st->done) return;
-    if (threadIdx.x < 12) s_pose[threadIdx.x] = threadIdx.x < 9 ? st->r[threadIdx.x] : st->t[threadIdx.x - 9];
-    __syncthreads();
-    double acc[27];
-#pragma unroll
-    for (int k = 0; k < 27; ++k) acc[k] = 0.0;
-    const long long n = (long long)a.w1 * a.h1;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-         idx += (long long)gridDim.x * blockDim.x) {
-        float3 p1, m1, o;
-        const bool found = ic_match<BILINEAR>(a, s_pose, s_pose + 9, idx, &p1, &m1, &o);
-        if (inl) inl[idx] = found ? 0xff : 0;
-        if (found) {
-            float row[6], b;
-            ic_row(p1, m1, o, row, &b);
-            int k = 0;
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-#pragma unroll
-                for (int j = i; j < 6; ++j) acc[k++] += (double)(row[i] * row[j]);
-            }
-#pragma unroll
-            for (int i = 0; i < 6; ++i) acc[21 + i] += (double)(row[i] * b);
-        }
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 27; ++k) {
-        double v = acc[k];
-#pragma unroll
-        for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_down_sync(0xffffffffu, v, o2);
-        if (lane == 0) s_red[wid][k] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 27) {
-        double v = 0.0;
-        for (int w = 0; w < IC_THREADS / 32; ++w) v += s_red[w][threadIdx.x];
-        partial[(long long)blockIdx.x * 27 + threadIdx.x] = v;
-    }
+// ---- the loop ------------------------------------------------------------------
+// One cooperative launch runs a level's whole loop.  Per iteration every CTA
+// adds up the products of its pixels (27 sums: 21 of A_i A_j, i <= j, row-major
+// upper triangle, 6 of A_i b; the products in binary32 as nppsMul_32f forms
+// them, the sums in binary64) and stores them, one grid barrier makes them
+// visible, and every CTA then adds the CTAs' sums in the same order and solves
+// for itself, so that no second barrier has to bring the pose back.  Partial
+// sums alternate between two buffers: a CTA can be at most one barrier ahead
+// of another that still reads.
+//
+// What bounds it: the binary64 units (two sums a clock and SM).  A warp
+// reduces its 27 sums by halving (each step a lane keeps half of the values
+// and adds the other lane's: 31 sums and shuffles, against 135 for a tree per
+// value), the solve spreads over lanes (rows of the factorisation, columns of
+// the inverse beside the right-hand side).  Before, an iteration was two
+// launches, the second one warp adding 304 CTAs' sums one after another and
+// one thread solving, 76 us; the launches after the loop's end cost 4 us each.
+// Tracking a 640x480 frame (pyramid, maps, three levels): 1286 -> 633 us, of
+// which the loops 810 -> 261 us.
+constexpr int IL_THREADS = 512;
+constexpr int IL_WARPS = IL_THREADS / 32;
+constexpr int IL_SUMS = 27;
+constexpr unsigned long long IL_LIMIT_NS = 2000000000ull;  // longest wait at the grid barrier
+
+struct IcpShared {
+    double red[IL_WARPS][32];
+    double sum[IL_SUMS];
+    double L[6][6];
+    double x[6], md, prev_md;
+    float pose[12];
+    float inc[12];
+    int it, rt, done, iters, late;
+};
+
+__device__ __forceinline__ unsigned long long ic_now() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
 }
 
-// Cholesky solve with the reference's tests; returns false to stop the loop
-__device__ bool ic_solve(const double *ata21, const double *atb, double *x, double *md) {
-    double M[6][6], L[6][6];
-    int k = 0, count = 0;
-    for (int i = 0; i < 6; ++i)
-        for (int j = i; j < 6; ++j) M[i][j] = M[j][i] = ata21[k++];
-    for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < i; ++j)
-            if (M[i][j] != 0.0) ++count;
-    if (count == 0) return false;  // empty
-    for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < 6; ++j) L[i][j] = 0.0;
-    for (int j = 0; j < 6; ++j) {
-        double d = M[j][j];
-        for (int p = 0; p < j; ++p) d -= L[j][p] * L[j][p];
-        if (!(d > 0.0)) return false;  // not positive definite
-        L[j][j] = sqrt(d);
-        for (int i = j + 1; i < 6; ++i) {
-            double s = M[i][j];
-            for (int p = 0; p < j; ++p) s -= L[i][p] * L[j][p];
-            L[i][j] = s / L[j][j];
+// all CTAs of the launch (one cooperative launch: they run together); false
+// when the wait ran out
+__device__ __forceinline__ bool ic_grid_barrier(IcpShared &S, unsigned int *arrived, unsigned int target) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        const unsigned long long t0 = ic_now();
+        for (;;) {
+            unsigned int v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+            if (v >= target) break;
+            if (ic_now() - t0 > IL_LIMIT_NS) {
+                S.late = 1;
+                break;
+            }
         }
     }
+    __syncthreads();
+    return S.late == 0;
+}
+
+// warp-wide sums of 32 values per lane: lane k returns the sum of value k
+__device__ __forceinline__ double ic_warp_sums(double (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < o; ++k) {
+            const double keep = up ? v[k + o] : v[k], send = up ? v[k] : v[k + o];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+// Cholesky solve with the reference's tests by one warp: lane i < 6 has row i
+// of the factor, then column i of the inverse, lane 6 the right-hand side.
+// Fills S.x and S.md; returns false (on every lane) to stop the loop.
+__device__ bool ic_solve(IcpShared &S) {
+    const unsigned int full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, i = min(lane, 5);
+    double M[6];  // row i of AtA
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const int lo = min(i, j), hi = max(i, j);
+        M[j] = S.sum[lo * 6 - lo * (lo - 1) / 2 + hi - lo];
+    }
+    bool off = false;
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+        if (j < i && M[j] != 0.0) off = true;
+    if (!__any_sync(full, off)) return false;  // empty
     double det = 1.0;
-    for (int i = 0; i < 6; ++i) det *= L[i][i] * L[i][i];
-    if (!(fabs(det) > 1e-15)) return false;  // null space
-    double anorm = 0.0, inorm = 0.0;
+#pragma unroll
     for (int j = 0; j < 6; ++j) {
-        double c = 0.0;
-        for (int i = 0; i < 6; ++i) c += fabs(M[i][j]);
-        anorm = c > anorm ? c : anorm;
+        double s = M[j];
+        for (int p = 0; p < j; ++p) s -= S.L[i][p] * S.L[j][p];
+        const double d = __shfl_sync(full, s, j);
+        if (!(d > 0.0)) return false;  // not positive definite
+        const double l = sqrt(d);
+        __syncwarp();
+        if (lane < 6) S.L[lane][j] = lane > j ? s / l : lane == j ? l : 0.0;
+        __syncwarp();
+        det *= l * l;
     }
-    for (int j = 0; j < 6; ++j) {  // column j of the inverse
-        double y[6], z[6];
-        for (int i = 0; i < 6; ++i) {
-            double s = i == j ? 1.0 : 0.0;
-            for (int p = 0; p < i; ++p) s -= L[i][p] * y[p];
-            y[i] = s / L[i][i];
+    if (!(fabs(det) > 1e-15)) return false;  // null space
+    double anorm = 0.0;  // column i of AtA (symmetric: row i)
+#pragma unroll
+    for (int j = 0; j < 6; ++j) anorm += fabs(M[j]);
+    double y[6], z[6];
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+        double s = lane == 6 ? S.sum[21 + r] : (r == lane ? 1.0 : 0.0);
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+            if (p < r) s -= S.L[r][p] * y[p];
+        y[r] = s / S.L[r][r];
+    }
+#pragma unroll
+    for (int r = 5; r >= 0; --r) {
+        double s = y[r];
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+            if (p > r) s -= S.L[p][r] * z[p];
+        z[r] = s / S.L[r][r];
+    }
+    double inorm = 0.0;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) inorm += fabs(z[r]);
+    if (lane == 6) inorm = 0.0;
+    double a = anorm, b = inorm;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        a = fmax(a, __shfl_xor_sync(full, a, o));
+        b = fmax(b, __shfl_xor_sync(full, b, o));
+    }
+    a = __shfl_sync(full, a, 0);  // the maximum over lanes 0 .. 7 (6 and 7 repeat row 5 of AtA)
+    b = __shfl_sync(full, lane < 8 ? b : 0.0, 0);
+    if (!(1.0 / (a * b) > 5e-5)) return false;  // ill-conditioned
+    if (lane == 6) {
+        double m = 0.0;
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+            S.x[r] = z[r];
+            m += S.sum[21 + r] * z[r];
         }
-        for (int i = 5; i >= 0; --i) {
-            double s = y[i];
-            for (int p = i + 1; p < 6; ++p) s -= L[p][i] * z[p];
-            z[i] = s / L[i][i];
-        }
-        double c = 0.0;
-        for (int i = 0; i < 6; ++i) c += fabs(z[i]);
-        inorm = c > inorm ? c : inorm;
+        S.md = m;
     }
-    if (!(1.0 / (anorm * inorm) > 5e-5)) return false;  // ill-conditioned
-    double y[6];
-    for (int i = 0; i < 6; ++i) {
-        double s = atb[i];
-        for (int p = 0; p < i; ++p) s -= L[i][p] * y[p];
-        y[i] = s / L[i][i];
-    }
-    for (int i = 5; i >= 0; --i) {
-        double s = y[i];
-        for (int p = i + 1; p < 6; ++p) s -= L[p][i] * x[p];
-        x[i] = s / L[i][i];
-    }
-    double m = 0.0;
-    for (int i = 0; i < 6; ++i) m += atb[i] * x[i];
-    *md = m;
+    __syncwarp();
     return true;
 }
 
-__global__ void icp_solve(IcpState *__restrict__ st, const double *__restrict__ partial, int nblocks, float rtb,
-                          float ttb) {
-    __shared__ double s_sum[27];
-    if (st->done) return;
-    if (threadIdx.x < 27) {
-        double v = 0.0;
-        for (int b = 0; b < nblocks; ++b) v += partial[(long long)b * 27 + threadIdx.x];
-        s_sum[threadIdx.x] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    st->iters += 1;
-    double x[6], md = 0.0;
-    bool rt = ic_solve(s_sum, s_sum + 21, x, &md);
+// one step of the loop after the sums, by warp 0: the increment, its bounds,
+// exp([w]x) by Rodrigues' formula, compose, the stopping rule (kf.cu:1177-1262)
+__device__ void ic_step(IcpShared &S, float rtb, float ttb) {
+    const int lane = threadIdx.x & 31;
+    bool rt = ic_solve(S);
     if (rt) {
-        if (fabs(x[0]) > rtb || fabs(x[1]) > rtb || fabs(x[2]) > rtb || fabs(x[3]) > ttb || fabs(x[4]) > ttb ||
-            fabs(x[5]) > ttb) {
+        const double x0 = S.x[0], x1 = S.x[1], x2 = S.x[2];
+        if (fabs(x0) > rtb || fabs(x1) > rtb || fabs(x2) > rtb || fabs(S.x[3]) > ttb || fabs(S.x[4]) > ttb ||
+            fabs(S.x[5]) > ttb) {
             rt = false;  // out of bound
         } else {
-            // exp([w]x) by Rodrigues' formula, column-major
-            const double th2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2], th = sqrt(th2);
+            const double th2 = x0 * x0 + x1 * x1 + x2 * x2, th = sqrt(th2);
             const double ca = th < 1e-12 ? 1.0 : sin(th) / th, cb = th < 1e-12 ? 0.5 : (1.0 - cos(th)) / th2;
-            const double K[3][3] = {{0.0, -x[2], x[1]}, {x[2], 0.0, -x[0]}, {-x[1], x[0], 0.0}};
-            float ri[9];
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r) {
-                    double kk = 0.0;
-                    for (int p = 0; p < 3; ++p) kk += K[r][p] * K[p][c];
-                    ri[3 * c + r] = (float)((r == c ? 1.0 : 0.0) + ca * K[r][c] + cb * kk);
+            const int c = min(lane / 3, 2), r = lane % 3;
+            if (lane < 9) {
+                const double K[3][3] = {{0.0, -x2, x1}, {x2, 0.0, -x0}, {-x1, x0, 0.0}};
+                double kk = 0.0, kr = 0.0;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const double krp = r == 0 ? K[0][p] : r == 1 ? K[1][p] : K[2][p];
+                    const double kpc = c == 0 ? K[p][0] : c == 1 ? K[p][1] : K[p][2];
+                    kk += krp * kpc;
+                    if (p == c) kr = krp;
                 }
-            const float ti[3] = {(float)x[3], (float)x[4], (float)x[5]};
+                S.inc[lane] = (float)((r == c ? 1.0 : 0.0) + ca * kr + cb * kk);  // column-major
+            } else if (lane < 12) {
+                S.inc[lane] = (float)S.x[lane - 6];
+            }
+            __syncwarp();
             // float_camera_extrinsic_compose(pose, inc): R = Ri R, t = Ri t + ti (binary32)
-            float nr[9], nt[3];
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 3; ++r)
-                    nr[3 * c + r] = ri[r] * st->r[3 * c] + ri[3 + r] * st->r[3 * c + 1] + ri[6 + r] * st->r[3 * c + 2];
-            for (int r = 0; r < 3; ++r) nt[r] = ri[r] * st->t[0] + ri[3 + r] * st->t[1] + ri[6 + r] * st->t[2];
-            for (int r = 0; r < 3; ++r) nt[r] = nt[r] + ti[r];
-            for (int i = 0; i < 9; ++i) st->r[i] = nr[i];
-            for (int i = 0; i < 3; ++i) st->t[i] = nt[i];
-            if (md > st->md || md < 1e-5) st->it = 1;
-            st->md = md;
+            float v = 0.0f;
+            if (lane < 9)
+                v = S.inc[r] * S.pose[3 * c] + S.inc[3 + r] * S.pose[3 * c + 1] + S.inc[6 + r] * S.pose[3 * c + 2];
+            else if (lane < 12)
+                v = S.inc[r] * S.pose[9] + S.inc[3 + r] * S.pose[10] + S.inc[6 + r] * S.pose[11] + S.inc[lane];
+            __syncwarp();
+            if (lane < 12) S.pose[lane] = v;
         }
     }
-    st->rt = rt ? 1 : 0;
-    st->it -= 1;
-    if (st->it == 0 || !rt) st->done = 1;
+    __syncwarp();
+    if (lane == 0) {
+        S.iters += 1;
+        if (rt) {
+            const double md = S.md;
+            if (md > S.prev_md || md < 1e-5) S.it = 1;
+            S.prev_md = md;
+        }
+        S.rt = rt ? 1 : 0;
+        S.it -= 1;
+        S.done = S.it == 0 || !rt;
+    }
+}
+
+struct IcpInit {
+    float pose[12];
+    int it_max;
+    float rt, tt;
+};
+
+template <bool BILINEAR>
+__global__ void __launch_bounds__(IL_THREADS, 1)
+    icp_loop(IcpArgs a, IcpInit in, IcpState *__restrict__ st, double *partial, unsigned int *arrived,
+             uint8_t *__restrict__ flags, uint8_t *__restrict__ inl) {
+    __shared__ IcpShared S;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = (int)gridDim.x;
+    if (tid < 12) S.pose[tid] = in.pose[tid];
+    if (tid == 0) {
+        S.it = in.it_max;
+        S.rt = 1;
+        S.done = S.iters = S.late = 0;
+        S.prev_md = (double)FLT_MAX;
+    }
+    __syncthreads();
+    const long long n = (long long)a.w1 * a.h1;
+    for (int pass = 0;; ++pass) {
+        double acc[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) acc[k] = 0.0;
+        for (long long idx = (long long)blockIdx.x * IL_THREADS + tid; idx < n; idx += (long long)G * IL_THREADS) {
+            float3 p1, m1, o;
+            const bool found = ic_match<BILINEAR>(a, S.pose, S.pose + 9, idx, &p1, &m1, &o);
+            if (flags) flags[idx] = found ? 0xff : 0;
+            if (found) {
+                float row[6], b;
+                ic_row(p1, m1, o, row, &b);
+                int k = 0;
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+#pragma unroll
+                    for (int j = i; j < 6; ++j) acc[k++] += (double)(row[i] * row[j]);
+                }
+#pragma unroll
+                for (int i = 0; i < 6; ++i) acc[21 + i] += (double)(row[i] * b);
+            }
+        }
+        S.red[warp][lane] = ic_warp_sums(acc);
+        __syncthreads();
+        double *buf = partial + (long long)(pass & 1) * G * IL_SUMS;
+        if (tid < IL_SUMS) {
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < IL_WARPS; ++w) v += S.red[w][tid];
+            __stcg(buf + (long long)blockIdx.x * IL_SUMS + tid, v);
+        }
+        if (!ic_grid_barrier(S, arrived, (unsigned int)(pass + 1) * (unsigned int)G)) break;
+        // warp w adds the sums of CTAs w, w + IL_WARPS, ...; then the warps' in order
+        if (lane < IL_SUMS) {
+            double v = 0.0;
+            for (int c = warp; c < G; c += IL_WARPS) v += __ldcg(buf + (long long)c * IL_SUMS + lane);
+            S.red[warp][lane] = v;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (lane < IL_SUMS) {
+                double v = 0.0;
+#pragma unroll
+                for (int w = 0; w < IL_WARPS; ++w) v += S.red[w][lane];
+                S.sum[lane] = v;
+            }
+            __syncwarp();
+            ic_step(S, in.rt, in.tt);
+        }
+        __syncthreads();
+        if (S.done) break;
+    }
+    // the caller's map receives the last pass's flags only when the loop
+    // succeeds (kf.cu:1285-1292); each thread copies what it wrote
+    if (inl && S.rt && !S.late)
+        for (long long idx = (long long)blockIdx.x * IL_THREADS + tid; idx < n; idx += (long long)G * IL_THREADS)
+            inl[idx] = flags[idx];
+    if (tid == 0 && S.late) st->late = 1;
+    if (blockIdx.x == 0) {
+        if (tid < 12) (tid < 9 ? st->r[tid] : st->t[tid - 9]) = S.pose[tid];
+        if (tid == 0) {
+            st->rt = S.rt;
+            st->iters = S.iters;
+        }
+    }
 }
 
 // kf.cu:226-261
@@ -452,9 +578,11 @@ extern "C" mcg_status mcg_icp(mcg_context *ctx, const mcg_icp_params *p, const m
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     const cudaStream_t s = (cudaStream_t)stream;
-    const int nblocks = ctx->num_sms * 2;
+    const long long npx = (long long)w1 * h1;
+    // one CTA per SM at most: the launch is cooperative and its CTAs wait for each other
+    int G = (int)std::min<long long>((npx + IL_THREADS - 1) / IL_THREADS, (long long)ctx->num_sms);
     if (!ensure(&ctx->icp_state, &ctx->icp_state_cap, sizeof(IcpState)) ||
-        !ensure(&ctx->icp_partial, &ctx->icp_partial_cap, (size_t)nblocks * 27))
+        !ensure(&ctx->icp_partial, &ctx->icp_partial_cap, (size_t)2 * ctx->num_sms * IL_SUMS))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     if (!ctx->h_icp_state && cudaMallocHost((void **)&ctx->h_icp_state, sizeof(IcpState)) != cudaSuccess) {
         ctx->h_icp_state = nullptr;
@@ -462,43 +590,33 @@ extern "C" mcg_status mcg_icp(mcg_context *ctx, const mcg_icp_params *p, const m
     }
     IcpState *hs = reinterpret_cast<IcpState *>(ctx->h_icp_state);
     IcpState *ds = reinterpret_cast<IcpState *>(ctx->icp_state);
-    for (int i = 0; i < 9; ++i) hs->r[i] = pose_rel->r[i];
-    for (int i = 0; i < 3; ++i) hs->t[i] = pose_rel->t[i];
-    hs->md = (double)FLT_MAX;
-    hs->it = p->it_max;
-    hs->rt = 1;
-    hs->done = 0;
-    hs->iters = 0;
-    if ((e = cudaMemcpyAsync(ds, hs, sizeof(IcpState), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return mcg_cuda_fail(ctx, e);
-    // the flags of every pass go to scratch; the caller's map receives the
-    // last pass's flags only when the loop succeeds (kf.cu:1285-1292)
-    const long long npx = (long long)w1 * h1;
+    IcpInit in;
+    for (int i = 0; i < 9; ++i) in.pose[i] = pose_rel->r[i];
+    for (int i = 0; i < 3; ++i) in.pose[9 + i] = pose_rel->t[i];
+    in.it_max = p->it_max;
+    in.rt = p->rt;
+    in.tt = p->tt;
+    if ((e = cudaMemsetAsync(ds, 0, sizeof(IcpState), s)) != cudaSuccess) return mcg_cuda_fail(ctx, e);
     uint8_t *flags = nullptr;
     if (inlier) {
         if (!ensure(&ctx->icp_inlier, &ctx->icp_inlier_cap, (size_t)npx))
             return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
         flags = ctx->icp_inlier;
     }
-    const IcpArgs a = make_args(p, k2, w1, h1, w2, h2, v1, n1, v2, n2);
-    for (int it = 0; it < p->it_max; ++it) {
-        if (p->bilinear)
-            icp_reduce<true><<<nblocks, IC_THREADS, 0, s>>>(a, ds, ctx->icp_partial, flags);
-        else
-            icp_reduce<false><<<nblocks, IC_THREADS, 0, s>>>(a, ds, ctx->icp_partial, flags);
-        icp_solve<<<1, 32, 0, s>>>(ds, ctx->icp_partial, nblocks, p->rt, p->tt);
-    }
-    if ((e = cudaGetLastError()) != cudaSuccess ||
+    IcpArgs a = make_args(p, k2, w1, h1, w2, h2, v1, n1, v2, n2);
+    unsigned int *arrived = &ds->arrived;
+    void *args[] = {&a, &in, &ds, &ctx->icp_partial, &arrived, &flags, &inlier};
+    const void *fn = p->bilinear ? (const void *)icp_loop<true> : (const void *)icp_loop<false>;
+    if ((e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(IL_THREADS), args, 0, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(hs, ds, sizeof(IcpState), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return mcg_cuda_fail(ctx, e);
+    if (hs->late) return MCG_ERR_TIMEOUT;
     *ok = hs->rt;
     if (iterations) *iterations = hs->iters;
     if (hs->rt) {
         for (int i = 0; i < 9; ++i) pose_rel->r[i] = hs->r[i];
         for (int i = 0; i < 3; ++i) pose_rel->t[i] = hs->t[i];
-        if (inlier && (e = cudaMemcpyAsync(inlier, flags, (size_t)npx, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-            return mcg_cuda_fail(ctx, e);
     }
     return MCG_OK;
 }
