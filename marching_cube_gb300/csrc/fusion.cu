@@ -387,9 +387,15 @@ __device__ __forceinline__ bool integ_block_kept(const IntegParams &p, int x0, i
     const int pu0 = (int)fmaxf(floorf(u0 - mu), 0.0f), pu1 = (int)fminf(ceilf(u1 + mu), (float)(p.w - 3));
     const int pv0 = (int)fmaxf(floorf(v0 - mv), 0.0f), pv1 = (int)fminf(ceilf(v1 + mv), (float)(p.h - 3));
     if (pu1 < pu0 || pv1 < pv0) return false;
+    // a block close to the camera covers up to the whole image, and nearly
+    // all of those hold updates: not searched (the one thread's search of some
+    // hundred tiles was most of this launch, 27 us at 512^3)
+    const int tu0 = pu0 / TILE_W, tu1 = pu1 / TILE_W, tv0 = pv0 / TILE_H, tv1 = pv1 / TILE_H;
+    if ((tu1 - tu0 + 1) * (tv1 - tv0 + 1) > 64) return true;
     float zt = 0.0f;
-    for (int ty = pv0 / TILE_H; ty <= pv1 / TILE_H; ++ty)
-        for (int tx = pu0 / TILE_W; tx <= pu1 / TILE_W; ++tx) zt = fmaxf(zt, p.tiles[(long long)ty * p.tiles_x + tx]);
+    for (int ty = tv0; ty <= tv1; ++ty)
+#pragma unroll 4
+        for (int tx = tu0; tx <= tu1; ++tx) zt = fmaxf(zt, p.tiles[(long long)ty * p.tiles_x + tx]);
     if (zt == 0.0f) return false;  // no valid pixel
     const float near = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) - sqrtf(half);
     return !(near > zt + p.min_t + 1e-5f * (size + zt + p.min_t));
