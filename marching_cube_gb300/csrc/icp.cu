@@ -175,7 +175,6 @@ constexpr unsigned long long IL_LIMIT_NS = 2000000000ull;  // longest wait at th
 struct IcpShared {
     double red[IL_WARPS][32];
     double sum[IL_SUMS];
-    double L[6][6];
     double x[6], md, prev_md;
     float pose[12];
     float inc[12];
@@ -225,81 +224,96 @@ __device__ __forceinline__ double ic_warp_sums(double (&v)[32]) {
     return v[0];
 }
 
-// Cholesky solve with the reference's tests by one warp: lane i < 6 has row i
-// of the factor, then column i of the inverse, lane 6 the right-hand side.
+// Cholesky solve with the reference's tests by one warp.  A lane holds a row of
+// six values and the factorisation runs over the rows of AtA (lanes 0-5), the
+// right-hand side (lane 6) and the unit vectors (lanes 8-13) alike: what it
+// leaves in a row v is the solution of L y = v, so the forward substitutions
+// come with the factor.  The back substitutions then give the increment (lane
+// 6) and the columns of the inverse for the condition number.  Updates run
+// ahead (right-looking) and the diagonal enters as its reciprocal square root,
+// because a chain of dependent binary64 operations is what this takes: the
+// same solve by substitution with divisions took about 20 us, this 4.
 // Fills S.x and S.md; returns false (on every lane) to stop the loop.
 __device__ bool ic_solve(IcpShared &S) {
     const unsigned int full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, i = min(lane, 5);
-    double M[6];  // row i of AtA
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-        const int lo = min(i, j), hi = max(i, j);
-        M[j] = S.sum[lo * 6 - lo * (lo - 1) / 2 + hi - lo];
-    }
+    const int lane = threadIdx.x & 31;
+    double v[6], anorm = 0.0;
     bool off = false;
 #pragma unroll
-    for (int j = 0; j < 6; ++j)
-        if (j < i && M[j] != 0.0) off = true;
+    for (int j = 0; j < 6; ++j) {
+        v[j] = lane == 8 + j ? 1.0 : 0.0;
+        if (lane < 6) {
+            const int lo = min(lane, j), hi = max(lane, j);
+            v[j] = S.sum[lo * 6 - lo * (lo - 1) / 2 + hi - lo];
+            anorm += fabs(v[j]);  // column `lane` (AtA is symmetric)
+            if (j < lane && v[j] != 0.0) off = true;
+        }
+        if (lane == 6) v[j] = S.sum[21 + j];
+    }
     if (!__any_sync(full, off)) return false;  // empty
-    double det = 1.0;
+    double det = 1.0, rinv[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-        double s = M[j];
-        for (int p = 0; p < j; ++p) s -= S.L[i][p] * S.L[j][p];
-        const double d = __shfl_sync(full, s, j);
+        const double d = __shfl_sync(full, v[j], j);
         if (!(d > 0.0)) return false;  // not positive definite
-        const double l = sqrt(d);
-        __syncwarp();
-        if (lane < 6) S.L[lane][j] = lane > j ? s / l : lane == j ? l : 0.0;
-        __syncwarp();
-        det *= l * l;
+        rinv[j] = rsqrt(d);
+        v[j] *= rinv[j];
+        det *= d;
+#pragma unroll
+        for (int k = j + 1; k < 6; ++k) v[k] = fma(-v[j], __shfl_sync(full, v[j], k), v[k]);
     }
     if (!(fabs(det) > 1e-15)) return false;  // null space
-    double anorm = 0.0;  // column i of AtA (symmetric: row i)
+    double z[6], inorm = 0.0;
 #pragma unroll
-    for (int j = 0; j < 6; ++j) anorm += fabs(M[j]);
-    double y[6], z[6];
+    for (int r = 0; r < 6; ++r) z[r] = v[r];
 #pragma unroll
-    for (int r = 0; r < 6; ++r) {
-        double s = lane == 6 ? S.sum[21 + r] : (r == lane ? 1.0 : 0.0);
+    for (int p = 5; p >= 0; --p) {
+        z[p] *= rinv[p];
+        inorm += fabs(z[p]);
 #pragma unroll
-        for (int p = 0; p < 6; ++p)
-            if (p < r) s -= S.L[r][p] * y[p];
-        y[r] = s / S.L[r][r];
+        for (int r = 0; r < 6; ++r)
+            if (r < p) z[r] = fma(-__shfl_sync(full, v[r], p), z[p], z[r]);
     }
+    if (lane < 8 || lane > 13) inorm = 0.0;
 #pragma unroll
-    for (int r = 5; r >= 0; --r) {
-        double s = y[r];
-#pragma unroll
-        for (int p = 0; p < 6; ++p)
-            if (p > r) s -= S.L[p][r] * z[p];
-        z[r] = s / S.L[r][r];
+    for (int o = 16; o > 0; o >>= 1) {
+        anorm = fmax(anorm, __shfl_xor_sync(full, anorm, o));
+        inorm = fmax(inorm, __shfl_xor_sync(full, inorm, o));
     }
-    double inorm = 0.0;
-#pragma unroll
-    for (int r = 0; r < 6; ++r) inorm += fabs(z[r]);
-    if (lane == 6) inorm = 0.0;
-    double a = anorm, b = inorm;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-        a = fmax(a, __shfl_xor_sync(full, a, o));
-        b = fmax(b, __shfl_xor_sync(full, b, o));
-    }
-    a = __shfl_sync(full, a, 0);  // the maximum over lanes 0 .. 7 (6 and 7 repeat row 5 of AtA)
-    b = __shfl_sync(full, lane < 8 ? b : 0.0, 0);
-    if (!(1.0 / (a * b) > 5e-5)) return false;  // ill-conditioned
+    if (!(1.0 > 5e-5 * (anorm * inorm))) return false;  // ill-conditioned
     if (lane == 6) {
         double m = 0.0;
 #pragma unroll
         for (int r = 0; r < 6; ++r) {
             S.x[r] = z[r];
-            m += S.sum[21 + r] * z[r];
+            m = fma(S.sum[21 + r], z[r], m);
         }
         S.md = m;
     }
     __syncwarp();
     return true;
+}
+
+// sin(th) / th and (1 - cos(th)) / th^2 from th^2: their power series, to
+// 1e-19 below half a radian (th2^8 / 17!)
+__device__ __forceinline__ void ic_rodrigues(double th2, double &ca, double &cb) {
+    if (th2 < 0.25) {
+        double a = -1.0 / 1307674368000.0, b = -1.0 / 20922789888000.0;  // 1 / 15!, 1 / 16!
+        const double ka[7] = {1.0, 6.0, 120.0, 5040.0, 362880.0, 39916800.0, 6227020800.0};
+        const double kb[7] = {2.0, 24.0, 720.0, 40320.0, 3628800.0, 479001600.0, 87178291200.0};
+#pragma unroll
+        for (int k = 6; k >= 0; --k) {
+            const double sg = k & 1 ? -1.0 : 1.0;
+            a = fma(a, th2, sg / ka[k]);
+            b = fma(b, th2, sg / kb[k]);
+        }
+        ca = a;
+        cb = b;
+    } else {
+        const double th = sqrt(th2);
+        ca = sin(th) / th;
+        cb = (1.0 - cos(th)) / th2;
+    }
 }
 
 // one step of the loop after the sums, by warp 0: the increment, its bounds,
@@ -313,8 +327,8 @@ __device__ void ic_step(IcpShared &S, float rtb, float ttb) {
             fabs(S.x[5]) > ttb) {
             rt = false;  // out of bound
         } else {
-            const double th2 = x0 * x0 + x1 * x1 + x2 * x2, th = sqrt(th2);
-            const double ca = th < 1e-12 ? 1.0 : sin(th) / th, cb = th < 1e-12 ? 0.5 : (1.0 - cos(th)) / th2;
+            double ca, cb;
+            ic_rodrigues(x0 * x0 + x1 * x1 + x2 * x2, ca, cb);
             const int c = min(lane / 3, 2), r = lane % 3;
             if (lane < 9) {
                 const double K[3][3] = {{0.0, -x2, x1}, {x2, 0.0, -x0}, {-x1, x0, 0.0}};
