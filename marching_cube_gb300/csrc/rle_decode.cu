@@ -14,8 +14,8 @@
 //    state from the chunk before) gives every word its state;
 //  * a block scan of the run lengths of the headers places each run in the
 //    slice; runs go to shared memory as (start, voxel);
-//  * the chunk's voxels are written by all threads, coalesced, each voxel
-//    finding its run by binary search over the run starts.
+//  * the chunk's voxels are written by all threads, 16 bytes at a time, each
+//    voxel's run found by counting the run starts up to it.
 // The slice is full once its voxels are placed; records after that are
 // ignored.  A record that is needed and has length 0, runs past the slice
 // or lacks its literal, or a stream that ends early, is an error
@@ -275,6 +275,75 @@ __global__ void __launch_bounds__(RD_THREADS) rle_slice_scan(Dir d, int z0, long
     if (threadIdx.x == 0 && out < xy) atomicOr(err, 1);
 }
 
+// Voxels [out, end) of a slice from the chunk's runs (rs: starts counted from
+// `out`, rv: voxels, n of them), RD_TILE voxels at a time: a bit is set where a
+// run starts, the set bits before each 32-bit word are counted, and a voxel's
+// run is the number of bits up to its own.  Each lane writes four consecutive
+// voxels, 16 bytes.  Bound: the instructions of this, then writing the volume.
+// Expanding 512^3 voxels from 26 MB: a binary search over the chunk's runs for
+// each voxel took 967 us, for each four voxels between those of a warp's ends
+// 431 us; this 171 us.
+constexpr int RD_TILE = 16384;
+
+struct RunTile {
+    uint32_t start[RD_TILE / 32];  // bit: a run starts at this voxel
+    int before[RD_TILE / 32];      // runs that start before the word's first voxel
+    int w[RD_THREADS / 32];
+};
+
+__device__ __forceinline__ void rd_write_runs(RunTile &S, uint32_t *__restrict__ slice, long long out, long long end,
+                                              const int *rs, const uint32_t *rv, int n) {
+    constexpr int WPT = RD_TILE / 32 / RD_THREADS;  // words per thread
+    const int tid = threadIdx.x;
+    const int total = (int)(end - out);
+    // tiles start on 16-byte boundaries: the first one at or below `out`
+    const int lead = (int)((reinterpret_cast<uintptr_t>(slice + out) >> 2) & 3u);
+    int base = 0;  // runs that start before the tile
+    for (int t0 = -lead; t0 < total; t0 += RD_TILE) {
+        for (int i = tid; i < RD_TILE / 32; i += RD_THREADS) S.start[i] = 0u;
+        __syncthreads();
+        for (int r = tid; r < n; r += RD_THREADS) {
+            const unsigned int p = (unsigned int)(rs[r] - t0);
+            if (p < (unsigned int)RD_TILE) atomicOr(&S.start[p >> 5], 1u << (p & 31));
+        }
+        __syncthreads();
+        int c[WPT], sum = 0;
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) {
+            c[i] = sum;
+            sum += __popc(S.start[tid * WPT + i]);
+        }
+        int all;
+        const int ex = base + rd_block_scan<int>(sum, 0, [](int a, int b) { return a + b; }, S.w, &all);
+#pragma unroll
+        for (int i = 0; i < WPT; ++i) S.before[tid * WPT + i] = ex + c[i];
+        base += all;
+        __syncthreads();
+        const int stop = min(RD_TILE, total - t0);
+        for (int p = 4 * tid; p < stop; p += 4 * RD_THREADS) {
+            const uint32_t word = S.start[p >> 5];
+            const int bit = p & 31;
+            int r = S.before[p >> 5] + __popc(word & ((1u << bit) - 1u)) - 1;
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                r += (word >> (bit + k)) & 1u;
+                w[k] = rv[max(r, 0)];  // (before the first run: voxels below `out`, not written)
+            }
+            const int v = t0 + p;
+            uint32_t *dst = slice + out + v;
+            if (v >= 0 && v + 4 <= total) {
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (v + k >= 0 && v + k < total) dst[k] = w[k];
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // pass 3: expand chunks cfirst + blockIdx.x
 __global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restrict__ img, Dir d, long long cfirst,
                                                          long long xy, const unsigned char *__restrict__ entry_of,
@@ -283,6 +352,7 @@ __global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restri
     __shared__ __align__(16) uint16_t W[RD_CHUNK + 8];
     __shared__ int rs[RD_CHUNK];
     __shared__ uint32_t rv[RD_CHUNK];
+    __shared__ RunTile S;
     __shared__ unsigned s_f[RD_THREADS / 32];
     __shared__ int s_i[RD_THREADS / 32];
     const long long c = cfirst + blockIdx.x;
@@ -355,18 +425,7 @@ __global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restri
     }
     __syncthreads();
     const long long end = min(n, out + vtot);
-    for (long long q = out + threadIdx.x; q < end; q += RD_THREADS) {
-        const int rel = (int)(q - out);
-        int lo = 0, hi = rtot - 1;  // last run with start <= rel
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (rs[mid] <= rel)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        out_slice[q] = rv[lo];
-    }
+    rd_write_runs(S, out_slice, out, end, rs, rv, rtot);
     if (bad) atomicOr(err, 1);
 }
 
