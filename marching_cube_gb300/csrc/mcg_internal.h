@@ -140,7 +140,12 @@ struct mcg_context {
     int64_t *batch_caps = nullptr;  // host, last generate's capacities
     size_t batch_caps_cap = 0;
 
-    // GPU run-length encoder: per-slice byte counts / offsets and the image
+    // GPU run-length encoder: per chunk what it holds and its run-start bits,
+    // per-slice byte counts / offsets and the image
+    unsigned char *rle_chunks = nullptr;
+    size_t rle_chunks_cap = 0;
+    uint32_t *rle_marks = nullptr;
+    size_t rle_marks_cap = 0;
     unsigned long long *rle_slices = nullptr;
     size_t rle_slices_cap = 0;
     uint8_t *rle_image = nullptr;

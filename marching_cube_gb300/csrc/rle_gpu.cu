@@ -2,37 +2,37 @@
 // cu_kinect_fusion_v1.cu:1303-1600, described in rle.cpp).
 //
 // The reference encodes slice after slice on one host thread
-// (cu_voxel_run_length_encode_slice, :1367-1417).  Here one CTA encodes one
-// z-slice, sweeping it in chunks of 4096 voxels (16 per thread) and carrying
-// the run state from chunk to chunk:
-//   - voxel i starts a run when i = 0 or it differs from voxel i-1 (tsdf
-//     only in the reference format, the whole voxel in the lossless one);
+// (cu_voxel_run_length_encode_slice, :1367-1417).  The format:
+//   - voxel i of a slice starts a run when i = 0 or it differs from voxel i-1
+//     (tsdf only in the reference format, the whole voxel in the lossless one);
 //   - a record starts at every run start and every 16383 voxels into a run
 //     (the 14-bit count), as the sequential encoder splits long runs;
 //   - a record is 2 bytes (kinds 1/2: +-32766 with, in the lossless format,
 //     w = 0) or 6 bytes (kind 3: header + the record's first voxel).
-// Pass 1 (count) sums each slice's record bytes; the host turns them into
-// slice offsets; pass 2 (write) emits the records into a device image, each
-// record's count being the distance to the next record start (the last one
-// of a chunk waits for the next chunk).  The image then crosses to the host
-// in one copy.
+// Here every chunk of 4096 voxels of a slice is encoded on its own:
+//   1. rle_mark: one pass over the volume; a bit per voxel that starts a run,
+//      and per chunk the bytes of those records and the first and last of them;
+//   2. rle_place: one CTA per slice; the run in force at each chunk's start,
+//      hence the chunk's split (a run that reaches into a chunk has at most one
+//      there: chunks are shorter than 16383), byte offset and the record that
+//      follows it;  rle_slices: the slices' offsets and the image's size;
+//   3. rle_emit: per chunk with records, from its bits, the voxels at record
+//      starts only; the bytes are laid out in shared memory and leave coalesced.
+// The image then crosses to the host in one copy.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
 
-#include <type_traits>
-#include <vector>
-
 #include "mcg_internal.h"
-#include "tma.cuh"
 
 namespace mcg {
 namespace {
 
 constexpr int RT = 256;            // threads per CTA
-constexpr int RV = 16;             // voxels per thread per chunk
-constexpr int RCHUNK = RT * RV;    // 4096
-constexpr unsigned kMaxRun = 0x3fffu;
+constexpr int RCHUNK = 4096;       // voxels per chunk
+constexpr int RWORDS = RCHUNK / 32;
+constexpr int RWARPS = RT / 32;
+constexpr int kMaxRun = 0x3fff;
 
 __device__ __forceinline__ bool same_voxel(uint32_t a, uint32_t b, bool lossless) {
     return lossless ? a == b : ((a ^ b) & 0xffffu) == 0u;
@@ -47,259 +47,277 @@ __device__ __forceinline__ unsigned record_kind(uint32_t v, bool lossless) {
     return 3u;
 }
 
-// write pass: the chunk's record starts
-struct RleSmem {
-    uint32_t pos[RCHUNK];   // record starts of the chunk (slice index)
-    uint32_t vox[RCHUNK];   // their first voxels
-    uint32_t boff[RCHUNK];  // their byte offsets from the chunk's first record
-    uint32_t wn[RT / 32], wb[RT / 32];
-    int wr[RT / 32];
+// a chunk's record starts: the run starts it holds, then what rle_place adds
+struct RleChunk {
+    int first, last;  // slice index of the first and last run start; first = INT32_MAX, last = -1: none
+    int bytes;        // bytes of the records at run starts
+    int split;        // slice index of the record that splits a run from before the chunk, or -1
+    int off;          // byte offset of the chunk's first record in the slice's records
+    int next;         // slice index of the first record after the chunk (the slice's end if none)
 };
 
-// count pass: two chunk buffers, the next chunk's asynchronous copies in
-// flight while the current one is scanned
-struct RleCountSmem {
-    alignas(16) uint32_t stage[2][RCHUNK];
-    uint32_t wn[RT / 32], wb[RT / 32];
-    int wr[RT / 32];
-};
-
-template <bool WRITE>
-using RleS = typename std::conditional<WRITE, RleSmem, RleCountSmem>::type;
-
-// block-wide exclusive sums of two values; totals returned through refs
-template <class SM>
-__device__ __forceinline__ void scan2(SM &S, uint32_t a, uint32_t b, uint32_t &ea, uint32_t &eb, uint32_t &ta,
-                                      uint32_t &tb) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = a, y = b;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t p = __shfl_up_sync(0xffffffffu, x, o), q = __shfl_up_sync(0xffffffffu, y, o);
-        if (lane >= o) {
-            x += p;
-            y += q;
-        }
-    }
-    if (lane == 31) {
-        S.wn[warp] = x;
-        S.wb[warp] = y;
-    }
-    __syncthreads();
-    uint32_t ba = 0, bb = 0, sa = 0, sb = 0;
-#pragma unroll
-    for (int w = 0; w < RT / 32; ++w) {
-        if (w < warp) {
-            ba += S.wn[w];
-            bb += S.wb[w];
-        }
-        sa += S.wn[w];
-        sb += S.wb[w];
-    }
-    __syncthreads();
-    ea = ba + x - a;
-    eb = bb + y - b;
-    ta = sa;
-    tb = sb;
-}
-
-// block-wide inclusive max-scan of a signed value (run starts, -1 = none)
-template <class SM>
-__device__ __forceinline__ int scan_max(SM &S, int v, int carry) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int p = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o && p > x) x = p;
-    }
-    if (lane == 31) S.wr[warp] = x;
-    __syncthreads();
-    int m = carry;
-#pragma unroll
-    for (int w = 0; w < RT / 32; ++w)
-        if (w < warp && S.wr[w] > m) m = S.wr[w];
-    __syncthreads();
-    return x > m ? x : m;
-}
-
-__device__ __forceinline__ void put16(uint8_t *img, unsigned long long off, unsigned v) {
-    *reinterpret_cast<uint16_t *>(img + off) = (uint16_t)v;
-}
-
-// emit one record at byte offset off
-__device__ __forceinline__ void emit(uint8_t *img, unsigned long long off, uint32_t v, unsigned count,
-                                     bool lossless) {
-    const unsigned kind = record_kind(v, lossless);
-    put16(img, off, count | (kind << 14));
-    if (kind == 3u) {
-        put16(img, off + 2, v & 0xffffu);
-        put16(img, off + 4, v >> 16);
-    }
-}
-
-// count pass: chunk starting at c0 into buffer buf by asynchronous copies
-// (16 bytes at a time when vec: the slice is 16-byte aligned), zero past
-// the slice; one commit group per call
-__device__ __forceinline__ void rle_issue_chunk(RleCountSmem &S, const uint32_t *__restrict__ sl, int xy, int c0,
-                                                int buf, bool vec) {
-    const int i0 = c0 + threadIdx.x * RV;
-    uint32_t *dst = S.stage[buf] + threadIdx.x * RV;
-    if (vec && i0 + RV <= xy) {
-#pragma unroll
-        for (int q = 0; q < RV / 4; ++q) cp_async_16(dst + 4 * q, sl + i0 + 4 * q);
-    } else {
-#pragma unroll
-        for (int j = 0; j < RV; ++j) {
-            const bool in = i0 + j < xy;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst + j)),
-                         "l"(in ? sl + i0 + j : sl), "r"(in ? 4u : 0u)
-                         : "memory");
-        }
-    }
-    cp_async_commit();
-}
-
-// WRITE = false: slice_bytes[z] = record bytes of slice z.  WRITE = true:
-// slice z goes to img + slice_off[z]: its byte count (uint32) then records.
-// vec: the slices are 16-byte aligned (count pass only).
-template <bool WRITE>
-__global__ void __launch_bounds__(RT) rle_encode_kernel(const uint32_t *__restrict__ vol, int xy, int lossless_i,
-                                                        unsigned long long *__restrict__ slice_bytes,
-                                                        const unsigned long long *__restrict__ slice_off,
-                                                        uint8_t *__restrict__ img, int vec) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    RleS<WRITE> &S = *reinterpret_cast<RleS<WRITE> *>(smem_raw);
+// Pass 1.  A warp reads 512 consecutive voxels, 16 bytes a lane at a time, all
+// loads ahead of their use.  Bound: HBM.  One CTA sweeping a slice, a block
+// scan per chunk, took 311 us for 512^3 voxels just to count and 563 us more
+// to write (26 MB); the passes here take 138, 5, 2 and 128 us.
+__global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
+                                               RleChunk *__restrict__ chunks, uint32_t *__restrict__ marks, int vec) {
+    constexpr int Q = RCHUNK / RT / 4;  // 16-byte words per lane
+    __shared__ int s_first[RWARPS], s_last[RWARPS], s_bytes[RWARPS];
     const bool lossless = lossless_i != 0;
-    const int z = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long c = blockIdx.x;
+    const int z = (int)(c / nchunks), c0 = (int)(c - (long long)z * nchunks) * RCHUNK;
     const uint32_t *sl = vol + (long long)z * xy;
-    const int tid = threadIdx.x;
-    uint8_t *out = WRITE ? img + slice_off[z] + 4 : nullptr;
-    uint32_t prev = 0;            // voxel before the chunk
-    int rs_carry = -1;            // run start in force at the chunk's start
-    unsigned long long bytes = 0; // bytes of the records started before the chunk
-    int pend = -1;                // record open at the chunk's start (WRITE)
-    uint32_t pend_v = 0;
-    unsigned long long pend_off = 0;
-    // slice indices fit 32 bits: the host rejects slices whose image could
-    // pass the format's 32-bit byte count
-    if constexpr (!WRITE) rle_issue_chunk(S, sl, xy, 0, 0, vec != 0);
-    int buf = 0;
-    for (int c0 = 0; c0 < xy; c0 += RCHUNK, buf ^= 1) {
-        const int i0 = c0 + tid * RV;
-        uint32_t v[RV];
-        uint32_t left;
-        if constexpr (WRITE) {
+    const int w0 = c0 + warp * 128 * Q;  // the warp's voxels w0 .. w0 + 128 Q - 1
+    uint4 v[Q];
 #pragma unroll
-            for (int j = 0; j < RV; ++j) v[j] = i0 + j < xy ? __ldg(sl + i0 + j) : 0u;
-            // previous voxel of each thread's first voxel
-            left = __shfl_up_sync(0xffffffffu, v[RV - 1], 1);
-            if ((tid & 31) == 0) {
-                if (tid == 0) left = prev;
-                else left = i0 - 1 < xy ? __ldg(sl + i0 - 1) : 0u;
-            }
+    for (int q = 0; q < Q; ++q) {
+        const int i = w0 + 128 * q + 4 * lane;
+        if (vec && i < xy) {  // xy is a multiple of 4
+            v[q] = __ldg(reinterpret_cast<const uint4 *>(sl + i));
         } else {
-            // the next chunk's copies go out first (its buffer was last read
-            // before the barriers of the previous chunk), then this chunk's land
-            if (c0 + RCHUNK < xy) rle_issue_chunk(S, sl, xy, c0 + RCHUNK, buf ^ 1, vec != 0);
-            else cp_async_commit();
-            cp_async_wait_group<1>();
-            __syncthreads();
-            const uint4 *src = reinterpret_cast<const uint4 *>(S.stage[buf] + tid * RV);
+            v[q].x = i < xy ? __ldg(sl + i) : 0u;
+            v[q].y = i + 1 < xy ? __ldg(sl + i + 1) : 0u;
+            v[q].z = i + 2 < xy ? __ldg(sl + i + 2) : 0u;
+            v[q].w = i + 3 < xy ? __ldg(sl + i + 3) : 0u;
+        }
+    }
+    uint32_t before = w0 > 0 && w0 <= xy ? __ldg(sl + w0 - 1) : 0u;
+    int bytes = 0, first = INT32_MAX, last = -1;
+    uint32_t *out = marks + c * RWORDS + warp * 4 * Q;
 #pragma unroll
-            for (int q = 0; q < RV / 4; ++q) {
-                const uint4 w = src[q];
-                v[4 * q] = w.x;
-                v[4 * q + 1] = w.y;
-                v[4 * q + 2] = w.z;
-                v[4 * q + 3] = w.w;
-            }
-            left = tid == 0 ? prev : S.stage[buf][tid * RV - 1];
-        }
-        // run starts (local inclusive max), then the block max-scan
-        int rs_loc = -1;
-        uint32_t chg = 0;
+    for (int q = 0; q < Q; ++q) {
+        const int i = w0 + 128 * q + 4 * lane;
+        uint32_t left = __shfl_up_sync(0xffffffffu, v[q].w, 1);
+        if (lane == 0) left = before;
+        before = __shfl_sync(0xffffffffu, v[q].w, 31);
+        const uint32_t x[5] = {left, v[q].x, v[q].y, v[q].z, v[q].w};
+        uint32_t bits = 0;
 #pragma unroll
-        for (int j = 0; j < RV; ++j) {
-            const int i = i0 + j;
-            const uint32_t pv = j == 0 ? left : v[j - 1];
-            const bool c = i < xy && (i == 0 || !same_voxel(v[j], pv, lossless));
-            if (c) {
-                chg |= 1u << j;
-                rs_loc = i;
+        for (int k = 0; k < 4; ++k) {
+            const bool start = i + k < xy && (i + k == 0 || !same_voxel(x[k + 1], x[k], lossless));
+            if (start) {
+                bits |= 1u << k;
+                bytes += record_kind(x[k + 1], lossless) == 3u ? 6 : 2;
             }
         }
-        const int rs_incl = scan_max(S, rs_loc, rs_carry);
-        // run start in force before this thread's first voxel: the exclusive value
-        int rs = __shfl_up_sync(0xffffffffu, rs_incl, 1);
-        if ((tid & 31) == 0) {
-            // exclusive across warps: the block max of everything before this warp
-            rs = rs_carry;
-            for (int w = 0; w < (tid >> 5); ++w)
-                if (S.wr[w] > rs) rs = S.wr[w];
+        if (bits) {
+            first = min(first, i + __ffs(bits) - 1);
+            last = i + 31 - __clz(bits);
         }
-        // record starts and their bytes; d = voxels since the run start, mod 16383
-        uint32_t rec = 0, nrec = 0, nb = 0;
-        unsigned d = (unsigned)(i0 - rs) % kMaxRun;
+        // eight lanes' bits make a word
+        uint32_t word = bits << (4 * (lane & 7));
+        word |= __shfl_xor_sync(0xffffffffu, word, 1);
+        word |= __shfl_xor_sync(0xffffffffu, word, 2);
+        word |= __shfl_xor_sync(0xffffffffu, word, 4);
+        if ((lane & 7) == 0) out[4 * q + (lane >> 3)] = word;
+    }
+    bytes = __reduce_add_sync(0xffffffffu, bytes);
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+        s_first[warp] = first;
+        s_last[warp] = last;
+        s_bytes[warp] = bytes;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        RleChunk r{INT32_MAX, -1, 0, -1, 0, 0};
 #pragma unroll
-        for (int j = 0; j < RV; ++j) {
-            const int i = i0 + j;
-            if (i >= xy) break;
-            if (chg & (1u << j)) d = 0;
-            if (d == 0) {
-                rec |= 1u << j;
-                ++nrec;
-                nb += record_kind(v[j], lossless) == 3u ? 6u : 2u;
-            }
-            d = d + 1 == kMaxRun ? 0u : d + 1;
+        for (int w = 0; w < RWARPS; ++w) {
+            r.first = min(r.first, s_first[w]);
+            r.last = max(r.last, s_last[w]);
+            r.bytes += s_bytes[w];
         }
-        uint32_t er, eb, tr, tb;
-        scan2(S, nrec, nb, er, eb, tr, tb);
-        if constexpr (WRITE) {
-            uint32_t k = er, b = eb;
+        chunks[c] = r;
+    }
+}
+
+// Pass 2.  One warp per slice, 32 chunks at a time: forward for the run in
+// force, the split and the offsets, then backward for the record after each.
+__global__ void __launch_bounds__(32) rle_place(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
+                                                RleChunk *__restrict__ chunks,
+                                                unsigned long long *__restrict__ slice_bytes) {
+    const unsigned int full = 0xffffffffu;
+    const int z = blockIdx.x, lane = threadIdx.x;
+    RleChunk *ch = chunks + (long long)z * nchunks;
+    const uint32_t *sl = vol + (long long)z * xy;
+    int run = 0;                  // start of the run in force at the first of the 32 chunks
+    unsigned long long off = 0;   // bytes before it
+    for (int k0 = 0; k0 < nchunks; k0 += 32) {
+        const int k = k0 + lane, c0 = k * RCHUNK, c1 = min(c0 + RCHUNK, xy);
+        RleChunk r{INT32_MAX, -1, 0, -1, 0, 0};
+        if (k < nchunks) r = ch[k];
+        int m = r.last;  // run starts ascend: the last one so far
 #pragma unroll
-            for (int j = 0; j < RV; ++j) {
-                if (!(rec & (1u << j))) continue;
-                S.pos[k] = (uint32_t)(i0 + j);
-                S.vox[k] = v[j];
-                S.boff[k] = b;
-                b += record_kind(v[j], lossless) == 3u ? 6u : 2u;
-                ++k;
-            }
-            __syncthreads();
-            if (tr > 0) {
-                if (tid == 0 && pend >= 0) emit(out, pend_off, pend_v, (unsigned)((int)S.pos[0] - pend), lossless);
-                for (uint32_t q = tid; q + 1 < tr; q += RT)
-                    emit(out, bytes + S.boff[q], S.vox[q], S.pos[q + 1] - S.pos[q], lossless);
-                pend = (int)S.pos[tr - 1];
-                pend_v = S.vox[tr - 1];
-                pend_off = bytes + S.boff[tr - 1];
-            }
-            __syncthreads();  // pos / vox / boff are rewritten by the next chunk
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(full, m, o);
+            if (lane >= o) m = max(m, u);
         }
-        (void)buf;
-        bytes += tb;
-        // carries: the run start in force and the voxel at the chunk's end
-        if (tid == RT - 1) {
-            S.wr[0] = rs_incl;
-            S.wn[0] = v[RV - 1];
+        int in = __shfl_up_sync(full, m, 1);
+        if (lane == 0) in = -1;
+        in = max(in, run);
+        int split = -1, bytes = r.bytes;
+        if (k < nchunks) {
+            // the first record past c0 - 1 that a run from before the chunk would start
+            const int s = in + (c0 - in + kMaxRun - 1) / kMaxRun * kMaxRun;
+            if (in < c0 && s < min(c1, r.first)) {
+                split = s;
+                bytes += record_kind(__ldg(sl + s), lossless_i != 0) == 3u ? 6 : 2;
+            }
+        }
+        unsigned int sum = (unsigned int)bytes;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int u = __shfl_up_sync(full, sum, o);
+            if (lane >= o) sum += u;
+        }
+        if (k < nchunks) {
+            ch[k].split = split;
+            ch[k].off = (int)(off + sum - (unsigned int)bytes);
+            ch[k].bytes = bytes;
+        }
+        run = max(run, __shfl_sync(full, m, 31));
+        off += __shfl_sync(full, sum, 31);
+    }
+    if (lane == 0) slice_bytes[z] = off;
+    __syncwarp();
+    int after = xy;  // first record after the 32 chunks
+    for (int k0 = (nchunks - 1) / 32 * 32; k0 >= 0; k0 -= 32) {
+        const int k = k0 + lane;
+        int f = INT32_MAX;
+        if (k < nchunks) f = ch[k].split >= 0 ? ch[k].split : ch[k].first;
+        int m = f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_down_sync(full, m, o);
+            if (lane + o < 32) m = min(m, u);
+        }
+        int next = __shfl_down_sync(full, m, 1);
+        if (lane == 31) next = INT32_MAX;
+        if (k < nchunks) ch[k].next = min(next, after);
+        after = min(after, __shfl_sync(full, m, 0));
+    }
+}
+
+// The slices' offsets in the image (after the 40-byte header, each with its
+// 4-byte count) and, behind them, the image's size.  One CTA.
+__global__ void __launch_bounds__(RT) rle_slices(const unsigned long long *__restrict__ bytes, int nz,
+                                                 unsigned long long *__restrict__ off) {
+    __shared__ unsigned long long s_w[RWARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long at = 40;
+    for (int z0 = 0; z0 < nz; z0 += RT) {
+        const int z = z0 + (int)threadIdx.x;
+        const unsigned long long own = z < nz ? 4 + bytes[z] : 0;
+        unsigned long long sum = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += u;
+        }
+        if (lane == 31) s_w[warp] = sum;
+        __syncthreads();
+        unsigned long long pre = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < RWARPS; ++w) {
+            if (w < warp) pre += s_w[w];
+            all += s_w[w];
         }
         __syncthreads();
-        rs_carry = S.wr[0];
-        prev = S.wn[0];
+        if (z < nz) off[z] = at + pre + sum - own;
+        at += all;
+    }
+    if (threadIdx.x == 0) off[nz] = at;
+}
+
+// Pass 3.
+struct RleEmit {
+    int pos[RCHUNK + 1];            // record starts (slice index), then the record after the chunk
+    uint16_t img[3 * RCHUNK + 4];   // the records
+    int wn[RWARPS], wb[RWARPS];
+};
+
+__global__ void __launch_bounds__(RT) rle_emit(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
+                                               const RleChunk *__restrict__ chunks, const uint32_t *__restrict__ marks,
+                                               const unsigned long long *__restrict__ slice_bytes,
+                                               const unsigned long long *__restrict__ slice_off,
+                                               uint8_t *__restrict__ img) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RleEmit &S = *reinterpret_cast<RleEmit *>(smem_raw);
+    const bool lossless = lossless_i != 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long c = blockIdx.x;
+    const int z = (int)(c / nchunks), c0 = (int)(c - (long long)z * nchunks) * RCHUNK;
+    const RleChunk r = chunks[c];
+    const unsigned long long so = slice_off[z];  // even: 40, then 4 and even record bytes a slice
+    if (c0 == 0 && tid < 2) reinterpret_cast<uint16_t *>(img + so)[tid] = (uint16_t)(slice_bytes[z] >> (16 * tid));
+    if (r.bytes == 0) return;  // no record starts here
+    // record starts in order: the split, then the marked voxels
+    const uint32_t word = tid < RWORDS ? marks[c * RWORDS + tid] : 0u;
+    int n = __popc(word), incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) S.wn[warp] = incl;
+    __syncthreads();
+    const int extra = r.split >= 0 ? 1 : 0;
+    int at = extra + incl - n, total = extra;
+#pragma unroll
+    for (int w = 0; w < RWARPS; ++w) {
+        if (w < warp) at += S.wn[w];
+        total += S.wn[w];
+    }
+    for (uint32_t m = word; m; m &= m - 1) S.pos[at++] = c0 + 32 * tid + __ffs(m) - 1;
+    if (tid == 0) {
+        if (extra) S.pos[0] = r.split;
+        S.pos[total] = r.next;
+    }
+    __syncthreads();
+    const uint32_t *sl = vol + (long long)z * xy;
+    int base = 0;  // halfwords before these records
+    for (int j0 = 0; j0 < total; j0 += RT) {
+        const int j = j0 + tid;
+        uint32_t v = 0;
+        int halves = 0, count = 0;
+        unsigned kind = 0;
+        if (j < total) {
+            const int p = S.pos[j];
+            v = __ldg(sl + p);
+            count = S.pos[j + 1] - p;
+            kind = record_kind(v, lossless);
+            halves = kind == 3u ? 3 : 1;
+        }
+        int sum = halves;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += u;
+        }
+        if (lane == 31) S.wb[warp] = sum;
+        __syncthreads();
+        int pre = base, all = 0;
+#pragma unroll
+        for (int w = 0; w < RWARPS; ++w) {
+            if (w < warp) pre += S.wb[w];
+            all += S.wb[w];
+        }
+        const int h = pre + sum - halves;
+        if (halves) {
+            S.img[h] = (uint16_t)((unsigned)count | (kind << 14));
+            if (halves == 3) {
+                S.img[h + 1] = (uint16_t)(v & 0xffffu);
+                S.img[h + 2] = (uint16_t)(v >> 16);
+            }
+        }
+        base += all;
         __syncthreads();
     }
-    if (WRITE) {
-        if (tid == 0) {
-            if (pend >= 0) emit(out, pend_off, pend_v, (unsigned)(xy - pend), lossless);
-            const uint32_t n32 = (uint32_t)bytes;
-            uint8_t *cnt = img + slice_off[z];
-            put16(cnt, 0, n32 & 0xffffu);
-            put16(cnt, 2, n32 >> 16);
-        }
-    } else if (tid == 0) {
-        slice_bytes[z] = bytes;
-    }
+    uint16_t *out = reinterpret_cast<uint16_t *>(img + so + 4 + (unsigned int)r.off);
+    for (int h = tid; h < base; h += RT) out[h] = S.img[h];
 }
 
 const char kTagRef[16] = "VOLUME_TSDF_RGB";
@@ -323,35 +341,34 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    if (!ensure(&ctx->rle_slices, &ctx->rle_slices_cap, (size_t)2 * nz))
+    const long long nchunks = (xy + RCHUNK - 1) / RCHUNK, total = nchunks * nz;
+    if (total > INT32_MAX) return MCG_ERR_TOO_LARGE;  // one CTA each
+    if (!ensure(&ctx->rle_slices, &ctx->rle_slices_cap, (size_t)2 * nz + 1) ||
+        !ensure(&ctx->rle_chunks, &ctx->rle_chunks_cap, (size_t)total * sizeof(RleChunk)) ||
+        !ensure(&ctx->rle_marks, &ctx->rle_marks_cap, (size_t)total * RWORDS))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     unsigned long long *d_bytes = ctx->rle_slices, *d_off = ctx->rle_slices + nz;
-    const size_t smem = sizeof(RleSmem), csmem = sizeof(RleCountSmem);
-    cudaFuncSetAttribute(rle_encode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem);
-    cudaFuncSetAttribute(rle_encode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    RleChunk *chunks = reinterpret_cast<RleChunk *>(ctx->rle_chunks);
+    const uint32_t *v = static_cast<const uint32_t *>(vol);
     const int vec = ((reinterpret_cast<uintptr_t>(vol) & 15u) == 0 && xy % 4 == 0) ? 1 : 0;
-    rle_encode_kernel<false><<<nz, RT, csmem, s>>>(static_cast<const uint32_t *>(vol), (int)xy, lossless ? 1 : 0,
-                                                   d_bytes, nullptr, nullptr, vec);
+    const int ll = lossless ? 1 : 0;
+    rle_mark<<<(unsigned int)total, RT, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks, vec);
+    rle_place<<<nz, 32, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, d_bytes);
+    rle_slices<<<1, RT, 0, s>>>(d_bytes, nz, d_off);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    std::vector<unsigned long long> bytes(nz), off(nz);
-    e = cudaMemcpyAsync(bytes.data(), d_bytes, sizeof(unsigned long long) * nz, cudaMemcpyDeviceToHost, s);
+    unsigned long long o = 0;
+    e = cudaMemcpyAsync(&o, d_off + nz, sizeof(o), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    unsigned long long o = 40;
-    for (int z = 0; z < nz; ++z) {
-        off[z] = o;
-        o += 4 + bytes[z];
-    }
     if (query || (long long)o > capacity) {
         *size = (int64_t)o;
         return query ? MCG_OK : MCG_ERR_CAPACITY;
     }
     if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
-    e = cudaMemcpyAsync(d_off, off.data(), sizeof(unsigned long long) * nz, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    rle_encode_kernel<true><<<nz, RT, smem, s>>>(static_cast<const uint32_t *>(vol), (int)xy, lossless ? 1 : 0, nullptr,
-                                                 d_off, ctx->rle_image, 0);
+    cudaFuncSetAttribute(rle_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RleEmit));
+    rle_emit<<<(unsigned int)total, RT, sizeof(RleEmit), s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks,
+                                                             d_bytes, d_off, ctx->rle_image);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     // header (:1303-1310), then the slices
