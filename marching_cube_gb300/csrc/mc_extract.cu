@@ -48,6 +48,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <type_traits>
 #include <utility>
 
 #include "mc_common.cuh"
@@ -69,7 +70,6 @@ constexpr int CTILE = CTX * CTY * CTZ;
 constexpr int TXO = 0, TYO = 0, TZO = 0;
 constexpr int TX = BX + 4, TY = BY + 2, TZ = BZ + 2;
 constexpr int GTILE = TX * TY * TZ;
-constexpr int GSTAGES = 2;
 // tile stages and minimum resident CTAs per SM of the single-volume generate
 // launch.  One stage measured faster than two at 4 CTAs/SM (a brick's work
 // hides most of its next tile's load, and the smaller footprint lets the next
@@ -757,19 +757,44 @@ struct GenParams {
     long long n_grad;
 };
 
-template <int VT, int NST = GSTAGES>
+// generate_shared's split: soup vertices and records in hand at a time,
+// occupied cubes per brick, slots (see there).  As many as four CTAs per SM
+// leave room for: with 1280 soup vertices and 512 records the 64-volume batch
+// takes 267 us instead of 244 at the same occupancy, and at three CTAs per SM
+// the 1024^3 volume 1204 us instead of 1104.
+constexpr int SH_VERTS = 1536, SH_RECS = 608, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
+
+template <int VT, int NST>
 struct GenSmem {
     static constexpr int STAGE_BYTES = pad128(GTILE * Vox<VT>::bytes);
     unsigned char tiles[NST][STAGE_BYTES];
     unsigned long long neg[ROWS], dead[ROWS];
     uint64_t bars[NST];
-    unsigned int stage[WARPS][32 * 7];
-    unsigned short occ_cube[BRICK_CUBES];  // local cube index (z*8 + y)*32 + x, in that order
-    unsigned short occ_off[BRICK_CUBES];   // exclusive soup-vertex offset inside the brick
-    unsigned char occ_ci[BRICK_CUBES];
+    union {
+        struct {  // one soup vertex at a time (generate_brick, backward_brick)
+            unsigned int stage[WARPS][32 * 7];
+            unsigned short occ_cube[BRICK_CUBES];  // local cube index (z*8 + y)*32 + x, in that order
+            unsigned short occ_off[BRICK_CUBES];   // exclusive soup-vertex offset inside the brick
+            unsigned char occ_ci[BRICK_CUBES];
+        };
+        struct {  // generate_shared: the records of crossed edges
+            unsigned int rec[SH_RECS * 7];
+            float nrm[SH_RECS * 3];
+        };
+    };
+    unsigned int cubes[SH_CUBES];     // occupied cubes in order: cube | case << 11 | soup vertices before it << 19
+    uint2 slot[SH_SLOTS];             // the edges of a slot that are used (bits 0-31 of 33), its first record
+    unsigned int occp[(BY + 2) * (BZ + 2)];  // occupied cubes of cube row (cy, cz) at (cz + 1) * (BY + 2) + cy + 1, zero around
+    unsigned int elut[12];            // edge -> slot step | x step << 16
+    unsigned int wtot[2][WARPS];
+    unsigned short rowcube[CUBE_ROWS];  // occupied cubes before each cube row, and all
+    unsigned int ncube;
+    unsigned int first[(SH_RECS + 31) / 32];  // bit: the first record of a used slot
+    unsigned short used[SH_SLOTS + 1];  // the used slots, in order
     alignas(16) signed char tri[256][16];  // read a row at a time as 16 bytes
     unsigned char nv[256];
-    unsigned short vmap[BRICK_CUBES];      // soup vertex -> local cube << 4 | edge, when the brick has <= 2048
+    unsigned short vmap[SH_VERTS + 1];     // soup vertex -> local cube << 4 | edge, when the brick has <= SH_VERTS;
+                                           // generate_shared: -> record (one more entry is read, not used)
     long long sbrick[NST];                 // brick id, soup offset and origin of each stage's tile
     unsigned long long svbase[NST];
     int4 spos[NST];
@@ -799,7 +824,7 @@ struct GenOut {
 // Occupied-cube list of a brick whose tile is in shared memory: S.occ_cube /
 // occ_ci / occ_off in (z, y, x) order, S.nocc entries, S.total soup
 // vertices, and S.vmap (each vertex's cube and edge) when the brick has at
-// most 2048 of them.  Called by
+// most SH_VERTS of them.  Called by
 // every thread (contains __syncthreads); the list is valid after return.
 template <int VT, class Smem>
 __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T *tile, int nx, int ny, int zlim,
@@ -862,7 +887,7 @@ __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T
         // index << 4 | edge, the edge of output slot k of triangle j being
         // tri[3j + 2 - k] (cu_marching_cubes_v1.cu:322-333); cube offsets are
         // multiples of 3, so a vertex's slot is its index mod 3
-        if (S.total <= BRICK_CUBES) {
+        if (S.total <= SH_VERTS) {
             const unsigned int nocc = S.nocc;
             for (unsigned int i = tid; i < nocc; i += THREADS) {
                 const unsigned int off = S.occ_off[i], ci = S.occ_ci[i], nvc = S.nv[ci];
@@ -879,6 +904,91 @@ __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T
         }
 }
 
+// The soup vertex on the edge from node ga (value f0) to node gb (f1) of the
+// brick at (x0, y0, z0): its position, voxel, that voxel's tsdf and w (also
+// scattered to ver_voxel if given), and its normal.  rcell: mcg_div_reciprocal
+// of the cell, or 0.
+template <int VT>
+__device__ __forceinline__ void make_vertex(const typename Vox<VT>::T *tile,
+                                            const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz,
+                                            float cell, float rcell, int x0, int y0, int z0, float f0, float f1,
+                                            const int ga[3],
+                                            const int gb[3], bool normals, int16_t *ver_voxel, float P[3], int vox[3],
+                                            short &vt, short &vw, float3 &nrm) {
+    using V = Vox<VT>;
+    using T = typename V::T;
+    // getNodeCoo (:243-254) and vertex_interp (:256-264)
+    const float t = (0.0f - f0) / (f1 - f0 + 1e-15f);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float p0 = ((float)ga[d] + 0.5f) * cell;
+        const float p1 = ((float)gb[d] + 0.5f) * cell;
+        P[d] = p0 + t * (p1 - p0);
+    }
+    // store_point (:336-367): voxel of the vertex, its tsdf / w
+    const int dims[3] = {nx, ny, nz};
+    const int org[3] = {x0 - TXO, y0 - TYO, z0 - TZO};
+    const int tdim[3] = {TX, TY, TZ};
+    // P / cell serves both the voxel (:344-350) and the normal sample (kf.cu:3241)
+    float pf[3];
+    if (rcell != 0.0f) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) pf[d] = mcg_div_exact(P[d], cell, rcell);
+    } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) pf[d] = P[d] / cell;
+    }
+    // 16-bit distances: 0 <= t <= 1, so the voxel lies between the one before ga
+    // (by rounding) and gb, and the normal's first sample between ga and gb:
+    // inside the tile but for a voxel below its origin, inside the volume but
+    // for a last sample past its end.  Floats can give any t.
+    bool inside = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        vox[d] = (int)floorf(pf[d] - 0.5f);
+        if (VT == MCG_VOXEL_SHORT2) inside &= vox[d] >= org[d];
+        else inside &= vox[d] >= 0 && vox[d] < dims[d] && vox[d] - org[d] >= 0 && vox[d] - org[d] < tdim[d];
+    }
+    if (inside) {
+        const T vv = tile[tidx(vox[0] - org[0], vox[1] - org[1], vox[2] - org[2])];
+        vt = V::tsdf(vv);
+        vw = V::wt(vv);
+    }
+    if (!inside || ver_voxel) {
+        const long long N = (long long)nx * ny * nz;
+        const long long li = lin3(nx, ny, vox[0], vox[1], vox[2]);
+        if (!inside && li >= 0 && li < N) {
+            const T vv = vol[li];
+            vt = V::tsdf(vv);
+            vw = V::wt(vv);
+        }
+        if (ver_voxel && li >= 0 && li < N) ver_voxel[li] = vt;
+    }
+    if (normals) {
+        const float fx = pf[0], fy = pf[1], fz = pf[2];
+        const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
+        const int lx = ix - org[0], ly = iy - org[1], lz = iz - org[2];
+        if (ix + 1 < nx && iy + 1 < ny && iz + 1 < nz &&
+            (VT == MCG_VOXEL_SHORT2 ||
+             (lx >= 0 && ly >= 0 && lz >= 0 && lx + 1 < TX && ly + 1 < TY && lz + 1 < TZ))) {
+            const T smp[8] = {tile[tidx(lx, ly, lz)],         tile[tidx(lx + 1, ly, lz)],
+                              tile[tidx(lx + 1, ly + 1, lz)], tile[tidx(lx, ly + 1, lz)],
+                              tile[tidx(lx, ly, lz + 1)],     tile[tidx(lx + 1, ly, lz + 1)],
+                              tile[tidx(lx + 1, ly + 1, lz + 1)], tile[tidx(lx, ly + 1, lz + 1)]};
+            bool sent = false;
+            float sd[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                sent |= V::sentinel(smp[q]);
+                put_slot(sd, q, V::f(smp[q]));
+            }
+            if (!sent) nrm = normal_from_samples(sd, fx - (float)ix, fy - (float)iy, fz - (float)iz);
+        } else {
+            nrm = normal_global<VT>(vol, nx, ny, nz, cell, P[0], P[1], P[2]);
+        }
+    }
+}
+
 template <int VT, class Smem>
 __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::T *tile,
                                                const typename Vox<VT>::T *__restrict__ vol, int nx, int ny,
@@ -887,11 +997,10 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
     using V = Vox<VT>;
     using T = typename V::T;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long N = (long long)nx * ny * nz;
 
         occupied_list<VT>(S, tile, nx, ny, o.zlim, x0, y0, z0);
         const unsigned int nocc = S.nocc, T_brick = S.total;
-        const bool use_map = T_brick <= BRICK_CUBES;
+        const bool use_map = T_brick <= SH_VERTS;
 
         // emission: one soup vertex per thread, warps take 32 consecutive vertices
         for (unsigned int v0 = warp * 32; v0 < T_brick; v0 += THREADS) {
@@ -933,65 +1042,10 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
                     V::f(tile[tidx(lcx + TXO + c_cx(a), lcy + TYO + c_cy(a), lcz + TZO + c_cz(a))]);
                 const float f1 =
                     V::f(tile[tidx(lcx + TXO + c_cx(bb), lcy + TYO + c_cy(bb), lcz + TZO + c_cz(bb))]);
-                // getNodeCoo (:243-254) and vertex_interp (:256-264)
-                const float t = (0.0f - f0) / (f1 - f0 + 1e-15f);
                 const int ga[3] = {gx + c_cx(a), gy + c_cy(a), gz + c_cz(a)};
                 const int gb[3] = {gx + c_cx(bb), gy + c_cy(bb), gz + c_cz(bb)};
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const float p0 = ((float)ga[d] + 0.5f) * cell;
-                    const float p1 = ((float)gb[d] + 0.5f) * cell;
-                    P[d] = p0 + t * (p1 - p0);
-                }
-                // store_point (:336-367): voxel of the vertex, its tsdf / w
-                const int dims[3] = {nx, ny, nz};
-                const int org[3] = {x0 - TXO, y0 - TYO, z0 - TZO};
-                const int tdim[3] = {TX, TY, TZ};
-                // P / cell serves both the voxel (:344-350) and the normal sample (kf.cu:3241)
-                const float pf[3] = {P[0] / cell, P[1] / cell, P[2] / cell};
-                bool inside = true;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    vox[d] = (int)floorf(pf[d] - 0.5f);
-                    inside &= vox[d] >= 0 && vox[d] < dims[d] && vox[d] - org[d] >= 0 && vox[d] - org[d] < tdim[d];
-                }
-                if (inside) {
-                    const T vv = tile[tidx(vox[0] - org[0], vox[1] - org[1], vox[2] - org[2])];
-                    vt = V::tsdf(vv);
-                    vw = V::wt(vv);
-                }
-                if (!inside || o.ver_voxel) {
-                    const long long li = lin3(nx, ny, vox[0], vox[1], vox[2]);
-                    if (!inside && li >= 0 && li < N) {
-                        const T vv = vol[li];
-                        vt = V::tsdf(vv);
-                        vw = V::wt(vv);
-                    }
-                    if (o.ver_voxel && li >= 0 && li < N && vbase + v < (unsigned long long)o.cap)
-                        o.ver_voxel[li] = vt;
-                }
-                if (o.normals) {
-                    const float fx = pf[0], fy = pf[1], fz = pf[2];
-                    const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
-                    const int lx = ix - org[0], ly = iy - org[1], lz = iz - org[2];
-                    if (ix + 1 < nx && iy + 1 < ny && iz + 1 < nz && lx >= 0 && ly >= 0 && lz >= 0 &&
-                        lx + 1 < TX && ly + 1 < TY && lz + 1 < TZ) {
-                        const T smp[8] = {tile[tidx(lx, ly, lz)],         tile[tidx(lx + 1, ly, lz)],
-                                          tile[tidx(lx + 1, ly + 1, lz)], tile[tidx(lx, ly + 1, lz)],
-                                          tile[tidx(lx, ly, lz + 1)],     tile[tidx(lx + 1, ly, lz + 1)],
-                                          tile[tidx(lx + 1, ly + 1, lz + 1)], tile[tidx(lx, ly + 1, lz + 1)]};
-                        bool sent = false;
-                        float sd[8];
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            sent |= V::sentinel(smp[q]);
-                            put_slot(sd, q, V::f(smp[q]));
-                        }
-                        if (!sent) nrm = normal_from_samples(sd, fx - (float)ix, fy - (float)iy, fz - (float)iz);
-                    } else {
-                        nrm = normal_global<VT>(vol, nx, ny, nz, cell, P[0], P[1], P[2]);
-                    }
-                }
+                make_vertex<VT>(tile, vol, nx, ny, nz, cell, 0.0f, x0, y0, z0, f0, f1, ga, gb, o.normals != nullptr,
+                                vbase + v < (unsigned long long)o.cap ? o.ver_voxel : nullptr, P, vox, vt, vw, nrm);
             }
             // ---- coalesced stores through the warp stage ----
             const unsigned long long g0 = vbase + v0;  // first record of this warp
@@ -1047,6 +1101,345 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
         }
 }
 
+// A brick's soup, each crossed edge worked out once.
+//
+// A mesh has about six soup vertices per crossed grid edge, and they are two
+// values at most: the reference interpolates an edge in its cube's corner
+// order, which runs against the axis for some of the edges along x (2, 6) and
+// y (3, 7), so an edge along x or y has up to two records, one per direction,
+// and one along z has one.  Each of the brick's 9 x 9 voxel rows has five
+// slots -- x up, x down, y up, y down, z -- of edges whose lower voxel lies in
+// the row, bit x = voxel x; an edge is used where an occupied cube of the
+// brick touches it (such a cube emits every crossed edge of its own).
+//   1. row masks, occupied cubes per cube row;
+//   2. one thread an occupied cube: its case and, by a scan, its soup offset; one thread
+//      a voxel row: its slots' edges, numbered by a scan of their counts;
+//   3. one thread a cube: the record number of each of its soup vertices
+//      (S.vmap); one thread a record: position, voxel and normal;
+//   4. the soup is copied out of the records, whole lines at a time.
+// A brick with more than SH_VERTS soup vertices is taken some layers of cubes
+// at a time.  Bound: instructions (a third of them the records', a quarter the
+// steps before) and, while copying, the shared-memory pipe.  Working out each
+// soup vertex for itself took 578 warp-instructions per 32 soup vertices, this
+// about 400: 512^3 with 1.2 M triangles 100 -> 82 us, 1024^3 with 19 M 1373 ->
+// 1079 us, 64 volumes with 2.7 M 281 -> 204 us (there also with one tile stage
+// and four CTAs per SM instead of two stages).  Returns false (the caller
+// runs generate_brick) where a layer or its records do not fit, or the output
+// ends inside the brick; else tile_done() has been called by every thread
+// between the last use of the tile and the last copy, so that the next brick's
+// tile is fetched meanwhile.  Called by every thread (contains __syncthreads).
+__device__ __forceinline__ unsigned int shared_elut(int e) {
+    // edge e of cube (x, cy, cz): voxel row (cy + dy, cz + dz), slot kind, x step
+    constexpr unsigned int dy[12] = {0, 0, 1, 0, 0, 0, 1, 0, 0, 0, 1, 1};
+    constexpr unsigned int dz[12] = {0, 0, 0, 0, 1, 1, 1, 1, 0, 0, 0, 0};
+    constexpr unsigned int kind[12] = {0, 2, 1, 3, 0, 2, 1, 3, 4, 4, 4, 4};
+    constexpr unsigned int dx[12] = {0, 1, 0, 0, 0, 1, 0, 0, 0, 1, 1, 0};
+    unsigned int v = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+        if (k == e) v = ((dz[k] * (BY + 1) + dy[k]) * 5 + kind[k]) | dx[k] << 16;
+    return v;
+}
+
+__device__ __forceinline__ unsigned int lds_u32(unsigned int addr) {
+    unsigned int v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned int lds_u16(unsigned int addr) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// position of the j-th set bit of m (j < popc(m))
+__device__ __forceinline__ int select_bit(unsigned int m, unsigned int j) {
+    int at = 0;
+#pragma unroll
+    for (int h = 16; h; h >>= 1) {
+        const unsigned int c = __popc(m & ((1u << h) - 1u));
+        if (j >= c) {
+            j -= c;
+            m >>= h;
+            at += h;
+        }
+    }
+    return at;
+}
+
+// the parts of shared memory that no brick changes; before the kernel's first barrier
+template <class Smem>
+__device__ __forceinline__ void shared_init(Smem &S) {
+    const int tid = threadIdx.x;
+    if (tid < 12) S.elut[tid] = shared_elut(tid);
+    if (tid < (BY + 2) * (BZ + 2)) S.occp[tid] = 0u;
+}
+
+template <int VT, class Smem, class Done>
+__device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>::T *tile,
+                                                const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz,
+                                                float cell, int x0, int y0, int z0, unsigned long long vbase,
+                                                const GenOut &o, Done tile_done) {
+    using V = Vox<VT>;
+    const unsigned int full = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // (float distances can make a position infinite)
+    const float rcell = VT == MCG_VOXEL_SHORT2 ? mcg_div_reciprocal(cell) : 0.0f;
+    if (tid < ROWS) {
+        const int ry = tid % (BY + 1), rz = tid / (BY + 1);
+        RowMask<VT>::build(tile + tidx(TXO, ry + TYO, rz + TZO), S.neg[tid], S.dead[tid]);
+    }
+    __syncthreads();
+    // 1. occupied cubes: lane l of the first two warps has cube rows l and
+    // l + 32, both for the counts before row tid
+    if (tid < CUBE_ROWS) {
+        unsigned int occ[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int cy = lane & (BY - 1), cz = lane / BY + 4 * h;
+            occ[h] = y0 + cy < ny - 1 && z0 + cz < o.zlim ? cube_row(S.neg, S.dead, cy, cz, valid_mask(x0, nx)).occ : 0u;
+        }
+        const unsigned int own = __popc(occ[0]) | (__popc(occ[1]) << 16);
+        unsigned int incl = own;
+#pragma unroll
+        for (int q = 1; q < 32; q <<= 1) {
+            const unsigned int u = __shfl_up_sync(full, incl, q);
+            if (lane >= q) incl += u;
+        }
+        const unsigned int all = __shfl_sync(full, incl, 31);
+        incl -= own;
+        const int cy = tid & (BY - 1), cz = tid / BY;
+        S.occp[(cz + 1) * (BY + 2) + cy + 1] = warp == 0 ? occ[0] : occ[1];
+        S.rowcube[tid] = (unsigned short)(warp == 0 ? incl & 0xffffu : (all & 0xffffu) + (incl >> 16));
+        if (tid == 0) S.ncube = (all & 0xffffu) + (all >> 16);
+    }
+    __syncthreads();
+    const unsigned int nocc = S.ncube;
+    if (nocc > SH_CUBES) return false;
+    // slots of layers [za, zb): this thread's voxel row; then their numbers
+    unsigned long long m[5];
+    int at = 0;
+    auto count_slots = [&](int za, int zb) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) m[k] = 0ull;
+        if (tid < ROWS) {
+            const int lz = tid / (BY + 1), ly = tid - (BY + 1) * lz;
+            const unsigned int *q = S.occp + (lz + 1) * (BY + 2) + ly + 1;  // cube row (ly, lz)
+            const bool up = lz >= za && lz < zb, dn = lz > za && lz <= zb;  // layers lz and lz - 1
+            const unsigned int o11 = up ? q[0] : 0u, o01 = up ? q[-1] : 0u;
+            const unsigned int o10 = dn ? q[-(BY + 2)] : 0u, o00 = dn ? q[-(BY + 2) - 1] : 0u;
+            const unsigned long long n = S.neg[tid];
+            const unsigned int cx = (unsigned int)(n ^ (n >> 1));
+            m[0] = cx & (o11 | o10);
+            m[1] = cx & (o01 | o00);
+            if (ly < BY) {
+                const unsigned long long cy = n ^ S.neg[tid + 1], u = o11 | o10;
+                m[2] = cy & (u << 1);
+                m[3] = cy & u;
+            }
+            if (lz < BZ) {
+                const unsigned long long cz = n ^ S.neg[tid + BY + 1], u = o11 | o01;
+                m[4] = cz & (u | (u << 1));
+            }
+        }
+        if (tid < (SH_RECS + 31) / 32) S.first[tid] = 0u;
+        if (warp < (ROWS + 31) / 32) {
+            int sum = 0;  // records | used slots << 16
+#pragma unroll
+            for (int k = 0; k < 5; ++k) sum += __popcll(m[k]) + (m[k] ? 0x10000 : 0);
+            at = sum;
+#pragma unroll
+            for (int q = 1; q < 32; q <<= 1) {
+                const int u = __shfl_up_sync(full, at, q);
+                if (lane >= q) at += u;
+            }
+            if (lane == 31) S.wtot[1][warp] = (unsigned int)at;
+            at -= sum;
+        }
+    };
+    auto number_slots = [&]() -> int {
+        const int t0 = (int)S.wtot[1][0], t1 = (int)S.wtot[1][1], R = (t0 + t1 + (int)S.wtot[1][2]) & 0xffff;
+        if (R <= SH_RECS && tid < ROWS) {
+            at += (warp > 0 ? t0 : 0) + (warp > 1 ? t1 : 0);
+            int u = at >> 16;
+            at &= 0xffff;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (m[k]) {
+                    S.slot[5 * tid + k] = make_uint2((unsigned int)m[k], (unsigned int)at);
+                    S.used[u++] = (unsigned short)(5 * tid + k);
+                    atomicOr(&S.first[at >> 5], 1u << (at & 31));
+                    at += __popcll(m[k]);
+                }
+            }
+        }
+        return R;
+    };
+    // 2. cases and soup offsets of the cubes, and the slots of the whole brick
+    unsigned int T_brick = 0;
+    int R = 0;
+    for (unsigned int i0 = 0; i0 < nocc; i0 += THREADS) {
+        const unsigned int i = i0 + tid;
+        unsigned int c = 0, nv = 0;
+        if (i < nocc) {
+            // the last row with rowcube <= i is the cube's, and it is the (i - rowcube)-th there
+            unsigned int row = 0;
+#pragma unroll
+            for (int h = CUBE_ROWS / 2; h; h >>= 1)
+                if (S.rowcube[row + h] <= i) row += h;
+            const int x0r = select_bit(S.occp[(row / BY + 1) * (BY + 2) + (row & (BY - 1)) + 1], i - S.rowcube[row]);
+            c = row * BX + x0r;
+            const int x = x0r, r = (int)(c >> 8) * (BY + 1) + ((int)(c >> 5) & 7);
+            const unsigned int a = (unsigned int)(S.neg[r] >> x) & 3u, b = (unsigned int)(S.neg[r + 1] >> x) & 3u;
+            const unsigned int d = (unsigned int)(S.neg[r + BY + 1] >> x) & 3u;
+            const unsigned int e = (unsigned int)(S.neg[r + BY + 2] >> x) & 3u;
+            // corners 2, 3 and 6, 7 run against x
+            const unsigned int ci = a | (b >> 1) << 2 | (b & 1u) << 3 | d << 4 | (e >> 1) << 6 | (e & 1u) << 7;
+            nv = S.nv[ci];
+            c |= ci << 11;
+        }
+        unsigned int incl = nv;
+#pragma unroll
+        for (int q = 1; q < 32; q <<= 1) {
+            const unsigned int u = __shfl_up_sync(full, incl, q);
+            if (lane >= q) incl += u;
+        }
+        if (lane == 31) S.wtot[0][warp] = incl;
+        if (i0 == 0) count_slots(0, BZ);
+        __syncthreads();
+        unsigned int pre = T_brick + incl - nv;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const unsigned int t = S.wtot[0][w];
+            if (w < warp) pre += t;
+            T_brick += t;
+        }
+        if (i < nocc) S.cubes[i] = c | (pre << 19);
+        if (i0 == 0) R = number_slots();
+        __syncthreads();
+    }
+    if (T_brick >= (1u << 13) || (long long)(vbase + T_brick) > o.cap) return false;
+    for (int za = 0, zb = BZ; za < BZ; za = zb, zb = BZ) {
+        unsigned int i0 = 0, i1 = nocc, va = 0, nT = T_brick;
+        if (T_brick > SH_VERTS) {
+            // the layers from za on that fit; soup vertices before layer z: its first cube's
+            auto verts = [&](int z) -> unsigned int {
+                const unsigned int i = z < BZ ? S.rowcube[z * BY] : nocc;
+                return i < nocc ? S.cubes[i] >> 19 : T_brick;
+            };
+            va = verts(za);
+            while (zb > za && verts(zb) - va > (unsigned int)SH_VERTS) --zb;
+            if (zb == za) return false;  // one layer is too much
+            i0 = S.rowcube[za * BY];
+            i1 = zb < BZ ? S.rowcube[zb * BY] : nocc;
+            nT = verts(zb) - va;
+            if (nT == 0) continue;
+            count_slots(za, zb);
+            __syncthreads();
+            R = number_slots();
+            __syncthreads();
+        }
+        if (R > SH_RECS) return false;  // uniform
+        // 3. the record of every soup vertex (the last threads first: the
+        // first ones have the records)
+        const unsigned long long g0 = vbase + va;
+        for (unsigned int i = i0 + (THREADS - 1 - tid); i < i1; i += THREADS) {
+            const unsigned int w = S.cubes[i], ci = (w >> 11) & 0xffu, off = (w >> 19) - va;
+            const int x = (int)(w & 31u), cy = (int)(w >> 5) & 7, cz = (int)(w >> 8) & 7;
+            const uint2 *sl = S.slot + 5 * (cz * (BY + 1) + cy);
+            const unsigned int below = (1u << x) - 1u, below1 = below << 1 | 1u;
+            const signed char *tri = S.tri[ci];
+            const unsigned int nvc = S.nv[ci];
+            for (unsigned int q = 0; q < nvc; q += 3) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const unsigned int l = S.elut[tri[q + 2 - k]];
+                    const uint2 v = sl[l & 0xffffu];
+                    S.vmap[off + q + k] = (unsigned short)(v.y + __popc(v.x & (l >> 16 ? below1 : below)));
+                }
+                if (o.tri_cube) o.tri_cube[(g0 + off + q) / 3] = lin3(nx, ny, x0 + x, y0 + cy, z0 + cz);
+            }
+        }
+        // and the records
+        const unsigned int firsts = lane < (SH_RECS + 31) / 32 ? S.first[lane] : 0u;
+        for (int r = tid; r - lane < R; r += THREADS) {
+            // its slot: used slots that start up to it; the warp's 32 records are one word of S.first
+            const int word = r >> 5;
+            const int slots = __reduce_add_sync(full, lane < word ? __popc(firsts) : 0) +
+                              __popc(__shfl_sync(full, firsts, word) & (0xffffffffu >> (31 - lane)));
+            if (r >= R) break;
+            const int s = S.used[slots - 1], row = s / 5, kind = s - 5 * row;
+            const uint2 sl = S.slot[s];
+            const int lz = row / (BY + 1), ly = row - (BY + 1) * lz;
+            const int j = r - (int)sl.y, x = j < __popc(sl.x) ? select_bit(sl.x, (unsigned int)j) : 32, dx = kind < 2, dy = kind == 2 || kind == 3, dz = kind == 4;
+            const bool down = kind == 1 || kind == 3;
+            const int t = tidx(x + TXO, ly + TYO, lz + TZO);
+            const float lo = V::f(tile[t]), hi = V::f(tile[t + dx + dy * TX + dz * (TX * TY)]);
+            const int l[3] = {x0 + x, y0 + ly, z0 + lz}, h[3] = {l[0] + dx, l[1] + dy, l[2] + dz};
+            const int ga[3] = {down ? h[0] : l[0], down ? h[1] : l[1], l[2]};
+            const int gb[3] = {down ? l[0] : h[0], down ? l[1] : h[1], h[2]};
+            float P[3];
+            int vox[3];
+            short vt = 0, vw = 0;
+            float3 nrm = make_float3(0.f, 0.f, 0.f);
+            make_vertex<VT>(tile, vol, nx, ny, nz, cell, rcell, x0, y0, z0, down ? hi : lo, down ? lo : hi, ga, gb,
+                            o.normals != nullptr, o.ver_voxel, P, vox, vt, vw, nrm);
+            unsigned int *rec = S.rec + 7 * r;
+            rec[0] = __float_as_uint(P[0]);
+            rec[1] = __float_as_uint(P[1]);
+            rec[2] = __float_as_uint(P[2]);
+            rec[3] = (unsigned int)vox[0];
+            rec[4] = (unsigned int)vox[1];
+            rec[5] = (unsigned int)vox[2];
+            rec[6] = (unsigned int)(unsigned short)vt | ((unsigned int)(unsigned short)vw << 16);
+            S.nrm[3 * r] = nrm.x;
+            S.nrm[3 * r + 1] = nrm.y;
+            S.nrm[3 * r + 2] = nrm.z;
+        }
+        __syncthreads();
+        if (zb == BZ) tile_done();
+        // 4. out, 16 bytes a thread from the first 16-byte boundary on.  Bound:
+        // the shared-memory and store pipe; with a word a thread (an entry of
+        // the map, a word of the record and a store for each) this was a
+        // quarter of the launch.
+        auto copy = [&](unsigned int *out, const unsigned int *from, auto words, unsigned int stride, unsigned int first) {
+            constexpr int W = decltype(words)::value;
+            unsigned int *dst = out + g0 * W;
+            const int n = (int)nT * W, lead = (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 3u);
+            const unsigned int rec0 = smem_u32(from) + 4 * first, map0 = smem_u32(S.vmap);
+            for (int i = 4 * tid - lead; i < n; i += 4 * THREADS) {
+                // words i .. i + 3 (i = -lead: from 0 on); they lie in at most two soup vertices
+                const int i0 = max(i, 0);
+                const unsigned int v = W == 7 ? (i0 * 9363u) >> 16 : (i0 * 21846u) >> 16;  // i0 / W
+                const int w = i - W * (int)v;
+                const unsigned int a0 = rec0 + 4 * stride * lds_u16(map0 + 2 * v) + 4 * w;
+                const unsigned int a1 = rec0 + 4 * stride * lds_u16(map0 + 2 * v + 2) + 4 * (w - W);
+                if (i >= 0 && i + 4 <= n) {
+                    uint4 q;
+                    q.x = lds_u32(a0);
+                    q.y = lds_u32((w + 1 < W ? a0 : a1) + 4);
+                    q.z = lds_u32((w + 2 < W ? a0 : a1) + 8);
+                    q.w = lds_u32((w + 3 < W ? a0 : a1) + 12);
+                    *reinterpret_cast<uint4 *>(dst + i) = q;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (i + k >= 0 && i + k < n) dst[i + k] = lds_u32((w + k < W ? a0 : a1) + 4 * k);
+                }
+            }
+        };
+        const std::integral_constant<int, 7> seven;
+        const std::integral_constant<int, 3> three;
+        if (o.soup) copy(reinterpret_cast<unsigned int *>(o.soup), S.rec, seven, 7, 0);
+        if (o.normals)
+            copy(reinterpret_cast<unsigned int *>(o.normals), reinterpret_cast<const unsigned int *>(S.nrm), three, 3, 0);
+        if (o.vi2vox) copy(reinterpret_cast<unsigned int *>(o.vi2vox), S.rec, three, 7, 3);
+        if (zb < BZ) __syncthreads();  // the next layers' slots and records
+    }
+    return true;
+}
+
 // Adjoint of the soup positions with respect to the voxel values, for one
 // brick whose tile is in shared memory.  Soup vertex v of the brick lies on
 // edge (a, b) of its cube: P = p_a + t (p_b - p_a), t = -f_a / D,
@@ -1065,7 +1458,7 @@ __device__ __forceinline__ void backward_brick(Smem &S, const typename Vox<VT>::
     const int tid = threadIdx.x;
     occupied_list<VT>(S, tile, nx, ny, zlim, x0, y0, z0);
     const unsigned int nocc = S.nocc, T_brick = S.total;
-    const bool use_map = T_brick <= BRICK_CUBES;
+    const bool use_map = T_brick <= SH_VERTS;
     for (unsigned int v = tid; v < T_brick; v += THREADS) {
         const unsigned long long gv = vbase + v;
         if ((long long)gv >= n_grad) break;
@@ -1120,6 +1513,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
 
     load_tri_table(S.tri, tid, THREADS);
     S.nv[tid] = (tid == 0 || tid == 255) ? 0 : g_nverts[tid];
+    shared_init(S);
     if (tid == 0) {
         S.abort = 0;
         if (TMA) {
@@ -1217,6 +1611,21 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
                                       bp.y0 - TYO, bp.z0 - TZO);
             __syncthreads();
         }
+        // the tile of stage s is free: the next brick of this stage
+        auto refill = [&]() {
+            if (TMA && tid == 0) {
+                cp_async_wait_all();
+                const unsigned int pb = S.pipe_b;
+                stage_brick(s, pb == 0xffffffffu ? -1ll : (long long)pb, S.pipe_v);
+                S.pipe_b = 0xffffffffu;
+                if (ptk < nactive) {
+                    cp_async_4(&S.pipe_b, p.active + ptk);
+                    cp_async_8(&S.pipe_v, p.list_vofs + ptk);
+                } else {
+                    ptk = 0xffffffffu;  // the list is exhausted: draw no more tickets
+                }
+            }
+        };
         if (MODE == 0) {
             GenOut o;
             o.soup = p.soup;
@@ -1226,27 +1635,20 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
             o.tri_cube = p.tri_cube;
             o.cap = p.cap;
             o.zlim = p.zlim;
-            generate_brick<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o);
+            if (!generate_shared<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o, refill)) {
+                __syncthreads();
+                generate_brick<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o);
+                __syncthreads();
+                refill();
+            }
         } else {
             backward_brick<VT>(S, tile, nx, ny, nz, p.zlim, cell, bp.x0, bp.y0, bp.z0, vbase, p.grad_pos,
                                p.grad_f, p.n_grad);
+            __syncthreads();
+            refill();
         }
-        __syncthreads();  // tile s, the list and the stage are free again
-        if (TMA && tid == 0) {
-            cp_async_wait_all();
-            const unsigned int pb = S.pipe_b;
-            stage_brick(s, pb == 0xffffffffu ? -1ll : (long long)pb, S.pipe_v);
-            S.pipe_b = 0xffffffffu;
-            if (ptk < nactive) {
-                cp_async_4(&S.pipe_b, p.active + ptk);
-                cp_async_8(&S.pipe_v, p.list_vofs + ptk);
-            } else {
-                ptk = 0xffffffffu;  // the list is exhausted: draw no more tickets
-            }
-        }
-        // S.sbrick[s] is next read at the top of iteration it + GEN_STAGES, after the
-        // barriers of iteration it + 1 (with one stage: after this barrier)
-        if (GEN_STAGES == 1) __syncthreads();
+        __syncthreads();  // the brick's lists and records are free again, the next brick's number is there
+        // S.sbrick[s] is next read at the top of iteration it + GEN_STAGES, after that barrier
     }
     if (S.abort && tid == 0) {
         atomicOr(&p.totals->flags, 1u);
@@ -2030,23 +2432,22 @@ __global__ void __launch_bounds__(CTHREADS)
 }
 
 template <int VT>
-struct GenSmemMulti : GenSmem<VT, 2> {
-    int svol[2];
-    int stma[2];
+struct GenSmemMulti : GenSmem<VT, 1> {
+    int svol;  // volume of the staged brick, -1: none
+    int stma;
     alignas(16) BatchBrick pipe;  // entry staged at the next refill (thread 0's pipeline)
 };
 
 template <int VT>
-__device__ __forceinline__ void issue_gen_tile(GenSmemMulti<VT> &S, int s, const VolDesc *__restrict__ vols,
+__device__ __forceinline__ void issue_gen_tile(GenSmemMulti<VT> &S, const VolDesc *__restrict__ vols,
                                                const CUtensorMap *maps, const BatchBrick &r) {
-    S.svol[s] = r.v;
-    S.stma[s] = vols[r.v].tma;
-    S.sbrick[s] = 0;
-    S.svbase[s] = r.vbase;
-    S.spos[s] = make_int4(r.x0, r.y0, r.z0, 0);
+    S.svol = r.v;
+    S.stma = vols[r.v].tma;
+    S.svbase[0] = r.vbase;
+    S.spos[0] = make_int4(r.x0, r.y0, r.z0, 0);
     if (vols[r.v].tma) {
-        mbar_arrive_expect_tx(&S.bars[s], GTILE * Vox<VT>::bytes);
-        tma_load_3d(S.tiles[s], maps + r.v, &S.bars[s], r.x0 - TXO, r.y0 - TYO, r.z0 - TZO);
+        mbar_arrive_expect_tx(&S.bars[0], GTILE * Vox<VT>::bytes);
+        tma_load_3d(S.tiles[0], maps + r.v, &S.bars[0], r.x0 - TXO, r.y0 - TYO, r.z0 - TZO);
     }
 }
 
@@ -2063,49 +2464,54 @@ __global__ void __launch_bounds__(THREADS, 4)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     GenSmemMulti<VT> &S = *reinterpret_cast<GenSmemMulti<VT> *>(smem_raw);
     const int tid = threadIdx.x;
-    uint32_t phase[2] = {0, 0};
+    uint32_t phase = 0;
     load_tri_table(S.tri, tid, THREADS);
     S.nv[tid] = (tid == 0 || tid == 255) ? 0 : g_nverts[tid];
+    shared_init(S);
     pdl_wait();  // the batch's scan: active list, totals, cleared counter
     const unsigned int nactive = totals->active_bricks;
     unsigned int *ticket = &totals->gen_ticket;
     const unsigned int grid = gridDim.x, c = blockIdx.x;
-    const unsigned int tbase = 3 * grid;  // list entry of ticket 0
-    auto entry = [&](unsigned int r) { return r * grid + ((r & 1) ? grid - 1 - c : c); };
-    unsigned int ptk = 0xffffffffu;  // list entry of the ticket drawn at the top of this brick
+    const unsigned int nfix = 3, tbase = nfix * grid;  // list entry of ticket 0
+    auto next_entry = [&](unsigned int k) {
+        return k < nfix ? k * grid + ((k & 1) ? grid - 1 - c : c) : tbase + atomicAdd(ticket, 1u);
+    };
+    unsigned int ptk = 0xffffffffu;  // list entry drawn at the top of this brick
+    unsigned int kdraw = 2;          // entries assigned so far (thread 0)
     bool have_pipe = false;          // S.pipe holds the entry of the next refill
+    auto fetch = [&](unsigned int w) {  // list entry w into S.pipe
+        cp_async_16(&S.pipe, list + w);
+        cp_async_16(reinterpret_cast<unsigned char *>(&S.pipe) + 16, reinterpret_cast<const unsigned char *>(list + w) + 16);
+    };
     if (tid == 0) {
         S.abort = 0;
-        for (int s = 0; s < 2; ++s) mbar_init(&S.bars[s], 1);
+        mbar_init(&S.bars[0], 1);
         fence_barrier_init();
-        for (int s = 0; s < 2; ++s) {
-            S.svol[s] = -1;
-            const unsigned int w = entry(s);
-            if (w < nactive) issue_gen_tile<VT>(S, s, vols, maps, list[w]);
+        S.svol = -1;
+        unsigned int w = next_entry(0);
+        if (w < nactive) issue_gen_tile<VT>(S, vols, maps, list[w]);
+        w = next_entry(1);
+        have_pipe = w < nactive;
+        if (have_pipe) {
+            fetch(w);
+            ptk = 0;  // not ~0u: draw entries at the tops of the bricks
         }
-        const unsigned int w = entry(2);
-        if (w < nactive) {
-            cp_async_16(&S.pipe, list + w);
-            cp_async_16(reinterpret_cast<unsigned char *>(&S.pipe) + 16, reinterpret_cast<const unsigned char *>(list + w) + 16);
-            have_pipe = true;
-        }
-        if (tbase < nactive) ptk = 0;  // not ~0u: draw tickets at the tops of the bricks
     }
     __syncthreads();
-    for (int it = 0;; ++it) {
-        const int s = it & 1;
-        T *tile = reinterpret_cast<T *>(S.tiles[s]);
-        const int v = S.svol[s];
+    for (;;) {
+        T *tile = reinterpret_cast<T *>(S.tiles[0]);
+        const int v = S.svol;
         if (v < 0) break;  // uniform
+        const bool tma = S.stma != 0;
         if (tid == 0) {
-            if (ptk != 0xffffffffu) ptk = tbase + atomicAdd(ticket, 1u);
-            if (S.stma[s] && !mbar_wait(&S.bars[s], phase[s])) S.abort = 1;
+            if (ptk != 0xffffffffu) ptk = next_entry(kdraw++);
+            if (tma && !mbar_wait(&S.bars[0], phase)) S.abort = 1;
         }
-        if (S.stma[s]) phase[s] ^= 1u;
-        const unsigned long long vbase = S.svbase[s];
-        const int4 sp = S.spos[s];
+        if (tma) phase ^= 1u;
+        const unsigned long long vbase = S.svbase[0];
+        const int4 sp = S.spos[0];
         const VolDesc &d = vols[v];
-        if (!S.stma[s])
+        if (!tma)
             fill_tile<VT, TX, TY, TZ>(tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, sp.x - TXO, sp.y - TYO,
                                       sp.z - TZO);
         __syncthreads();
@@ -2118,30 +2524,32 @@ __global__ void __launch_bounds__(THREADS, 4)
         o.tri_cube = d.tri_cube;
         o.cap = d.cap;
         o.zlim = d.nz - 1;
-        generate_brick<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x, sp.y, sp.z,
-                           vbase, o);
-        __syncthreads();  // tile s, the list and the stage are free again
-        if (tid == 0) {
-            S.svol[s] = -1;
-            if (have_pipe) {
-                cp_async_wait_all();
-                issue_gen_tile<VT>(S, s, vols, maps, S.pipe);
+        // the tile is free: the next brick
+        auto refill = [&]() {
+            if (tid == 0) {
+                S.svol = -1;
+                if (have_pipe) {
+                    cp_async_wait_all();
+                    issue_gen_tile<VT>(S, vols, maps, S.pipe);
+                }
+                have_pipe = ptk < nactive;
+                if (have_pipe) fetch(ptk);
+                else ptk = 0xffffffffu;  // the list is exhausted: draw no more
             }
-            have_pipe = ptk < nactive;
-            if (have_pipe) {
-                cp_async_16(&S.pipe, list + ptk);
-                cp_async_16(reinterpret_cast<unsigned char *>(&S.pipe) + 16,
-                            reinterpret_cast<const unsigned char *>(list + ptk) + 16);
-            } else {
-                ptk = 0xffffffffu;  // the list is exhausted: draw no more tickets
-            }
+        };
+        if (!generate_shared<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x, sp.y, sp.z,
+                                 vbase, o, refill)) {
+            __syncthreads();
+            generate_brick<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x, sp.y, sp.z,
+                               vbase, o);
+            __syncthreads();
+            refill();
         }
-        // S.svol[s] is next read at the top of iteration it + 2, after the
-        // barriers of iteration it + 1
+        __syncthreads();  // the brick's lists and records are free again, the next brick is there
     }
     if (S.abort && tid == 0) {
         atomicOr(&totals->flags, 1u);
-        for (int s = 0; s < 2; ++s) mbar_wait(&S.bars[s], phase[s], 100000000ull);
+        mbar_wait(&S.bars[0], phase, 100000000ull);
     }
     // the last CTA out folds the flags into the mapped host copy, where the
     // batch's scan put the count launch's

@@ -26,3 +26,27 @@ MCG_HD float mcg_unpack_tsdf(int t) {
     const float e = fmaf(-q, c, a);
     return fmaf(e, r, q);
 }
+
+// RN(a / b) from y = RN(1 / b): two corrections of RN(a * y) by the exact
+// remainder.  With |y b - 1| <= 2^-24 b / 2 (b scaled to [1, 2)) the first
+// leaves an error of half an ulp and a 2^-23 of one; the second one's is then
+// below 2^-48 b / 2 (1 + 2^-22), and no quotient of 24-bit numbers lies nearer
+// than 2^-48 (2 / b) to a rounding boundary, unless b's significand is all
+// ones, for which mcg_div_reciprocal gives 0.  It gives 0 too where the
+// remainders could underflow; with y = 0 the caller divides.  The quotient must not overflow.
+MCG_HD float mcg_div_reciprocal(float b) {
+    const bool plain = b > 1e-25f && b < 1e25f;
+#if defined(__CUDA_ARCH__)
+    const unsigned int u = __float_as_uint(b);
+#else
+    unsigned int u;
+    __builtin_memcpy(&u, &b, 4);
+#endif
+    return plain && (u & 0x7fffffu) != 0x7fffffu ? 1.0f / b : 0.0f;
+}
+
+MCG_HD float mcg_div_exact(float a, float b, float y) {
+    const float q = a * y;
+    const float q1 = fmaf(fmaf(-q, b, a), y, q);
+    return fmaf(fmaf(-q1, b, a), y, q1);
+}
