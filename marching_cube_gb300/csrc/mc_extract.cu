@@ -48,6 +48,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <type_traits>
 #include <utility>
 
@@ -61,9 +62,8 @@ constexpr int WARPS = THREADS / 32;
 constexpr int ROWS = (BY + 1) * (BZ + 1);  // voxel rows feeding one brick: 81
 constexpr int CUBE_ROWS = BY * BZ;         // 64
 
-// classify tile: voxels [x0, x0+36) x [y0, y0+9) x [z0, z0+9)
-constexpr int CTX = 36, CTY = BY + 1, CTZ = BZ + 1;
-constexpr int CTILE = CTX * CTY * CTZ;
+// voxel rows and planes of a classify tile
+constexpr int CTY = BY + 1, CTZ = BZ + 1;
 // generate tile: voxels [x0, x0+36) x [y0, y0+10) x [z0, z0+10) -- every
 // corner and normal sample of the brick's cubes; the rare side-output reads
 // of voxel x0-1 / y0-1 / z0-1 go to global memory
@@ -172,81 +172,9 @@ __device__ __forceinline__ unsigned int valid_mask(int x0, int nx) {
 }
 
 // ---- pass 1: classify ------------------------------------------------------
-constexpr int CTHREADS = 128;
 
-// True when the tile holds both negative and non-negative voxels.  Most
-// bricks of a fusion volume lie wholly on one side of the surface (or in
-// unobserved space, all -32766), and no cube of such a brick changes sign, so
-// one OR / AND pass over the tile's sign bits settles them before any mask
-// work.  Called by every thread; contains a barrier.
-template <int VT, int NVOX = CTILE, class Smem>
-__device__ __forceinline__ bool tile_mixed(Smem &S, const typename Vox<VT>::T *tile) {
-    static_assert(NVOX * Vox<VT>::bytes % 16 == 0, "tile is a whole number of 16-byte words");
-    constexpr int NQ = NVOX * Vox<VT>::bytes / 16;
-    const uint4 *q = reinterpret_cast<const uint4 *>(tile);
-    unsigned int neg_any = 0, pos_any = 0;
-    for (int i = threadIdx.x; i < NQ; i += blockDim.x) {
-        const uint4 v = q[i];
-        if (VT == MCG_VOXEL_SHORT2) {
-            // bit 15 of each word is the tsdf sign
-            neg_any |= v.x | v.y | v.z | v.w;
-            pos_any |= ~(v.x & v.y & v.z & v.w);
-        } else {
-            // x and z are the tsdf of two voxels; -0.0f is not negative
-            const bool n0 = __uint_as_float(v.x) < 0.f, n1 = __uint_as_float(v.z) < 0.f;
-            neg_any |= (unsigned int)(n0 | n1) << 15;
-            pos_any |= (unsigned int)(!n0 | !n1) << 15;
-        }
-    }
-    neg_any = __reduce_or_sync(0xffffffffu, neg_any & 0x8000u);
-    pos_any = __reduce_or_sync(0xffffffffu, pos_any & 0x8000u);
-    if ((threadIdx.x & 31) == 0) S.mix[threadIdx.x >> 5] = (neg_any ? 1u : 0u) | (pos_any ? 2u : 0u);
-    __syncthreads();
-    unsigned int m = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m |= S.mix[w];
-    return m == 3u;
-}
-
-// Pass-1 work on one brick tile: row masks, cube rows, per-warp sums into
-// S.red (read after the caller's next __syncthreads).  Called by every
-// thread of the CTA.
-template <int VT, class Smem>
-__device__ __forceinline__ void classify_brick(Smem &S, const typename Vox<VT>::T *tile, int nx, int ny, int nz,
-                                               BrickPos bp) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < ROWS) RowMask<VT>::build(tile + tid * CTX, S.neg[tid], S.dead[tid]);
-        __syncthreads();
-        if (tid < CUBE_ROWS) {
-            const int cy = tid & (BY - 1), cz = tid / BY;
-            unsigned int tri = 0, occ = 0;
-            if (bp.y0 + cy < ny - 1 && bp.z0 + cz < nz - 1) {
-                const CubeRow cr = cube_row(S.neg, S.dead, cy, cz, valid_mask(bp.x0, nx));
-                occ = __popc(cr.occ);
-                unsigned int m = cr.occ;
-                while (m) {
-                    const int x = __ffs(m) - 1;
-                    m &= m - 1;
-                    tri += S.ntri[cube_index(cr, x)];
-                }
-            }
-            tri = __reduce_add_sync(0xffffffffu, tri);
-            occ = __reduce_add_sync(0xffffffffu, occ);
-            if (lane == 0) {
-                S.red[warp][0] = tri;
-                S.red[warp][1] = occ;
-            }
-        }
-}
-
-// next work item of the launch for this CTA (dynamic: CTAs take items in
-// order from a counter, so a CTA that drew cheap items takes more), -1 when
-// done; launches have fewer than 2^31 items
-__device__ __forceinline__ int next_item(unsigned int *ticket, int n) {
-    const unsigned int t = atomicAdd(ticket, 1u);
-    return t < (unsigned int)n ? (int)t : -1;
-}
-
-// the same over a 64-bit count
+// next brick of the launch for this CTA (dynamic: CTAs take them in order from
+// a counter, so a CTA that drew cheap ones takes more), -1 when done
 __device__ __forceinline__ long long next_brick(unsigned int *ticket, long long n) {
     const unsigned int t = atomicAdd(ticket, 1u);
     return (long long)t < n ? (long long)t : -1ll;
@@ -338,10 +266,10 @@ __device__ __forceinline__ bool item_mixed(Smem &S, const typename Vox<VT>::T *t
 // Persistent CTAs of NT threads take work items from a counter into a ring
 // of CSTAGES tile stages (one thread issues the loads and polls the
 // barriers with a time bound).
-template <int VT, bool TMA, int G, int XH, int CSTAGES, int NT>
+template <int VT, int G, int XH, int CSTAGES, int NT>
 __global__ void __launch_bounds__(NT)
     mc_classify_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap hmap,
-                       const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz, int nbx, int nby,
+                       int nx, int ny, int nz, int nbx, int nby,
                        int nitems, int ngx, int zbase, int zlim, uint32_t *__restrict__ brick_tris,
                        uint32_t *__restrict__ chunk, unsigned int *__restrict__ flags,
                        unsigned int *__restrict__ ticket) {
@@ -359,7 +287,7 @@ __global__ void __launch_bounds__(NT)
     // waited for here
     pdl_wait();
     // stage st's item (drawn by thread 0, which alone divides): origin into
-    // S.sorg[st] and, with TMA, its loads -- the halo box only when column
+    // S.sorg[st] and its loads -- the halo box only when column
     // x0 + TXW is inside the volume (its voxel is used by no cube otherwise)
     auto stage_item = [&](int st, int it) {
         if (it < 0) {
@@ -371,12 +299,10 @@ __global__ void __launch_bounds__(NT)
         const int y0 = (int)(r % (unsigned int)nby) * BY, z0 = (int)(r / (unsigned int)nby) * BZ + zbase;
         const int x0 = bx0 * BX;
         S.sorg[st] = make_int4(x0, y0, z0, bx0);
-        if (TMA) {
-            const bool halo = XH == 0 && x0 + Geo::TXW < nx;
-            mbar_arrive_expect_tx(&S.bars[st], (Geo::TILE + (halo ? H::N : 0)) * V::bytes);
-            tma_load_3d(S.tiles[st], &map, &S.bars[st], x0, y0, z0);
-            if (halo) tma_load_3d(S.halo[st], &hmap, &S.bars[st], x0 + Geo::TXW, y0, z0);
-        }
+        const bool halo = XH == 0 && x0 + Geo::TXW < nx;
+        mbar_arrive_expect_tx(&S.bars[st], (Geo::TILE + (halo ? H::N : 0)) * V::bytes);
+        tma_load_3d(S.tiles[st], &map, &S.bars[st], x0, y0, z0);
+        if (halo) tma_load_3d(S.halo[st], &hmap, &S.bars[st], x0 + Geo::TXW, y0, z0);
     };
     // Thread 0 draws the ticket of the next refill one iteration ahead and
     // reads it only at that refill: the counter is contended by every CTA, and
@@ -386,36 +312,22 @@ __global__ void __launch_bounds__(NT)
     unsigned int ptk = 0xffffffffu;
     if (tid == 0) {
         S.abort = 0;
-        if (TMA) {
-            for (int s = 0; s < CSTAGES; ++s) mbar_init(&S.bars[s], 1);
-            fence_barrier_init();
-            const unsigned int t0 = atomicAdd(ticket, (unsigned int)CSTAGES);
-            for (int s = 0; s < CSTAGES; ++s) stage_item(s, t0 + s < (unsigned int)nitems ? (int)(t0 + s) : -1);
-            if (t0 + CSTAGES < (unsigned int)nitems) ptk = atomicAdd(ticket, 1u);
-        }
+        for (int s = 0; s < CSTAGES; ++s) mbar_init(&S.bars[s], 1);
+        fence_barrier_init();
+        const unsigned int t0 = atomicAdd(ticket, (unsigned int)CSTAGES);
+        for (int s = 0; s < CSTAGES; ++s) stage_item(s, t0 + s < (unsigned int)nitems ? (int)(t0 + s) : -1);
+        if (t0 + CSTAGES < (unsigned int)nitems) ptk = atomicAdd(ticket, 1u);
     }
     __syncthreads();
     for (int i = 0;; ++i) {
-        const int s = TMA ? i % CSTAGES : 0;
-        if (!TMA) {
-            if (tid == 0) stage_item(0, next_item(ticket, nitems));
-            __syncthreads();
-        }
+        const int s = i % CSTAGES;
         const int4 org = S.sorg[s];
         if (org.x < 0) break;  // uniform: every thread reads the same entry
         const int x0 = org.x, y0 = org.y, z0 = org.z, bx0 = org.w;
         T *tile = reinterpret_cast<T *>(S.tiles[s]);
         T *hal = XH ? nullptr : reinterpret_cast<T *>(S.halo[s]);
-        if (TMA) {
-            // one thread polls the barrier; the others wait at __syncthreads
-            if (tid == 0 && !mbar_wait(&S.bars[s], (uint32_t)((i / CSTAGES) & 1))) S.abort = 1;
-        } else {
-            fill_tile<VT, Geo::TXW, CTY, CTZ>(tile, vol, nx, ny, nz, x0, y0, z0);
-            if (XH == 0 && tid < ROWS) {
-                const int gx = x0 + Geo::TXW, gy = y0 + tid % CTY, gz = z0 + tid / CTY;
-                hal[tid * H::HW] = (gx < nx && gy < ny && gz < nz) ? vol[lin3(nx, ny, gx, gy, gz)] : V::fill();
-            }
-        }
+        // one thread polls the barrier; the others wait at __syncthreads
+        if (tid == 0 && !mbar_wait(&S.bars[s], (uint32_t)((i / CSTAGES) & 1))) S.abort = 1;
         __syncthreads();
         if (S.abort) break;
         const bool mixed = item_mixed<VT, G, XH, NT>(S, tile, hal, nx, ny, nz, x0, y0, z0);
@@ -433,7 +345,7 @@ __global__ void __launch_bounds__(NT)
         }
         // the tile has been read for the last time: refill its stage now, so the
         // load overlaps the cube rows below
-        if (TMA && tid == 0) {
+        if (tid == 0) {
             const int it = ptk < (unsigned int)nitems ? (int)ptk : -1;
             stage_item(s, it);
             if (it >= 0) ptk = atomicAdd(ticket, 1u);
@@ -484,7 +396,7 @@ __global__ void __launch_bounds__(NT)
             }
         }
         // with one stage, the entry read at the top is the one just rewritten
-        if (!TMA || CSTAGES == 1) __syncthreads();
+        if (CSTAGES == 1) __syncthreads();
     }
     pdl_trigger();  // no more work: the scan may start its launch
     if (S.abort && tid == 0) {
@@ -537,6 +449,214 @@ struct BatchBrick {
     int pad[2];
 };
 static_assert(sizeof(BatchBrick) == 32, "two 16-byte copies");
+
+// volume of the bricks [base, end) that a warp resolved last: most bricks lie in
+// the volume of the one before and skip the search
+struct VolCache {
+    int v = -1;
+    long long base = 0, end = 0;
+};
+
+__device__ __forceinline__ int cached_volume(VolCache &c, const VolDesc *__restrict__ vols, int nvol, long long b) {
+    if (c.v < 0 || b < c.base || b >= c.end) {
+        c.v = find_volume(vols, nvol, b);
+        c.base = vols[c.v].brick_base;
+        c.end = c.base + vols[c.v].nbricks;
+    }
+    return c.v;
+}
+
+// Count pass by rows: one warp per brick, straight from global memory, for
+// volumes TMA cannot describe and for batches.  Lane x loads voxel x0 + x of
+// the brick's 9 x 9 voxel rows, nine rows ahead, and two votes give a row's
+// sign and weight-0 masks (the 33rd voxels of all rows: three more loads, lane
+// by row); most bricks lie on one side of the surface and end there, the others
+// count their cubes, two cube rows a lane.  No barrier: a warp's loads wait
+// for nothing but its own votes.  Four consecutive bricks are drawn at a time
+// (they share most of their halo, and the counter is contended), the next
+// draw in flight meanwhile.  Bound: instructions (about 11 a row), then L2
+// (every voxel is read 1.3 times).  Filling a shared-memory tile by shifted
+// 16-byte words first took 83 us for a 385 x 257 x 321 short2 volume and, with
+// TMA where it applies, 228 us for 64 volumes of 66 M voxels; this 43 and 145.
+struct RowsParams {
+    // one volume ...
+    const void *vol;
+    int nx, ny, nz, nbx, nby, zbase, zlim;
+    // ... or a batch
+    const VolDesc *vols;
+    int nvol;
+    unsigned long long *vol_sums;
+    long long nbricks;
+    uint32_t *brick_tris, *chunk;
+    unsigned int *ticket;
+    int draw;  // consecutive bricks drawn at a time
+};
+
+constexpr int RW_THREADS = 256, RW_WARPS = RW_THREADS / 32;
+
+struct RowsSmem {
+    uint2 row[RW_WARPS][ROWS];   // bits 0-31 of each row: negative, weight 0
+    unsigned char ntri[256];
+};
+
+// Row masks of the brick whose first voxel is p (this lane's: p[lane]) into row[],
+// the 33rd voxels' into en / ed (row r: bit r % 32 of word r / 32), and whether
+// a voxel inside the volume is negative, or not.  FULL: 33 x 9 x 9 voxels are
+// inside; else nx1 x ny1 x nz1 of them, the others read as weight 0.
+template <int VT, bool FULL>
+__device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T *__restrict__ p, long long sy, long long sz,
+                                          int nx1, int ny1, int nz1, unsigned int en[3], unsigned int ed[3],
+                                          unsigned int &neg_any, unsigned int &pos_any) {
+    using V = Vox<VT>;
+    using T = typename V::T;
+    const unsigned int full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned int xmask = FULL || nx1 >= 32 ? full : (1u << nx1) - 1u;
+    T e[3];
+    bool ein[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int r = lane + 32 * j, lz = r / (BY + 1), ly = r - (BY + 1) * lz;
+        ein[j] = r < ROWS && (FULL || (nx1 > BX && ly < ny1 && lz < nz1));
+        e[j] = ein[j] ? p[lz * sz + ly * sy + BX] : V::fill();
+    }
+    // planes of nine rows, the next one's loads out before this one's votes
+    auto fetch = [&](T (&w)[BY + 1], int lz) {
+        const T *q = p + lz * sz + lane;
+#pragma unroll
+        for (int ly = 0; ly < BY + 1; ++ly) {
+            w[ly] = FULL || (lane < nx1 && ly < ny1 && lz < nz1) ? *q : V::fill();
+            q += sy;
+        }
+    };
+    unsigned int any = 0, every = full;  // negative anywhere, everywhere inside
+    auto vote = [&](const T (&w)[BY + 1], int lz) {
+#pragma unroll
+        for (int ly = 0; ly < BY + 1; ++ly) {
+            const unsigned int n = __ballot_sync(full, V::neg(w[ly])), d = __ballot_sync(full, V::w0(w[ly]));
+            row[lz * (BY + 1) + ly] = make_uint2(n, d);  // (every lane the same)
+            any |= n;
+            if (FULL) every &= n;
+            else if (ly < ny1 && lz < nz1) every &= n | ~xmask;
+        }
+    };
+    T a[BY + 1], b[BY + 1];
+    fetch(a, 0);
+#pragma unroll 1
+    for (int lz = 0; lz < BZ; lz += 2) {
+        fetch(b, lz + 1);
+        vote(a, lz);
+        fetch(a, lz + 2);
+        vote(b, lz + 1);
+    }
+    vote(a, BZ);
+    pos_any = ~every;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        en[j] = __ballot_sync(full, V::neg(e[j]));
+        ed[j] = __ballot_sync(full, V::w0(e[j]));
+        any |= en[j];
+        pos_any |= __ballot_sync(full, ein[j] && !V::neg(e[j]));
+    }
+    neg_any = any;
+}
+
+// triangles and occupied cubes of the brick at (x0, y0, z0); whole warp
+template <int VT>
+__device__ __forceinline__ void count_rows(uint2 *row, const unsigned char *ntri,
+                                           const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz,
+                                           int zlim, int x0, int y0, int z0, unsigned int &tri, unsigned int &occ) {
+    const unsigned int full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const typename Vox<VT>::T *p = vol + lin3(nx, ny, x0, y0, z0);
+    const long long sy = nx, sz = (long long)nx * ny;
+    unsigned int en[3], ed[3], neg_any, pos_any;
+    if (x0 + BX < nx && y0 + BY < ny && z0 + BZ < nz)
+        load_rows<VT, true>(row, p, sy, sz, 0, 0, 0, en, ed, neg_any, pos_any);
+    else load_rows<VT, false>(row, p, sy, sz, nx - x0, ny - y0, nz - z0, en, ed, neg_any, pos_any);
+    tri = occ = 0;
+    if (!neg_any || !pos_any) return;
+    __syncwarp();
+    const unsigned int valid = valid_mask(x0, nx);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = lane + 32 * h, cy = c & (BY - 1), cz = c / BY;
+        if (y0 + cy >= ny - 1 || z0 + cz >= zlim) continue;
+        unsigned long long n[4];
+        unsigned long long dead = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = (cz + (k >> 1)) * (BY + 1) + cy + (k & 1), w = r >> 5;
+            const unsigned int e = w == 0 ? en[0] : w == 1 ? en[1] : en[2], f = w == 0 ? ed[0] : w == 1 ? ed[1] : ed[2];
+            const uint2 q = row[r];
+            n[k] = q.x | (unsigned long long)((e >> (r & 31)) & 1u) << 32;
+            dead |= q.y | (unsigned long long)((f >> (r & 31)) & 1u) << 32;
+        }
+        CubeRow cr;
+        cr.a = n[0];
+        cr.b = n[1];
+        cr.c = n[2];
+        cr.d = n[3];
+        const unsigned long long any = n[0] | n[1] | n[2] | n[3], all = n[0] & n[1] & n[2] & n[3];
+        cr.occ = (unsigned int)((any | any >> 1) & ~(all & all >> 1) & ~(dead | dead >> 1)) & valid;
+        occ += __popc(cr.occ);
+        for (unsigned int m = cr.occ; m; m &= m - 1) tri += ntri[cube_index(cr, __ffs(m) - 1)];
+    }
+    tri = __reduce_add_sync(full, tri);
+    occ = __reduce_add_sync(full, occ);
+    __syncwarp();  // the rows are rewritten by the next brick
+}
+
+template <int VT, bool BATCH>
+__global__ void __launch_bounds__(RW_THREADS, VT == MCG_VOXEL_SHORT2 ? 4 : 3) mc_count_rows_kernel(RowsParams p) {
+    using T = typename Vox<VT>::T;
+    __shared__ RowsSmem S;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c = threadIdx.x; c < 256; c += RW_THREADS) S.ntri[c] = (c == 0 || c == 255) ? 0 : g_nverts[c] / 3;
+    __syncthreads();
+    pdl_wait();
+    VolCache vc;
+    unsigned int drawn = 0;
+    if (lane == 0) drawn = atomicAdd(p.ticket, 1u);
+    for (;;) {
+        const long long b0 = (long long)__shfl_sync(0xffffffffu, drawn, 0) * p.draw;
+        if (b0 >= p.nbricks) break;
+        if (lane == 0) drawn = atomicAdd(p.ticket, 1u);
+        for (int k = 0; k < p.draw && b0 + k < p.nbricks; ++k) {
+            const long long b = b0 + k;
+            unsigned int tri, occ;
+            int v = 0;
+            if (BATCH) {
+                v = cached_volume(vc, p.vols, p.nvol, b);
+                const VolDesc &d = p.vols[v];
+                const BrickPos bp = brick_pos((unsigned int)(b - vc.base), d.nbx, d.nby);
+                count_rows<VT>(S.row[warp], S.ntri, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.nz - 1, bp.x0,
+                               bp.y0, bp.z0, tri, occ);
+            } else {
+                const unsigned int q = (unsigned int)b / (unsigned int)p.nbx, z = q / (unsigned int)p.nby;
+                count_rows<VT>(S.row[warp], S.ntri, static_cast<const T *>(p.vol), p.nx, p.ny, p.nz, p.zlim,
+                               (int)((unsigned int)b - q * (unsigned int)p.nbx) * BX,
+                               (int)(q - z * (unsigned int)p.nby) * BY, (int)z * BZ + p.zbase, tri, occ);
+            }
+            if (lane == 0) {
+                p.brick_tris[b] = tri;
+                if (tri) {
+                    uint32_t *c = p.chunk + (b / CHUNK) * CHUNK_FIELDS;
+                    atomicAdd(c + 0, tri);
+                    atomicAdd(c + 1, 1u);
+                    atomicAdd(c + 2, occ);
+                    const int hc = heavy_class(tri);
+                    if (hc >= 0) atomicAdd(c + 3 + hc, 1u);
+                    if (BATCH) {
+                        atomicAdd(&p.vol_sums[2 * v + 0], (unsigned long long)tri);
+                        atomicAdd(&p.vol_sums[2 * v + 1], (unsigned long long)occ);
+                    }
+                }
+            }
+        }
+    }
+    pdl_trigger();  // no more work: the scan may start its launch
+}
 
 // ---- scan: brick counts -> soup offsets + active brick list ---------------------
 // One CTA per chunk of CHUNK consecutive bricks.  Classify has accumulated
@@ -2247,191 +2367,6 @@ __global__ void __launch_bounds__(FGeo<FG>::NT, MINB) mc_fused_kernel(const __gr
 
 // ---- batched extraction: count and generate launches -------------------------------
 template <int VT>
-struct ClsSmemMulti {
-    static constexpr int STAGE_BYTES = pad128(CTILE * Vox<VT>::bytes);
-    unsigned char tiles[2][STAGE_BYTES];
-    unsigned long long neg[ROWS], dead[ROWS];
-    uint64_t bars[2];
-    unsigned int red[2][2];
-    unsigned int mix[CTHREADS / 32];
-    unsigned char ntri[256];
-    int svol[2];
-    int stma[2];
-    int4 spos[2];  // origin of each stage's brick
-    long long sb[2];  // brick of each stage, -1: none
-    int4 nxt;      // the brick refilled at the end of this iteration: {volume, TMA, origin x, y}
-    int nxt_z;
-    long long nxt_b;  // its brick id, or -1
-    int abort;
-};
-
-// volume of the bricks [base, end) that thread 0 resolved last: a CTA's
-// bricks are a fixed stride apart, so most lie in the same volume as the one
-// before and skip the search
-struct VolCache {
-    int v = -1;
-    long long base = 0, end = 0;
-};
-
-__device__ __forceinline__ int cached_volume(VolCache &c, const VolDesc *__restrict__ vols, int nvol, long long b) {
-    if (c.v < 0 || b < c.base || b >= c.end) {
-        c.v = find_volume(vols, nvol, b);
-        c.base = vols[c.v].brick_base;
-        c.end = c.base + vols[c.v].nbricks;
-    }
-    return c.v;
-}
-
-template <int VT>
-__device__ __forceinline__ void issue_cls_tile(ClsSmemMulti<VT> &S, int s, const VolDesc *__restrict__ vols, int nvol,
-                                               const CUtensorMap *maps, long long b, VolCache &vc) {
-    const int v = cached_volume(vc, vols, nvol, b);
-    S.svol[s] = v;
-    S.stma[s] = vols[v].tma;
-    const BrickPos bp = brick_pos(b - vc.base, vols[v].nbx, vols[v].nby);
-    S.spos[s] = make_int4(bp.x0, bp.y0, bp.z0, 0);
-    if (vols[v].tma) {
-        mbar_arrive_expect_tx(&S.bars[s], CTILE * Vox<VT>::bytes);
-        tma_load_3d(S.tiles[s], maps + v, &S.bars[s], bp.x0, bp.y0, bp.z0);
-    }
-}
-
-// Count pass over all volumes of a batch, one brick per work item, bricks
-// drawn from a counter (`ticket`, zero at launch) so that CTAs whose bricks
-// were cheap take more, 2 tile stages: TMA volumes load by TMA, so the next
-// tile loads while the current one is classified; the others are filled by
-// 16-byte words (fill_tile) when their stage is refilled.  Thread 0 draws
-// each refill's ticket one brick before it is used, so no CTA waits on the
-// counter.
-template <int VT>
-__global__ void __launch_bounds__(CTHREADS)
-    mc_classify_multi_kernel(const VolDesc *__restrict__ vols, const CUtensorMap *maps, int nvol, long long nbricks,
-                             uint32_t *__restrict__ brick_tris, uint32_t *__restrict__ chunk,
-                             unsigned long long *__restrict__ vol_sums, unsigned int *__restrict__ flags,
-                             unsigned int *__restrict__ ticket) {
-    using V = Vox<VT>;
-    using T = typename V::T;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    ClsSmemMulti<VT> &S = *reinterpret_cast<ClsSmemMulti<VT> *>(smem_raw);
-    const int tid = threadIdx.x;
-    uint32_t phase[2] = {0, 0};
-    VolCache vc;
-    long long pend = -1;  // thread 0: the brick of the next refill
-    for (int c = tid; c < 256; c += CTHREADS) S.ntri[c] = (c == 0 || c == 255) ? 0 : g_nverts[c] / 3;
-    if (tid == 0) {
-        S.abort = 0;
-        for (int s = 0; s < 2; ++s) mbar_init(&S.bars[s], 1);
-        fence_barrier_init();
-        for (int s = 0; s < 2; ++s) {
-            const long long b = (long long)atomicAdd(ticket, 1u);
-            S.sb[s] = b < nbricks ? b : -1ll;
-            if (b < nbricks) issue_cls_tile<VT>(S, s, vols, nvol, maps, b, vc);
-        }
-        pend = (long long)atomicAdd(ticket, 1u);
-    }
-    __syncthreads();
-    // the plain-copy fills of the first two stages, one copy group each
-    for (int s = 0; s < 2; ++s) {
-        if (S.sb[s] >= 0 && !S.stma[s]) {
-            const VolDesc &d = vols[S.svol[s]];
-            fill_tile<VT, CTX, CTY, CTZ, false>(reinterpret_cast<T *>(S.tiles[s]), static_cast<const T *>(d.data),
-                                                d.nx, d.ny, d.nz, S.spos[s].x, S.spos[s].y, S.spos[s].z);
-        }
-        cp_async_commit();
-    }
-    for (int i = 0;; ++i) {
-        const int s = i & 1;
-        // written by thread 0 two iterations back, barriers in between
-        const long long b = S.sb[s];
-        if (b < 0) break;  // uniform; tickets go to the stages in processing order
-        T *tile = reinterpret_cast<T *>(S.tiles[s]);
-        const int v = S.svol[s];
-        const VolDesc &d = vols[v];
-        const int4 sp = S.spos[s];
-        BrickPos bp;
-        bp.x0 = sp.x;
-        bp.y0 = sp.y;
-        bp.z0 = sp.z;
-        if (S.stma[s]) {
-            if (tid == 0) {
-                if (!mbar_wait(&S.bars[s], phase[s])) S.abort = 1;
-            }
-            phase[s] ^= 1u;
-        } else {
-            cp_async_wait_group<1>();  // this stage's group (the newest is the other stage's)
-        }
-        __syncthreads();
-        if (S.abort) break;
-        // the brick that refills this stage: resolved by thread 0 now, read by
-        // all after the barrier in tile_mixed; the ticket after it is drawn now
-        // and used at the next refill
-        if (tid == 0) {
-            const long long nbt = pend < nbricks ? pend : -1ll;
-            S.nxt_b = nbt;
-            if (nbt >= 0) {
-                const int nv = cached_volume(vc, vols, nvol, nbt);
-                const BrickPos np = brick_pos(nbt - vc.base, vols[nv].nbx, vols[nv].nby);
-                S.nxt = make_int4(nv, vols[nv].tma, np.x0, np.y0);
-                S.nxt_z = np.z0;
-                pend = (long long)atomicAdd(ticket, 1u);
-            }
-        }
-        const bool mixed = tile_mixed<VT>(S, tile);
-        const long long nb = S.nxt_b;
-        if (mixed) {
-            classify_brick<VT>(S, tile, d.nx, d.ny, d.nz, bp);
-            __syncthreads();  // tile s consumed, red[] complete
-        }
-        // tile s is free: refill it
-        if (nb >= 0) {
-            const int4 nx4 = S.nxt;
-            const int nz0 = S.nxt_z;
-            if (nx4.y) {
-                if (tid == 0) {
-                    mbar_arrive_expect_tx(&S.bars[s], CTILE * Vox<VT>::bytes);
-                    tma_load_3d(S.tiles[s], maps + nx4.x, &S.bars[s], nx4.z, nx4.w, nz0);
-                }
-            } else {
-                const VolDesc &dn = vols[nx4.x];
-                fill_tile<VT, CTX, CTY, CTZ, false>(tile, static_cast<const T *>(dn.data), dn.nx, dn.ny, dn.nz, nx4.z,
-                                                    nx4.w, nz0);
-            }
-        }
-        cp_async_commit();
-        if (tid == 0) {
-            unsigned int t = 0, o = 0;
-            if (mixed) {
-                t = S.red[0][0] + S.red[1][0];
-                o = S.red[0][1] + S.red[1][1];
-            }
-            brick_tris[b] = t;
-            if (t) {
-                uint32_t *c = chunk + (b / CHUNK) * CHUNK_FIELDS;
-                atomicAdd(c + 0, t);
-                atomicAdd(c + 1, 1u);
-                atomicAdd(c + 2, o);
-                const int hc = heavy_class(t);
-                if (hc >= 0) atomicAdd(c + 3 + hc, 1u);
-                atomicAdd(&vol_sums[2 * v + 0], (unsigned long long)t);
-                atomicAdd(&vol_sums[2 * v + 1], (unsigned long long)o);
-            }
-            S.sb[s] = nb;
-            if (nb >= 0) {
-                S.svol[s] = S.nxt.x;
-                S.stma[s] = S.nxt.y;
-                S.spos[s] = make_int4(S.nxt.z, S.nxt.w, S.nxt_z, 0);
-            }
-        }
-    }
-    cp_async_wait_all();
-    pdl_trigger();  // the scan may be scheduled (it waits for this grid's completion)
-    if (S.abort && tid == 0) {
-        atomicOr(flags, 1u);
-        for (int s = 0; s < 2; ++s) mbar_wait(&S.bars[s], phase[s], 100000000ull);
-    }
-}
-
-template <int VT>
 struct GenSmemMulti : GenSmem<VT, 1> {
     int svol;  // volume of the staged brick, -1: none
     int stma;
@@ -2613,19 +2548,30 @@ cudaError_t launch_pdl(void (*kernel)(P...), unsigned int grid, unsigned int blo
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-template <int VT, bool TMA, int G, int XH, int CSTAGES, int NT>
+template <int VT, int G, int XH, int CSTAGES, int NT>
 void launch_classify_s(const CUtensorMap &map, const CUtensorMap &hmap, const mcg_volume *vol, const Geometry &g,
                        const Scratch &sc, int sms, cudaStream_t s) {
     const size_t smem = sizeof(ClsSmemG<VT, G, XH, CSTAGES, NT>);
     static int occ = 0;  // per instantiation; all devices of a run are the same part
-    if (!occ) occ = occupancy(mc_classify_kernel<VT, TMA, G, XH, CSTAGES, NT>, NT, smem);
+    if (!occ) occ = occupancy(mc_classify_kernel<VT, G, XH, CSTAGES, NT>, NT, smem);
     const int ngx = (g.nbx + G - 1) / G;
     const long long nitems = (long long)ngx * g.nby * g.nbz;
     long long grid = (long long)sms * occ;
     if (grid > nitems) grid = nitems;
-    launch_pdl(mc_classify_kernel<VT, TMA, G, XH, CSTAGES, NT>, (unsigned int)grid, NT, smem, s, map, hmap,
-               static_cast<const typename Vox<VT>::T *>(vol->data), vol->nx, vol->ny, vol->nz, g.nbx, g.nby,
-               (int)nitems, ngx, g.zbase, g.zlim, sc.tris, sc.chunk, &sc.totals->flags, &sc.totals->cls_ticket);
+    launch_pdl(mc_classify_kernel<VT, G, XH, CSTAGES, NT>, (unsigned int)grid, NT, smem, s, map, hmap, vol->nx, vol->ny,
+               vol->nz, g.nbx, g.nby, (int)nitems, ngx, g.zbase, g.zlim, sc.tris, sc.chunk, &sc.totals->flags,
+               &sc.totals->cls_ticket);
+}
+
+template <int VT, bool BATCH>
+void launch_count_rows(RowsParams p, int sms, cudaStream_t s) {
+    static int occ = 0;
+    if (!occ) occ = occupancy(mc_count_rows_kernel<VT, BATCH>, RW_THREADS, 0);
+    const long long grid = std::min<long long>((long long)sms * occ, (p.nbricks + RW_WARPS - 1) / RW_WARPS);
+    // four bricks a draw where every warp still gets several draws
+    p.draw = p.nbricks >= grid * RW_WARPS * 16 ? 4 : 1;
+    if (BATCH) mc_count_rows_kernel<VT, BATCH><<<(unsigned int)grid, RW_THREADS, 0, s>>>(p);
+    else launch_pdl(mc_count_rows_kernel<VT, BATCH>, (unsigned int)grid, RW_THREADS, 0, s, p);
 }
 
 // classify configurations (mcg_mc_config.classify_shape):
@@ -2645,32 +2591,20 @@ void classify_shape(int nx, int eb, int c, int &G, int &XH) {
     else if (pref >= 2 && nx >= BX * 2 + XH) G = 2;
 }
 
-template <int VT, bool TMA, int G, int XH>
+template <int VT, int G, int XH>
 void launch_classify_g(const CUtensorMap &map, const CUtensorMap &hmap, const mcg_volume *vol, const Geometry &g,
                        const Scratch &sc, int sms, cudaStream_t s, int c) {
-    // without TMA only one stage is ever used
-    if constexpr (!TMA) {
-        launch_classify_s<VT, TMA, G, XH, 1, 256>(map, hmap, vol, g, sc, sms, s);
-    } else {
-        if (c == 2) launch_classify_s<VT, TMA, G, XH, 4, 512>(map, hmap, vol, g, sc, sms, s);
-        else if (c >= 4) launch_classify_s<VT, TMA, G, XH, 1, 256>(map, hmap, vol, g, sc, sms, s);
-        else launch_classify_s<VT, TMA, G, XH, 2, 256>(map, hmap, vol, g, sc, sms, s);
-    }
+    if (c == 2) launch_classify_s<VT, G, XH, 4, 512>(map, hmap, vol, g, sc, sms, s);
+    else if (c >= 4) launch_classify_s<VT, G, XH, 1, 256>(map, hmap, vol, g, sc, sms, s);
+    else launch_classify_s<VT, G, XH, 2, 256>(map, hmap, vol, g, sc, sms, s);
 }
 
 template <int VT, int XH>
-void launch_classify_x(bool tma, int G, const CUtensorMap &map, const CUtensorMap &hmap, const mcg_volume *vol,
+void launch_classify_x(int G, const CUtensorMap &map, const CUtensorMap &hmap, const mcg_volume *vol,
                        const Geometry &g, const Scratch &sc, int sms, cudaStream_t s, int c) {
-    if (G == 4) {
-        if (tma) launch_classify_g<VT, true, 4, XH>(map, hmap, vol, g, sc, sms, s, c);
-        else launch_classify_g<VT, false, 4, XH>(map, hmap, vol, g, sc, sms, s, c);
-    } else if (G == 2) {
-        if (tma) launch_classify_g<VT, true, 2, XH>(map, hmap, vol, g, sc, sms, s, c);
-        else launch_classify_g<VT, false, 2, XH>(map, hmap, vol, g, sc, sms, s, c);
-    } else {
-        if (tma) launch_classify_g<VT, true, 1, XH>(map, hmap, vol, g, sc, sms, s, c);
-        else launch_classify_g<VT, false, 1, XH>(map, hmap, vol, g, sc, sms, s, c);
-    }
+    if (G == 4) launch_classify_g<VT, 4, XH>(map, hmap, vol, g, sc, sms, s, c);
+    else if (G == 2) launch_classify_g<VT, 2, XH>(map, hmap, vol, g, sc, sms, s, c);
+    else launch_classify_g<VT, 1, XH>(map, hmap, vol, g, sc, sms, s, c);
 }
 
 template <int VT, bool TMA, int MODE = 0>
@@ -2703,22 +2637,34 @@ cudaError_t launch_count_phase(const mcg_volume *vol, const Geometry &g, const S
     bool tma = encode_volume_map(&map, vol->data, vol->nx, vol->ny, vol->nz, eb, G * BX + XH, CTY, CTZ);
     if (tma && XH == 0) tma = encode_volume_map(&hmap, vol->data, vol->nx, vol->ny, vol->nz, eb, 16 / eb, CTY, CTZ);
     else memset(&hmap, 0, sizeof(hmap));
-    if (!tma) {
-        memset(&map, 0, sizeof(map));
-        memset(&hmap, 0, sizeof(hmap));
-    }
     const bool s2 = vol->voxel_type == MCG_VOXEL_SHORT2;
     if (t0) {
         const cudaError_t et = cudaEventRecord(t0, s);
         if (et != cudaSuccess) return et;
     }
     const int c = cfg.classify_shape;
-    if (XH) {
-        if (s2) launch_classify_x<MCG_VOXEL_SHORT2, 4>(tma, G, map, hmap, vol, g, sc, sms, s, c);
-        else launch_classify_x<MCG_VOXEL_FLOAT2, 4>(tma, G, map, hmap, vol, g, sc, sms, s, c);
+    if (!tma) {
+        RowsParams p = {};
+        p.vol = vol->data;
+        p.nx = vol->nx;
+        p.ny = vol->ny;
+        p.nz = vol->nz;
+        p.nbx = g.nbx;
+        p.nby = g.nby;
+        p.zbase = g.zbase;
+        p.zlim = g.zlim;
+        p.nbricks = g.nbricks;
+        p.brick_tris = sc.tris;
+        p.chunk = sc.chunk;
+        p.ticket = &sc.totals->cls_ticket;
+        if (s2) launch_count_rows<MCG_VOXEL_SHORT2, false>(p, sms, s);
+        else launch_count_rows<MCG_VOXEL_FLOAT2, false>(p, sms, s);
+    } else if (XH) {
+        if (s2) launch_classify_x<MCG_VOXEL_SHORT2, 4>(G, map, hmap, vol, g, sc, sms, s, c);
+        else launch_classify_x<MCG_VOXEL_FLOAT2, 4>(G, map, hmap, vol, g, sc, sms, s, c);
     } else {
-        if (s2) launch_classify_x<MCG_VOXEL_SHORT2, 0>(tma, G, map, hmap, vol, g, sc, sms, s, c);
-        else launch_classify_x<MCG_VOXEL_FLOAT2, 0>(tma, G, map, hmap, vol, g, sc, sms, s, c);
+        if (s2) launch_classify_x<MCG_VOXEL_SHORT2, 0>(G, map, hmap, vol, g, sc, sms, s, c);
+        else launch_classify_x<MCG_VOXEL_FLOAT2, 0>(G, map, hmap, vol, g, sc, sms, s, c);
     }
     if (t1) {
         const cudaError_t et = cudaEventRecord(t1, s);
@@ -3178,7 +3124,7 @@ namespace {
 
 // Device table layout: [VolDesc x nvol][pad to 64][classify maps x nvol][generate maps x nvol]
 size_t btab_desc_bytes(int nvol) { return ((sizeof(VolDesc) * (size_t)nvol + 63) / 64) * 64; }
-size_t btab_bytes(int nvol) { return btab_desc_bytes(nvol) + 2 * sizeof(CUtensorMap) * (size_t)nvol; }
+size_t btab_bytes(int nvol) { return btab_desc_bytes(nvol) + sizeof(CUtensorMap) * (size_t)nvol; }
 
 // staging slot k of at least n bytes; its last copy has completed
 mcg_status grow_pinned(mcg_context *ctx, int k, size_t n) {
@@ -3260,8 +3206,7 @@ mcg_status upload_btab(mcg_context *ctx, const mcg_volume *vols, const mcg_mesh_
         return MCG_ERR_STATE;
     }
     VolDesc *desc = reinterpret_cast<VolDesc *>(hb);
-    CUtensorMap *cmaps = reinterpret_cast<CUtensorMap *>(hb + btab_desc_bytes(nvol));
-    CUtensorMap *gmaps = cmaps + nvol;
+    CUtensorMap *gmaps = reinterpret_cast<CUtensorMap *>(hb + btab_desc_bytes(nvol));
     long long base = 0;
     const int eb = vols[0].voxel_type == MCG_VOXEL_SHORT2 ? 4 : 8;
     for (int v = 0; v < nvol; ++v) {
@@ -3286,18 +3231,12 @@ mcg_status upload_btab(mcg_context *ctx, const mcg_volume *vols, const mcg_mesh_
             d.tri_cube = outs[v].tri_cube;
             d.cap = outs[v].capacity_vertices;
         }
-        // TMA only when both boxes can be described (the flag serves both
-        // passes); the maps are encoded and copied with the count phase's
-        // table, the generate phase's table carries the flags it recorded
+        // the generate launch's maps are encoded and copied with the count
+        // phase's table, the generate phase's table carries the flags it recorded
         if (with_maps) {
-            const bool tc =
-                encode_volume_map(&cmaps[v], vols[v].data, vols[v].nx, vols[v].ny, vols[v].nz, eb, CTX, CTY, CTZ);
             const bool tg = encode_volume_map(&gmaps[v], vols[v].data, vols[v].nx, vols[v].ny, vols[v].nz, eb, TX, TY, TZ);
-            ctx->batch_tma[v] = tc && tg ? 1 : 0;
-            if (!ctx->batch_tma[v]) {
-                memset(&cmaps[v], 0, sizeof(CUtensorMap));
-                memset(&gmaps[v], 0, sizeof(CUtensorMap));
-            }
+            ctx->batch_tma[v] = tg ? 1 : 0;
+            if (!tg) memset(&gmaps[v], 0, sizeof(CUtensorMap));
         }
         d.tma = ctx->batch_tma[v];
     }
@@ -3318,16 +3257,15 @@ MeshTotals *batch_host(mcg_context *ctx) {
 
 template <int VT>
 void launch_classify_multi(mcg_context *ctx, int nvol, long long nbricks, cudaStream_t s) {
-    const size_t smem = sizeof(ClsSmemMulti<VT>);
-    static int occ = 0;
-    if (!occ) occ = occupancy(mc_classify_multi_kernel<VT>, CTHREADS, smem);
-    long long grid = (long long)ctx->num_sms * occ;
-    if (grid > nbricks) grid = nbricks;
-    const VolDesc *desc = reinterpret_cast<const VolDesc *>(ctx->d_btab);
-    const CUtensorMap *cmaps = reinterpret_cast<const CUtensorMap *>(ctx->d_btab + btab_desc_bytes(nvol));
-    mc_classify_multi_kernel<VT><<<(int)grid, CTHREADS, smem, s>>>(desc, cmaps, nvol, nbricks, ctx->brick_tris,
-                                                                    ctx->brick_occ, ctx->d_vol_sums,
-                                                                    &ctx->d_totals->flags, &ctx->d_totals->cls_ticket);
+    RowsParams p = {};
+    p.vols = reinterpret_cast<const VolDesc *>(ctx->d_btab);
+    p.nvol = nvol;
+    p.vol_sums = ctx->d_vol_sums;
+    p.nbricks = nbricks;
+    p.brick_tris = ctx->brick_tris;
+    p.chunk = ctx->brick_occ;
+    p.ticket = &ctx->d_totals->cls_ticket;
+    launch_count_rows<VT, true>(p, ctx->num_sms, s);
 }
 
 // generate launch of a batch, chained to the batch's scan (programmatic
@@ -3341,7 +3279,7 @@ cudaError_t launch_generate_multi(mcg_context *ctx, int nvol, long long nbricks,
     if (!occ) occ = occupancy(mc_generate_multi_kernel<VT>, THREADS, smem);
     long long grid = (long long)ctx->num_sms * occ;
     if (grid > nbricks) grid = nbricks;
-    const CUtensorMap *gmaps = reinterpret_cast<const CUtensorMap *>(ctx->d_btab + btab_desc_bytes(nvol)) + nvol;
+    const CUtensorMap *gmaps = reinterpret_cast<const CUtensorMap *>(ctx->d_btab + btab_desc_bytes(nvol));
     return launch_pdl(mc_generate_multi_kernel<VT>, (unsigned int)grid, THREADS, smem, s, desc, gmaps, nvol, list,
                       ctx->d_totals, batch_host(ctx));
 }

@@ -107,7 +107,7 @@ struct mcg_context {
     uint32_t *idx_cand = nullptr;     // indexed: bricks whose owned edges are counted
     size_t idx_cand_cap = 0;
 
-    // batched extraction: device tables (volume descriptors, classify and
+    // batched extraction: device tables (volume descriptors and
     // generate tensor maps), pinned staging for them, per-volume sums
     unsigned char *d_btab = nullptr;
     size_t d_btab_cap = 0;
@@ -125,7 +125,7 @@ struct mcg_context {
     std::vector<unsigned char *> btab_spare;
     size_t btab_spare_cap = 0;
     std::vector<unsigned char *> btab_kept;
-    unsigned char *batch_tma = nullptr;  // per volume of the classified batch: both boxes encodable
+    unsigned char *batch_tma = nullptr;  // per volume of the classified batch: its tile box encodable
     size_t batch_tma_cap = 0;
     unsigned long long *d_vol_sums = nullptr;
     size_t d_vol_sums_cap = 0;
