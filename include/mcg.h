@@ -263,6 +263,10 @@ mcg_status mcg_mc_normals(mcg_context *ctx, const mcg_volume *vol, const mcg_ver
  * cases is zero almost everywhere).  FP32 accumulation with atomics. */
 mcg_status mcg_mc_backward(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
                            float *grad_f, mcg_stream_t stream);
+/* The same for FLOAT2 volumes, accumulated into the tsdf channel of a
+ * gradient laid out as the volume (2 floats per voxel). */
+mcg_status mcg_mc_backward_volume(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
+                                  float *grad_vol, mcg_stream_t stream);
 
 /* ---- depth maps: kf.cu:99-151 (d_kinect_depth_to_meter, d_img_meter_to_vertex,
  * d_img_vertex_to_normal), fused --------------------------------------------- */
@@ -316,6 +320,14 @@ mcg_status mcg_integrate_backward(mcg_context *ctx, const void *vol0, int32_t nx
                                   const float *normals, int32_t is_dynamic, const float *grad_f,
                                   const float *grad_w, float *grad_depth, float *grad_f0, float *grad_w0,
                                   mcg_stream_t stream);
+/* The same with dL/dtsdf and dL/dweight in one array laid out as the volume
+ * (nx*ny*nz pairs). */
+mcg_status mcg_integrate_backward_volume(mcg_context *ctx, const void *vol0, int32_t nx, int32_t ny, int32_t nz,
+                                         float min_t, float max_t, float grid_s, const mcg_intrinsic *k,
+                                         int32_t n_frames, const float *poses_dev, int32_t w, int32_t h,
+                                         const float *depth_m, const float *normals, int32_t is_dynamic,
+                                         const float *grad_vol, float *grad_depth, float *grad_f0, float *grad_w0,
+                                         mcg_stream_t stream);
 
 /* ---- ray casting: kf.cu:786-986 (_cu_voxel_extract_depth_and_normal_map) */
 /* Depth (metres, z-depth; 0 where the ray finds no zero crossing) and, if

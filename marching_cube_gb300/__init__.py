@@ -717,6 +717,13 @@ def integrate_backward(shape, min_t, max_t, grid_s, k, poses, depth, grad_f, gra
     (grad_depth, grad_f0, grad_w0); the last two are None unless
     want_grad_vol0.  Pixel choices, truncation and clamping are held fixed;
     normal maps are constants."""
+    return _integrate_backward(shape, min_t, max_t, grid_s, k, poses, depth, grad_f, grad_w, vol0, normals, is_dynamic,
+                               grad_depth, want_grad_vol0, ctx, stream)
+
+
+def _integrate_backward(shape, min_t, max_t, grid_s, k, poses, depth, grad_f, grad_w, vol0, normals, is_dynamic,
+                        grad_depth, want_grad_vol0, ctx, stream, grad_vol=None):
+    """integrate_backward, or with both gradients in grad_vol (nz, ny, nx, 2)."""
     nz, ny, nx = shape
     dev = depth.device
     ctx = ctx or default_context(dev.index)
@@ -727,16 +734,28 @@ def integrate_backward(shape, min_t, max_t, grid_s, k, poses, depth, grad_f, gra
         raise ValueError("one pose per depth frame")
     if grad_depth is None:
         grad_depth = torch.zeros_like(depth)
-    gf = grad_f.to(torch.float32).contiguous()
-    gw = grad_w.to(torch.float32).contiguous() if grad_w is not None else None
-    if gf.numel() != nx * ny * nz or (gw is not None and gw.numel() != nx * ny * nz):
-        raise ValueError("grad_f / grad_w must hold one value per voxel")
+    if grad_vol is not None:
+        gv = grad_vol.to(torch.float32).contiguous()
+        if gv.numel() != 2 * nx * ny * nz:
+            raise ValueError("grad_vol must hold two values per voxel")
+    else:
+        gf = grad_f.to(torch.float32).contiguous()
+        gw = grad_w.to(torch.float32).contiguous() if grad_w is not None else None
+        if gf.numel() != nx * ny * nz or (gw is not None and gw.numel() != nx * ny * nz):
+            raise ValueError("grad_f / grad_w must hold one value per voxel")
     if vol0 is not None:
         if vol0.dtype != torch.float32 or tuple(vol0.shape) != (nz, ny, nx, 2) or not vol0.is_contiguous():
             raise ValueError("vol0 must be a contiguous float32 (nz, ny, nx, 2) tensor")
     nrm = normals.to(torch.float32).contiguous() if normals is not None else None
     gf0 = torch.empty((nz, ny, nx), dtype=torch.float32, device=dev) if want_grad_vol0 else None
     gw0 = torch.empty((nz, ny, nx), dtype=torch.float32, device=dev) if want_grad_vol0 else None
+    if grad_vol is not None:
+        ctx.check(_lib.mcg_integrate_backward_volume(ctx.handle, _ptr(vol0), nx, ny, nz, min_t, max_t, grid_s,
+                                                     ctypes.byref(k), nf, _ptr(pt), w, h, _ptr(depth), _ptr(nrm),
+                                                     1 if is_dynamic else 0, _ptr(gv), _ptr(grad_depth), _ptr(gf0),
+                                                     _ptr(gw0), _stream(stream)),
+                  "mcg_integrate_backward_volume")
+        return grad_depth, gf0, gw0
     ctx.check(_lib.mcg_integrate_backward(ctx.handle, _ptr(vol0), nx, ny, nz, min_t, max_t, grid_s, ctypes.byref(k),
                                           nf, _ptr(pt), w, h, _ptr(depth), _ptr(nrm), 1 if is_dynamic else 0,
                                           _ptr(gf), _ptr(gw), _ptr(grad_depth), _ptr(gf0), _ptr(gw0),
@@ -765,8 +784,13 @@ class MarchingCubesFunction(torch.autograd.Function):
             return None, None
         gv = torch.zeros_like(volume)
         if grad_pos.shape[0]:
-            gf = mc_backward(volume, fctx.cell, grad_pos)
-            gv[..., 0] = gf
+            grad_pos = grad_pos.to(torch.float32).contiguous()
+            ctx = default_context(volume.device.index)
+            cv = _cvol(volume, fctx.cell)
+            s = _stream()
+            ctx.check(_lib.mcg_mc_classify(ctx.handle, ctypes.byref(cv), s), "mcg_mc_classify")
+            ctx.check(_lib.mcg_mc_backward_volume(ctx.handle, ctypes.byref(cv), _ptr(grad_pos), grad_pos.shape[0],
+                                                  _ptr(gv), s), "mcg_mc_backward_volume")
         return gv, None
 
 
@@ -805,11 +829,10 @@ class IntegrateFunction(torch.autograd.Function):
     def backward(fctx, grad_vol):
         depth, pt, vol0, nrm = fctx.saved_tensors
         shape, min_t, max_t, grid_s, k, is_dynamic = fctx.params
-        grad_vol = grad_vol.contiguous()
         want0 = vol0 is not None and fctx.needs_input_grad[1]
-        gd, gf0, gw0 = integrate_backward(shape, min_t, max_t, grid_s, k, pt, depth, grad_vol[..., 0], grad_vol[..., 1],
-                                          vol0=vol0.detach().contiguous() if vol0 is not None else None,
-                                          normals=nrm, is_dynamic=is_dynamic, want_grad_vol0=want0)
+        gd, gf0, gw0 = _integrate_backward(shape, min_t, max_t, grid_s, k, pt, depth, None, None,
+                                           vol0.detach().contiguous() if vol0 is not None else None, nrm, is_dynamic,
+                                           None, want0, None, None, grad_vol=grad_vol)
         g0 = torch.stack([gf0, gw0], dim=-1) if want0 else None
         return (gd if fctx.needs_input_grad[0] else None), g0, None, None, None, None, None, None, None, None
 

@@ -92,6 +92,7 @@ SIGNATURES = {
     "mcg_mc_extract_noalloc": (c_int, [ctypes.POINTER(Volume), ctypes.POINTER(MeshOut),
                                        ctypes.POINTER(MeshCounts), c_void_p]),
     "mcg_mc_backward": (c_int, [c_void_p, ctypes.POINTER(Volume), c_void_p, c_int64, c_void_p, c_void_p]),
+    "mcg_mc_backward_volume": (c_int, [c_void_p, ctypes.POINTER(Volume), c_void_p, c_int64, c_void_p, c_void_p]),
     "mcg_mc_normals": (c_int, [c_void_p, ctypes.POINTER(Volume), c_void_p, c_int64, c_void_p, c_void_p]),
     "mcg_depth_to_maps": (c_int, [c_void_p, ctypes.POINTER(Intrinsic), c_int32, c_int32, c_void_p,
                                   c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
@@ -107,6 +108,9 @@ SIGNATURES = {
                                        ctypes.POINTER(Intrinsic), c_int32, c_void_p, c_int32, c_int32, c_void_p,
                                        c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p]),
+    "mcg_integrate_backward_volume": (c_int, [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_float, c_float, c_float,
+                                              ctypes.POINTER(Intrinsic), c_int32, c_void_p, c_int32, c_int32, c_void_p,
+                                              c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "mcg_integrate_device_pose": (c_int, [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_float, c_float,
                                           c_float, ctypes.POINTER(Intrinsic), c_void_p, c_int32, c_int32, c_void_p,
                                           c_void_p, c_int32, c_void_p]),

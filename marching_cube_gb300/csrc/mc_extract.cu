@@ -874,6 +874,7 @@ struct GenParams {
     // adjoint (MODE 1): dL/dP per soup vertex in, dL/df per voxel accumulated
     const float *grad_pos;
     float *grad_f;
+    int grad_step;  // voxel i's at i * grad_step
     long long n_grad;
 };
 
@@ -1573,7 +1574,7 @@ __device__ __forceinline__ void backward_brick(Smem &S, const typename Vox<VT>::
                                                int nz, int zlim, float cell, int x0, int y0, int z0,
                                                unsigned long long vbase,
                                                const float *__restrict__ grad_pos, float *__restrict__ grad_f,
-                                               long long n_grad) {
+                                               int grad_step, long long n_grad) {
     using V = Vox<VT>;
     const int tid = threadIdx.x;
     occupied_list<VT>(S, tile, nx, ny, zlim, x0, y0, z0);
@@ -1615,8 +1616,8 @@ __device__ __forceinline__ void backward_brick(Smem &S, const typename Vox<VT>::
         }
         const float D = f1 - f0 + 1e-15f;
         const float inv = 1.0f / (D * D);
-        atomicAdd(&grad_f[lin3(nx, ny, ga[0], ga[1], ga[2])], g * (-(f1 + 1e-15f) * inv));
-        atomicAdd(&grad_f[lin3(nx, ny, gb[0], gb[1], gb[2])], g * (f0 * inv));
+        atomicAdd(&grad_f[lin3(nx, ny, ga[0], ga[1], ga[2]) * grad_step], g * (-(f1 + 1e-15f) * inv));
+        atomicAdd(&grad_f[lin3(nx, ny, gb[0], gb[1], gb[2]) * grad_step], g * (f0 * inv));
     }
 }
 
@@ -1763,7 +1764,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
             }
         } else {
             backward_brick<VT>(S, tile, nx, ny, nz, p.zlim, cell, bp.x0, bp.y0, bp.z0, vbase, p.grad_pos,
-                               p.grad_f, p.n_grad);
+                               p.grad_f, p.grad_step, p.n_grad);
             __syncthreads();
             refill();
         }
@@ -3055,8 +3056,8 @@ mcg_status mcg_mc_normals(mcg_context *ctx, const mcg_volume *vol, const mcg_ver
 
 
 
-mcg_status mcg_mc_backward(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
-                           float *grad_f, mcg_stream_t stream) {
+static mcg_status mc_backward_impl(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
+                                   float *grad_f, int grad_step, mcg_stream_t stream) {
     if (!ctx || !vol_ok(vol) || n_vertices < 0 || !grad_f || (n_vertices > 0 && !grad_pos))
         return MCG_ERR_INVALID_ARG;
     if (!ctx->classified || ctx->cls_indexed || ctx->cls_fused || ctx->cls_data != vol->data ||
@@ -3088,6 +3089,7 @@ mcg_status mcg_mc_backward(mcg_context *ctx, const mcg_volume *vol, const float 
     p.fixed_rounds = (unsigned int)ctx->mc_cfg.gen_fixed_rounds;
     p.grad_pos = grad_pos;
     p.grad_f = grad_f;
+    p.grad_step = grad_step;
     p.n_grad = n_vertices;
     CUtensorMap map;
     const int eb = vol->voxel_type == MCG_VOXEL_SHORT2 ? 4 : 8;
@@ -3102,6 +3104,17 @@ mcg_status mcg_mc_backward(mcg_context *ctx, const mcg_volume *vol, const float 
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? MCG_OK : mcg_cuda_fail(ctx, e);
+}
+
+mcg_status mcg_mc_backward(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
+                           float *grad_f, mcg_stream_t stream) {
+    return mc_backward_impl(ctx, vol, grad_pos, n_vertices, grad_f, 1, stream);
+}
+
+mcg_status mcg_mc_backward_volume(mcg_context *ctx, const mcg_volume *vol, const float *grad_pos, int64_t n_vertices,
+                                  float *grad_vol, mcg_stream_t stream) {
+    if (vol && vol->voxel_type != MCG_VOXEL_FLOAT2) return MCG_ERR_INVALID_ARG;
+    return mc_backward_impl(ctx, vol, grad_pos, n_vertices, grad_vol, 2, stream);
 }
 
 // Zeroes what a batch's count launch accumulates into: the flags, the count
