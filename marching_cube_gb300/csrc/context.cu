@@ -125,6 +125,7 @@ mcg_status mcg_destroy(mcg_context *ctx) {
     cudaFree(ctx->integ_blocks);
     cudaFree(ctx->integ_tiles);
     cudaFree(ctx->integ_count);
+    for (void *b : ctx->integ_old) cudaFree(b);
     for (const auto &r : ctx->ray_x) cudaFree(r.d);
     cudaFree(ctx->tr_text);
     cudaFree(ctx->tr_tok);

@@ -673,6 +673,16 @@ __global__ void __launch_bounds__(BW_THREADS) integrate_backward_kernel(IntegBwP
 
 Intr intr_of(const mcg_intrinsic *k) { return Intr{k->fx, k->fy, k->cx, k->cy}; }
 
+// ensure() for integrate's scratch: what a captured graph may refer to is not freed
+template <class T>
+bool ensure_integ(mcg_context *ctx, T **ptr, size_t *cap, size_t n) {
+    if (*cap < n && *ptr && ctx->integ_captured) {
+        ctx->integ_old.push_back(*ptr);
+        *ptr = nullptr;
+    }
+    return ensure(ptr, cap, n);
+}
+
 }  // namespace
 }  // namespace mcg
 
@@ -813,10 +823,13 @@ static mcg_status integrate_impl(mcg_context *ctx, void *vol, int32_t voxel_type
     const size_t ntiles = (size_t)2 * g2.x * g2.y;
     // inside a stream capture nothing may be allocated: an earlier call of
     // the same shapes outside the capture has sized every buffer
-    if (mcg_capturing(s) && (ctx->depth_scaled_cap < (size_t)w * h || ctx->integ_blocks_cap < (size_t)nblocks ||
-                             ctx->integ_tiles_cap < ntiles || ctx->integ_count_cap < 1))
-        return MCG_ERR_STATE;
-    if (!ensure(&ctx->depth_scaled, &ctx->depth_scaled_cap, (size_t)w * h))
+    if (mcg_capturing(s)) {
+        if (ctx->depth_scaled_cap < (size_t)w * h || ctx->integ_blocks_cap < (size_t)nblocks ||
+            ctx->integ_tiles_cap < ntiles || ctx->integ_count_cap < 1)
+            return MCG_ERR_STATE;
+        ctx->integ_captured = true;
+    }
+    if (!ensure_integ(ctx, &ctx->depth_scaled, &ctx->depth_scaled_cap, (size_t)w * h))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     const float *ray_x = nullptr;
     {
@@ -835,8 +848,8 @@ static mcg_status integrate_impl(mcg_context *ctx, void *vol, int32_t voxel_type
     p.normals = (const float3 *)normals;
     p.ray_x = ray_x;
     p.is_dynamic = is_dynamic ? 1 : 0;
-    if (!ensure(&ctx->integ_blocks, &ctx->integ_blocks_cap, (size_t)nblocks) ||
-        !ensure(&ctx->integ_tiles, &ctx->integ_tiles_cap, ntiles) ||
+    if (!ensure_integ(ctx, &ctx->integ_blocks, &ctx->integ_blocks_cap, (size_t)nblocks) ||
+        !ensure_integ(ctx, &ctx->integ_tiles, &ctx->integ_tiles_cap, ntiles) ||
         !ensure(&ctx->integ_count, &ctx->integ_count_cap, (size_t)1))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     p.tiles = ctx->integ_tiles;

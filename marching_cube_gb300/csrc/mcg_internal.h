@@ -198,6 +198,10 @@ struct mcg_context {
     size_t integ_tiles_cap = 0;
     unsigned int *integ_count = nullptr;  // blocks listed
     size_t integ_count_cap = 0;
+    // a stream capture has recorded this scratch: buffers outgrown afterwards
+    // are kept here until the context goes, since graphs may still use them
+    bool integ_captured = false;
+    std::vector<void *> integ_old;
     // x coordinates of the voxel centres as the reference accumulates them
     // (p.x += grid_s per voxel), one device table per (nx, grid_s) seen on
     // this context, built once and never rewritten, so the calls on several

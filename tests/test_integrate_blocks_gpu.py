@@ -58,3 +58,37 @@ def test_blocks_keep_every_update(mcg, orc, dims, image, vtype):
     assert np.array_equal(got.view(bits)[~none], ref.view(bits)[~none])
     if w > 2:
         assert (ref[..., 1] != 0).any()
+
+
+def test_captured_integrate_outlives_larger_calls(mcg, orc):
+    """A graph captured around a small volume's integrate still works after
+    calls for a larger volume and image have outgrown the context's scratch."""
+    rng = np.random.default_rng(7)
+    k, ko = mcg.intrinsic(40.0, 40.0, 23.5, 17.5), orc.intrinsic(40.0, 40.0, 23.5, 17.5)
+    v = mcg.voxel_new((32, 32, 32), 0.08, 0.08, 1.0 / 32)
+    R, t = np.eye(3), np.array([0.5, 0.5, -0.6])
+    pose = mcg.extrinsic_tensor(R, t)
+    m = torch.zeros((36, 48), device="cuda")
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        mcg.volumetric_integration_device_pose(v, k, pose, m, None)  # no valid pixel: sizes the scratch only
+        st.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            mcg.volumetric_integration_device_pose(v, k, pose, m, None)
+    big = mcg.voxel_new((96, 80, 72), 0.03, 0.03, 1.0 / 96)
+    kb = mcg.intrinsic(200.0, 200.0, 99.5, 79.5)
+    mcg.volumetric_integration(big, kb, mcg.extrinsic(R, t), torch.full((160, 200), 1.0, device="cuda"), None)
+    torch.cuda.synchronize()
+    other = [torch.full((1 << 16,), 7, dtype=torch.int32, device="cuda") for _ in range(16)]
+    ref = v.data.cpu().numpy().copy()
+    for _ in range(2):
+        d = rng.uniform(0.7, 1.4, (36, 48)).astype(np.float32)
+        m.copy_(torch.from_numpy(d))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        orc.integrate(ref, 0.08, 0.08, 1.0 / 32, ko, orc.extrinsic(R, t), d, None)
+    assert (ref[..., 1] != 0).any()
+    assert np.array_equal(v.data.cpu().numpy(), ref)
+    assert all(bool((o == 7).all()) for o in other)
