@@ -301,6 +301,13 @@ mcg_status mcg_integrate_device_pose(mcg_context *ctx, void *vol, int32_t voxel_
                                      const float *pose_dev, int32_t w, int32_t h, const float *depth_m,
                                      const float *normals, int32_t is_dynamic, mcg_stream_t stream);
 
+/* n_frames such updates, one after another: poses_dev, depth_m and normals hold
+ * the frames' 12 floats, h x w metres and h x w float3 in turn. */
+mcg_status mcg_integrate_frames(mcg_context *ctx, void *vol, int32_t voxel_type, int32_t nx, int32_t ny, int32_t nz,
+                                float min_t, float max_t, float grid_s, const mcg_intrinsic *k, int32_t n_frames,
+                                const float *poses_dev, int32_t w, int32_t h, const float *depth_m,
+                                const float *normals, int32_t is_dynamic, mcg_stream_t stream);
+
 /* Adjoint of n_frames integrate steps on a FLOAT2 volume (no counterpart in
  * the reference; the forward is kf.cu:427-532 as mcg_integrate computes it).
  * vol0: the volume before the first frame (nx*ny*nz float2), or NULL for the

@@ -801,6 +801,26 @@ def mesh_positions(volume, cell):
     return MarchingCubesFunction.apply(volume, cell)
 
 
+def _integrate_frames(v: Voxel, k, pt, depth, normals, is_dynamic):
+    """volumetric_integration_device_pose of depth (K, h, w) with poses pt
+    (K, 12) and normals (K, h, w, 3) or None, one frame after another."""
+    vt = _check_volume(v.data)
+    nf, h, w = depth.shape
+    if pt.shape[0] < nf or (normals is not None and normals.shape[0] < nf):
+        raise IndexError("one pose and one normal map per depth frame")
+    if normals is not None and normals[:nf].numel() != 3 * nf * h * w:
+        # each frame takes the first h * w of its own map
+        normals = normals[:nf].reshape(nf, -1)[:, :3 * h * w].contiguous()
+        if normals.shape[1] != 3 * h * w:
+            raise ValueError("normals must be (K, h, w, 3)")
+    nx, ny, nz = v.size
+    ctx = default_context(v.data.device.index)
+    ctx.check(_lib.mcg_integrate_frames(ctx.handle, _ptr(v.data), vt, nx, ny, nz, v.min_t, v.max_t, v.grid_s,
+                                        ctypes.byref(k), nf, _ptr(pt), w, h, _ptr(depth), _ptr(normals),
+                                        1 if is_dynamic else 0, _stream()),
+              "mcg_integrate_frames")
+
+
 class IntegrateFunction(torch.autograd.Function):
     """depth frames (K, h, w) [+ initial volume] -> float32 volume
     (nz, ny, nx, 2) after integrating every frame in order."""
@@ -818,9 +838,8 @@ class IntegrateFunction(torch.autograd.Function):
             voxel_init(vol)
         v = Voxel(vol, min_t, max_t, grid_s)
         nrm = normals.to(torch.float32).contiguous() if normals is not None else None
-        for f in range(depth_c.shape[0]):
-            volumetric_integration_device_pose(v, k, pt[f], depth_c[f], None if nrm is None else nrm[f],
-                                               is_dynamic)
+        if depth_c.shape[0]:
+            _integrate_frames(v, k, pt, depth_c, nrm, is_dynamic)
         fctx.save_for_backward(depth_c, pt, vol0 if vol0 is not None else None, nrm)
         fctx.params = (tuple(shape), min_t, max_t, grid_s, k, is_dynamic)
         return vol

@@ -123,6 +123,7 @@ mcg_status mcg_destroy(mcg_context *ctx) {
     cudaFree(ctx->icp_inlier);
     cudaFree(ctx->depth_scaled);
     cudaFree(ctx->integ_blocks);
+    cudaFree(ctx->integ_masks);
     cudaFree(ctx->integ_tiles);
     cudaFree(ctx->integ_count);
     for (void *b : ctx->integ_old) cudaFree(b);

@@ -194,6 +194,8 @@ struct mcg_context {
     size_t depth_scaled_cap = 0;
     unsigned int *integ_blocks = nullptr;  // blocks of 8^3 voxels that the frame can update
     size_t integ_blocks_cap = 0;
+    unsigned int *integ_masks = nullptr;  // and which of several frames, one bit each
+    size_t integ_masks_cap = 0;
     float *integ_tiles = nullptr;  // largest valid ray-length depth per tile of pixels
     size_t integ_tiles_cap = 0;
     unsigned int *integ_count = nullptr;  // blocks listed

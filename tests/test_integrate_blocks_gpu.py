@@ -92,3 +92,36 @@ def test_captured_integrate_outlives_larger_calls(mcg, orc):
     assert (ref[..., 1] != 0).any()
     assert np.array_equal(v.data.cpu().numpy(), ref)
     assert all(bool((o == 7).all()) for o in other)
+
+
+@pytest.mark.parametrize("vtype", [torch.int16, torch.float32])
+@pytest.mark.parametrize("frames,with_normals", [(1, False), (2, True), (9, False), (33, True), (66, False)])
+@pytest.mark.parametrize("dims,image", [((9, 7, 17), (33, 25)), ((32, 24, 40), (48, 32))])
+def test_several_frames_in_one_pass(mcg, orc, dims, image, frames, with_normals, vtype):
+    """Up to 32 frames go through the volume in one pass: equal to the
+    oracle's frame by frame, at either side of 32 and with a remainder of 1."""
+    rng = np.random.default_rng(sum(dims) + frames)
+    (w, h), gs = image, 1.0 / max(dims)
+    trunc, f = 2.5 * gs, 0.9 * image[0]
+    k, ko = mcg.intrinsic(f, f, (w - 1) / 2.0, (h - 1) / 2.0), orc.intrinsic(f, f, (w - 1) / 2.0, (h - 1) / 2.0)
+    v = mcg.voxel_new(dims, trunc, trunc, gs, dtype=vtype)
+    ref = v.data.cpu().numpy().copy()
+    middle = np.array(dims) * gs / 2
+    poses = []
+    for i in range(frames):
+        eye = middle + rng.uniform(-1, 1, 3) * (1.2, 0.3, 0.55)[i % 3]
+        poses.append((_look_at(eye, middle + rng.uniform(-0.2, 0.2, 3)), eye))
+    m = rng.uniform(0.1, 1.6, (frames, h, w)).astype(np.float32)
+    m[rng.random(m.shape) < 0.3] = 0.0
+    n = rng.standard_normal((frames, h, w, 3)).astype(np.float32)
+    n[..., 2] = -np.abs(n[..., 2]) - 0.5
+    n /= np.linalg.norm(n, axis=-1, keepdims=True)
+    pt = torch.stack([mcg.extrinsic_tensor(R, t) for R, t in poses]).contiguous()
+    dyn = frames % 2 == 0
+    mcg._integrate_frames(v, k, pt, torch.from_numpy(m).cuda(), torch.from_numpy(n).cuda() if with_normals else None,
+                          dyn)
+    for i, (R, t) in enumerate(poses):
+        orc.integrate(ref, trunc, trunc, gs, ko, orc.extrinsic(R, t), m[i], n[i] if with_normals else None,
+                      is_dynamic=dyn)
+    assert np.array_equal(v.data.cpu().numpy(), ref)
+    assert (ref[..., 1] != 0).any()
