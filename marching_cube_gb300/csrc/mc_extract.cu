@@ -1244,7 +1244,9 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
 // soup vertex for itself took 578 warp-instructions per 32 soup vertices, this
 // about 400: 512^3 with 1.2 M triangles 100 -> 82 us, 1024^3 with 19 M 1373 ->
 // 1079 us, 64 volumes with 2.7 M 281 -> 204 us (there also with one tile stage
-// and four CTAs per SM instead of two stages).  Returns false (the caller
+// and four CTAs per SM instead of two stages).  Warps wait for barriers more
+// than for anything else: with up to three cubes a thread in step 2, one scan
+// and two barriers instead of those per 256 cubes, 79 and 1061 us.  Returns false (the caller
 // runs generate_brick) where a layer or its records do not fit, or the output
 // ends inside the brick; else tile_done() has been called by every thread
 // between the last use of the tile and the last copy, so that the next brick's
@@ -1400,44 +1402,55 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
     // 2. cases and soup offsets of the cubes, and the slots of the whole brick
     unsigned int T_brick = 0;
     int R = 0;
-    for (unsigned int i0 = 0; i0 < nocc; i0 += THREADS) {
-        const unsigned int i = i0 + tid;
-        unsigned int c = 0, nv = 0;
-        if (i < nocc) {
-            // the last row with rowcube <= i is the cube's, and it is the (i - rowcube)-th there
-            unsigned int row = 0;
+    {
+        constexpr int PER = SH_CUBES / THREADS;
+        const unsigned int per = (nocc + THREADS - 1) / THREADS, i0 = tid * per;
+        unsigned int c[PER], nv[PER], incl = 0;
 #pragma unroll
-            for (int h = CUBE_ROWS / 2; h; h >>= 1)
-                if (S.rowcube[row + h] <= i) row += h;
-            const int x0r = select_bit(S.occp[(row / BY + 1) * (BY + 2) + (row & (BY - 1)) + 1], i - S.rowcube[row]);
-            c = row * BX + x0r;
-            const int x = x0r, r = (int)(c >> 8) * (BY + 1) + ((int)(c >> 5) & 7);
-            const unsigned int a = (unsigned int)(S.neg[r] >> x) & 3u, b = (unsigned int)(S.neg[r + 1] >> x) & 3u;
-            const unsigned int d = (unsigned int)(S.neg[r + BY + 1] >> x) & 3u;
-            const unsigned int e = (unsigned int)(S.neg[r + BY + 2] >> x) & 3u;
-            // corners 2, 3 and 6, 7 run against x
-            const unsigned int ci = a | (b >> 1) << 2 | (b & 1u) << 3 | d << 4 | (e >> 1) << 6 | (e & 1u) << 7;
-            nv = S.nv[ci];
-            c |= ci << 11;
+        for (int j = 0; j < PER; ++j) {
+            const unsigned int i = i0 + j;
+            c[j] = nv[j] = 0;
+            if (j < per && i < nocc) {
+                // the last row with rowcube <= i is the cube's, and it is the (i - rowcube)-th there
+                unsigned int row = 0;
+#pragma unroll
+                for (int h = CUBE_ROWS / 2; h; h >>= 1)
+                    if (S.rowcube[row + h] <= i) row += h;
+                const int x = select_bit(S.occp[(row / BY + 1) * (BY + 2) + (row & (BY - 1)) + 1], i - S.rowcube[row]);
+                const int r = (int)(row / BY) * (BY + 1) + ((int)row & (BY - 1));
+                const unsigned int a = (unsigned int)(S.neg[r] >> x) & 3u, b = (unsigned int)(S.neg[r + 1] >> x) & 3u;
+                const unsigned int d = (unsigned int)(S.neg[r + BY + 1] >> x) & 3u;
+                const unsigned int e = (unsigned int)(S.neg[r + BY + 2] >> x) & 3u;
+                // corners 2, 3 and 6, 7 run against x
+                const unsigned int ci =
+                    a | (b >> 1) << 2 | (b & 1u) << 3 | d << 4 | (e >> 1) << 6 | (e & 1u) << 7;
+                nv[j] = S.nv[ci];
+                c[j] = (row * BX + x) | ci << 11;
+            }
+            incl += nv[j];
         }
-        unsigned int incl = nv;
+        const unsigned int own = incl;
 #pragma unroll
         for (int q = 1; q < 32; q <<= 1) {
             const unsigned int u = __shfl_up_sync(full, incl, q);
             if (lane >= q) incl += u;
         }
         if (lane == 31) S.wtot[0][warp] = incl;
-        if (i0 == 0) count_slots(0, BZ);
+        count_slots(0, BZ);
         __syncthreads();
-        unsigned int pre = T_brick + incl - nv;
+        unsigned int pre = incl - own;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) {
             const unsigned int t = S.wtot[0][w];
             if (w < warp) pre += t;
             T_brick += t;
         }
-        if (i < nocc) S.cubes[i] = c | (pre << 19);
-        if (i0 == 0) R = number_slots();
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            if (j < per && i0 + j < nocc) S.cubes[i0 + j] = c[j] | (pre << 19);
+            pre += nv[j];
+        }
+        R = number_slots();
         __syncthreads();
     }
     if (T_brick >= (1u << 13) || (long long)(vbase + T_brick) > o.cap) return false;
