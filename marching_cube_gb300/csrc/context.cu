@@ -111,6 +111,7 @@ mcg_status mcg_destroy(mcg_context *ctx) {
     cudaFree(ctx->rd_sum);
     cudaFree(ctx->rd_entry);
     cudaFree(ctx->rd_first);
+    cudaFree(ctx->rd_parts);
     if (ctx->h_rd_stage) cudaFreeHost(ctx->h_rd_stage);
     cudaFree(ctx->mw_keys);
     cudaFree(ctx->mw_int);

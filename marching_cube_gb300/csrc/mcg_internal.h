@@ -163,6 +163,8 @@ struct mcg_context {
     size_t rd_entry_cap = 0;
     long long *rd_first = nullptr;
     size_t rd_first_cap = 0;
+    long long *rd_parts = nullptr;  // parts of long chunks, (xy - 1) / RD_PART a slice
+    size_t rd_parts_cap = 0;
     uint8_t *h_rd_stage = nullptr;
 
     // mesh writers: key table, int scratch (first index per slot; slot,

@@ -145,13 +145,15 @@ struct Dir {
 
 // slice of chunk c, and its words [c0, c0 + cw) of nw
 __device__ __forceinline__ void rd_chunk(const Dir &d, long long c, int *z, long long *c0, int *cw, long long *nw) {
-    int lo = 0, hi = d.nz - 1;  // last slice with cbase <= c
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (d.cbase[mid] <= c)
-            lo = mid;
-        else
-            hi = mid - 1;
+    // last slice with cbase <= c (cbase[0] <= c): 32 probes a step
+    const int lane = threadIdx.x & 31;
+    int lo = 0, n = d.nz;
+    while (n > 1) {
+        const int step = (n + 31) / 32, i = lane * step;
+        const unsigned m = __ballot_sync(0xffffffffu, i < n && d.cbase[lo + i] <= c);
+        const int at = (31 - __clz(m)) * step;
+        lo += at;
+        n = min(step, n - at);
     }
     *z = lo;
     *nw = d.len[lo] / 2;
@@ -203,16 +205,43 @@ __device__ __forceinline__ void rd_load(const uint8_t *__restrict__ img, const D
 // registers with two 16-byte loads (conflict-free) and one 4-byte load
 __device__ __forceinline__ void rd_words(const uint16_t *W, int b, unsigned w[RD_WPT + 2]) {
     const uint4 *p = reinterpret_cast<const uint4 *>(W + b);
-    const uint4 a = p[0], c = p[1];
-    const unsigned x[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        w[2 * k] = x[k] & 0xffffu;
-        w[2 * k + 1] = x[k] >> 16;
+    for (int i = 0; i < RD_WPT / 8; ++i) {
+        const uint4 a = p[i];
+        const unsigned x[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            w[8 * i + 2 * k] = x[k] & 0xffffu;
+            w[8 * i + 2 * k + 1] = x[k] >> 16;
+        }
     }
     const unsigned t = *reinterpret_cast<const unsigned *>(W + b + RD_WPT);
     w[RD_WPT] = t & 0xffffu;
     w[RD_WPT + 1] = t >> 16;
+}
+
+// A thread's words (nk of them), entered in each state: the state it leaves
+// in, its headers and their voxels, as state | headers << 2 | voxels << 8.
+// From the last word to the first (walking each of the three entry states for
+// itself, with 64-bit voxel counts, rle_summarize took 51 us for 26 MB; now 27):
+// a header's walk is that of the word after
+// its record and its own, and entry state 1 (two literal words left) starts at
+// word 2, state 2 at word 1.
+__device__ __forceinline__ void rd_walk(const unsigned *w, int nk, unsigned t[3]) {
+    // words past the end: 0, 1 or 2 literal words of the next thread's left
+    unsigned f[RD_WPT + 3];
+#pragma unroll
+    for (int k = RD_WPT + 2; k >= 0; --k) {
+        if (k < RD_WPT && k < nk) {
+            const unsigned kind = w[k] >> 14;
+            f[k] = (kind == 0u || kind == 3u ? f[k + 3] : f[k + 1]) + ((w[k] & 0x3fffu) << 8 | 4u);
+        } else {
+            f[k] = k == nk ? 0u : k == nk + 1 ? 2u : 1u;
+        }
+    }
+    t[0] = f[0];
+    t[1] = f[2];
+    t[2] = f[1];
 }
 
 // pass 1: summaries of chunks c0 + blockIdx.x
@@ -228,46 +257,72 @@ __global__ void __launch_bounds__(RD_THREADS) rle_summarize(const uint8_t *__res
     const int b = threadIdx.x * RD_WPT, nk = max(0, min(cw, b + RD_WPT) - b);
     unsigned w[RD_WPT + 2];
     rd_words(W, b, w);
-    Sum t;
-    t.f = 0;
+    unsigned wk[3], f = 0, v[3];
+    rd_walk(w, nk, wk);
 #pragma unroll
-    for (unsigned en = 0; en < 3; ++en) {
-        unsigned s = en;
-        long long v = 0;
-#pragma unroll
-        for (int k = 0; k < RD_WPT; ++k) {
-            if (k < nk) {
-                if (s == 0u) v += w[k] & 0x3fff;
-                s = rd_apply(rd_word_map(w[k]), s);
-            }
-        }
-        t.v[en] = v;
-        t.f |= s << (2 * en);
+    for (int e = 0; e < 3; ++e) {
+        f |= (wk[e] & 3u) << (2 * e);
+        v[e] = wk[e] >> 8;
     }
-    Sum total;
-    sum_block_scan(t, s_w, &total);
-    if (threadIdx.x == 0) sums[c] = total;
+    // composed in order over the warp, then over the warps (a chunk's voxels fit 32 bits)
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned fb = __shfl_down_sync(0xffffffffu, f, o), v0 = __shfl_down_sync(0xffffffffu, v[0], o),
+                       v1 = __shfl_down_sync(0xffffffffu, v[1], o), v2 = __shfl_down_sync(0xffffffffu, v[2], o);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const unsigned at = rd_apply(f, (unsigned)e);
+            v[e] += at == 0u ? v0 : at == 1u ? v1 : v2;
+        }
+        f = rd_then(f, fb);
+    }
+    if (lane == 0) s_w[wid] = Sum{f, {(long long)v[0], (long long)v[1], (long long)v[2]}};
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        Sum total = s_w[0];
+#pragma unroll
+        for (int i = 1; i < RD_THREADS / 32; ++i) total = sum_then(total, s_w[i]);
+        sums[c] = total;
+    }
 }
 
+// A chunk of few records can hold a slice of voxels (16383 a record; 512^3
+// voxels of a scene: 3517 chunks of 38162 voxels on average, 254 of 262144),
+// so a chunk's voxels beyond the first RD_PART are expanded by CTAs of their
+// own, RD_PART each.  A slice has room for (xy - 1) / RD_PART of these: one
+// that would start at voxel s is entry s / RD_PART - 1, its own since those of
+// a chunk start RD_PART apart and the next chunk's begin at least RD_PART
+// after the chunk's end.  rle_expand there: 163 us without, 144 with parts of
+// 65536, 158 with parts of 32768 (the steps before a part's voxels are repeated).
+constexpr int RD_PART = 65536;
+
 // pass 2: one CTA per slice z0 + blockIdx.x: entry state and first voxel of
-// each of its chunks; a slice whose records end before it is full is an error
+// each of its chunks, and its parts (chunk << 16 | part, or -1); a slice whose records end before it is full is an error
 __global__ void __launch_bounds__(RD_THREADS) rle_slice_scan(Dir d, int z0, long long xy,
                                                              const Sum *__restrict__ sums,
                                                              unsigned char *__restrict__ entry,
-                                                             long long *__restrict__ first, int *__restrict__ err) {
+                                                             long long *__restrict__ first,
+                                                             long long *__restrict__ parts, int *__restrict__ err) {
     __shared__ Sum s_w[RD_THREADS / 32];
     const int z = z0 + blockIdx.x;
     const long long cb = d.cbase[z], ce = d.cbase[z + 1];
     unsigned state = 0;
     long long out = 0;
+    const long long np = (xy - 1) / RD_PART;
+    parts += z * np;
+    for (long long i = threadIdx.x; i < np; i += RD_THREADS) parts[i] = -1;
     for (long long k = cb; k < ce; k += RD_THREADS) {
         const long long c = k + threadIdx.x;
         const Sum x = c < ce ? sums[c] : Sum{RD_ID, {0, 0, 0}};
         Sum total;
-        const Sum pre = sum_block_scan(x, s_w, &total);
+        const Sum pre = sum_block_scan(x, s_w, &total);  // (a barrier between parts[] = -1 and its entries)
         if (c < ce) {
-            entry[c] = (unsigned char)rd_apply(pre.f, state);
-            first[c] = out + sum_pick(pre, state);
+            const unsigned en = rd_apply(pre.f, state);
+            const long long a = out + sum_pick(pre, state), b = min(xy, a + sum_pick(x, en));
+            entry[c] = (unsigned char)en;
+            first[c] = a;
+            for (long long s = a + RD_PART, p = 1; s < b; s += RD_PART, ++p) parts[s / RD_PART - 1] = c << 16 | p;
         }
         out += sum_pick(total, state);
         state = rd_apply(total.f, state);
@@ -276,13 +331,15 @@ __global__ void __launch_bounds__(RD_THREADS) rle_slice_scan(Dir d, int z0, long
 }
 
 // Voxels [out, end) of a slice from the chunk's runs (rs: starts counted from
-// `out`, rv: voxels, n of them), RD_TILE voxels at a time: a bit is set where a
+// `out`, rv: voxels from rv[1] on, n of them), RD_TILE voxels at a time: a bit is set where a
 // run starts, the set bits before each 32-bit word are counted, and a voxel's
 // run is the number of bits up to its own.  Each lane writes four consecutive
 // voxels, 16 bytes.  Bound: the instructions of this, then writing the volume.
 // Expanding 512^3 voxels from 26 MB: a binary search over the chunk's runs for
 // each voxel took 967 us, for each four voxels between those of a warp's ends
-// 431 us; this 171 us.
+// 431 us; this 171 us, 144 with long chunks in parts, 135 with the words and
+// bits of a full tile's voxels at fixed places and one look-up where no run
+// starts inside the four, 132 with six CTAs per SM instead of five.
 constexpr int RD_TILE = 16384;
 
 struct RunTile {
@@ -292,14 +349,22 @@ struct RunTile {
 };
 
 __device__ __forceinline__ void rd_write_runs(RunTile &S, uint32_t *__restrict__ slice, long long out, long long end,
-                                              const int *rs, const uint32_t *rv, int n) {
+                                              const int *rs, const uint32_t *rv, int n, int part) {
     constexpr int WPT = RD_TILE / 32 / RD_THREADS;  // words per thread
     const int tid = threadIdx.x;
     const int total = (int)(end - out);
     // tiles start on 16-byte boundaries: the first one at or below `out`
     const int lead = (int)((reinterpret_cast<uintptr_t>(slice + out) >> 2) & 3u);
+    // this part's voxels; the last one takes what is left
+    const int first = part * RD_PART - lead;
+    const int last = (part + 1) * (long long)RD_PART < total ? first + RD_PART : total;
     int base = 0;  // runs that start before the tile
-    for (int t0 = -lead; t0 < total; t0 += RD_TILE) {
+    if (part) {
+        int c = 0;
+        for (int r = tid; r < n; r += RD_THREADS) c += rs[r] < first;
+        rd_block_scan<int>(c, 0, [](int a, int b) { return a + b; }, S.w, &base);
+    }
+    for (int t0 = first; t0 < last; t0 += RD_TILE) {
         for (int i = tid; i < RD_TILE / 32; i += RD_THREADS) S.start[i] = 0u;
         __syncthreads();
         for (int r = tid; r < n; r += RD_THREADS) {
@@ -319,43 +384,75 @@ __device__ __forceinline__ void rd_write_runs(RunTile &S, uint32_t *__restrict__
         for (int i = 0; i < WPT; ++i) S.before[tid * WPT + i] = ex + c[i];
         base += all;
         __syncthreads();
-        const int stop = min(RD_TILE, total - t0);
-        for (int p = 4 * tid; p < stop; p += 4 * RD_THREADS) {
-            const uint32_t word = S.start[p >> 5];
-            const int bit = p & 31;
-            int r = S.before[p >> 5] + __popc(word & ((1u << bit) - 1u)) - 1;
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                r += (word >> (bit + k)) & 1u;
-                w[k] = rv[max(r, 0)];  // (before the first run: voxels below `out`, not written)
+        const int stop = min(RD_TILE, last - t0);
+        // four voxels a thread and step, at the same bits of their words every time
+        const int bit = (4 * tid) & 31;
+        const uint32_t below = (1u << bit) - 1u;
+        auto four = [&](int p) -> uint4 {
+            const uint32_t word = S.start[p >> 5], f = word >> bit;
+            const uint32_t *v = rv + S.before[p >> 5] + __popc(word & below);
+            if (f & 1u) ++v;
+            uint4 q;
+            q.x = q.y = q.z = q.w = v[0];
+            if (f & 14u) {
+                if (f & 2u) ++v;
+                q.y = v[0];
+                if (f & 4u) ++v;
+                q.z = v[0];
+                if (f & 8u) ++v;
+                q.w = v[0];
             }
-            const int v = t0 + p;
-            uint32_t *dst = slice + out + v;
-            if (v >= 0 && v + 4 <= total) {
-                *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-            } else {
+            return q;
+        };
+        uint32_t *dst = slice + out + t0;  // (not below the slice's buffer where it is written)
+        if (t0 >= 0 && stop == RD_TILE) {
+#pragma unroll 4
+            for (int i = 0; i < RD_TILE / (4 * RD_THREADS); ++i) {
+                const int p = 4 * tid + 4 * RD_THREADS * i;
+                *reinterpret_cast<uint4 *>(dst + p) = four(p);
+            }
+        } else {
+            for (int p = 4 * tid; p < stop; p += 4 * RD_THREADS) {
+                const uint4 q = four(p);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+                const int v = t0 + p;
+                if (v >= 0 && v + 4 <= total) {
+                    *reinterpret_cast<uint4 *>(dst + p) = q;
+                } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (v + k >= 0 && v + k < total) dst[k] = w[k];
+                    for (int k = 0; k < 4; ++k)
+                        if (v + k >= 0 && v + k < total) dst[p + k] = w[k];
+                }
             }
         }
         __syncthreads();
     }
 }
 
-// pass 3: expand chunks cfirst + blockIdx.x
-__global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restrict__ img, Dir d, long long cfirst,
+// pass 3: expand chunks cfirst + blockIdx.x, and the parts after them
+__global__ void __launch_bounds__(RD_THREADS, 6) rle_expand(const uint8_t *__restrict__ img, Dir d, long long cfirst,
                                                          long long xy, const unsigned char *__restrict__ entry_of,
                                                          const long long *__restrict__ first_of,
+                                                         const long long *__restrict__ parts, long long nc,
                                                          uint32_t *__restrict__ vol, int *__restrict__ err) {
-    __shared__ __align__(16) uint16_t W[RD_CHUNK + 8];
-    __shared__ int rs[RD_CHUNK];
-    __shared__ uint32_t rv[RD_CHUNK];
+    __shared__ union {
+        __align__(16) uint16_t W[RD_CHUNK + 8];  // until every thread has its words
+        int rs[RD_CHUNK];
+    } U;
+    uint16_t *const W = U.W;
+    int *const rs = U.rs;
+    __shared__ uint32_t rv[RD_CHUNK + 1];  // run r's voxel at r + 1; 0: voxels below `out`, not written
     __shared__ RunTile S;
     __shared__ unsigned s_f[RD_THREADS / 32];
-    __shared__ int s_i[RD_THREADS / 32];
-    const long long c = cfirst + blockIdx.x;
+    __shared__ unsigned long long s_l[RD_THREADS / 32];
+    long long c = cfirst + blockIdx.x;
+    int part = 0;
+    if (blockIdx.x >= nc) {
+        const long long i = parts[blockIdx.x - nc];
+        if (i < 0) return;
+        c = i >> 16;
+        part = (int)(i & 0xffff);
+    }
     const long long out = first_of[c], n = xy;
     if (out >= n) return;  // records after a full slice are ignored
     int z, cw;
@@ -368,35 +465,23 @@ __global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restri
     const int b = threadIdx.x * RD_WPT, nk = max(0, min(cw, b + RD_WPT) - b);
     unsigned w[RD_WPT + 2];
     rd_words(W, b, w);
-    unsigned f = RD_ID;
-#pragma unroll
-    for (int k = 0; k < RD_WPT; ++k)
-        if (k < nk) f = rd_then(f, rd_word_map(w[k]));
+    unsigned wk3[3];
+    rd_walk(w, nk, wk3);
     unsigned fall;
-    const unsigned fpre = rd_block_scan<unsigned>(f, RD_ID, [](unsigned a, unsigned c2) { return rd_then(a, c2); },
-                                                  s_f, &fall);
+    const unsigned fpre = rd_block_scan<unsigned>((wk3[0] & 3u) | (wk3[1] & 3u) << 2 | (wk3[2] & 3u) << 4, RD_ID,
+                                                  [](unsigned a, unsigned c2) { return rd_then(a, c2); }, s_f, &fall);
     const unsigned entry = rd_apply(fpre, state);
-    int nrec = 0;
-    long long nvox = 0;
+    const unsigned own = entry == 0u ? wk3[0] : entry == 1u ? wk3[1] : wk3[2];
+    // records and voxels before this thread's, in one scan
+    unsigned long long tot;
+    const unsigned long long pre = rd_block_scan<unsigned long long>(
+        (unsigned long long)(own >> 8) << 32 | ((own >> 2) & 63u), 0ull,
+        [](unsigned long long a, unsigned long long c2) { return a + c2; }, s_l, &tot);
+    const int rtot = (int)(unsigned int)tot;
+    const long long vtot = (long long)(tot >> 32);
     unsigned s = entry;
-#pragma unroll
-    for (int k = 0; k < RD_WPT; ++k) {
-        if (k < nk) {
-            if (s == 0u) {
-                ++nrec;
-                nvox += w[k] & 0x3fff;
-            }
-            s = rd_apply(rd_word_map(w[k]), s);
-        }
-    }
-    int rtot;
-    long long vtot;
-    const int r0 = rd_block_scan<int>(nrec, 0, [](int a, int c2) { return a + c2; }, s_i, &rtot);
-    __shared__ long long s_l[RD_THREADS / 32];
-    const long long v0 = rd_block_scan<long long>(nvox, 0, [](long long a, long long c2) { return a + c2; }, s_l, &vtot);
-    s = entry;
-    int r = r0;
-    long long o = v0;
+    int r = (int)(unsigned int)pre;
+    long long o = (long long)(pre >> 32);
 #pragma unroll
     for (int k = 0; k < RD_WPT; ++k) {
         if (k < nk) {
@@ -416,16 +501,17 @@ __global__ void __launch_bounds__(RD_THREADS) rle_expand(const uint8_t *__restri
                 const long long start = out + o;
                 if (start < n && (cnt == 0u || start + (long long)cnt > n || !lit_ok)) bad = true;
                 rs[r] = (int)min(o, (long long)INT32_MAX);
-                rv[r] = val;
+                rv[r + 1] = val;
                 ++r;
                 o += cnt;
             }
             s = rd_apply(rd_word_map(wk), s);
         }
     }
+    if (threadIdx.x == 0) rv[0] = 0u;
     __syncthreads();
     const long long end = min(n, out + vtot);
-    rd_write_runs(S, out_slice, out, end, rs, rv, rtot);
+    rd_write_runs(S, out_slice, out, end, rs, rv, rtot, part);
     if (bad) atomicOr(err, 1);
 }
 
@@ -444,24 +530,28 @@ cudaError_t launch_expand(mcg_context *ctx, const Slab &sl, const long long *cba
     const long long cf = cbase_host[sl.z0], nc = cbase_host[sl.z1] - cf;
     Sum *sums = reinterpret_cast<Sum *>(ctx->rd_sum);
     unsigned char *entry = ctx->rd_entry;
+    const long long np = (xy - 1) / RD_PART;  // parts a slice
     if (nc > 0) rle_summarize<<<(unsigned)nc, RD_THREADS, 0, s>>>(ctx->rle_image, d, cf, sums);
-    rle_slice_scan<<<sl.z1 - sl.z0, RD_THREADS, 0, s>>>(d, sl.z0, xy, sums, entry, ctx->rd_first, ctx->rd_err);
+    rle_slice_scan<<<sl.z1 - sl.z0, RD_THREADS, 0, s>>>(d, sl.z0, xy, sums, entry, ctx->rd_first, ctx->rd_parts,
+                                                         ctx->rd_err);
     if (nc > 0)
-        rle_expand<<<(unsigned)nc, RD_THREADS, 0, s>>>(ctx->rle_image, d, cf, xy, entry, ctx->rd_first,
-                                                      static_cast<uint32_t *>(vol), ctx->rd_err);
+        rle_expand<<<(unsigned)(nc + (sl.z1 - sl.z0) * np), RD_THREADS, 0, s>>>(
+            ctx->rle_image, d, cf, xy, entry, ctx->rd_first, ctx->rd_parts + sl.z0 * np, nc,
+            static_cast<uint32_t *>(vol), ctx->rd_err);
     return cudaGetLastError();
 }
 
 constexpr int64_t RD_SLAB = (int64_t)64 << 20;  // image bytes per copy
 
 // device buffers for an image of `size` bytes and nz slices: the image, the
-// directory (offsets, lengths, chunk bases) and the per-chunk arrays
-mcg_status prepare(mcg_context *ctx, int nz, int64_t size) {
+// directory (offsets, lengths, chunk bases) and the per-chunk arrays; xy >= 1
+mcg_status prepare(mcg_context *ctx, int64_t xy, int nz, int64_t size) {
     const size_t chunks = (size_t)(size / (2 * RD_CHUNK)) + (size_t)nz + 1;  // bounds the chunks of any image
     if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)size + 64) ||
         !ensure(&ctx->rd_dir, &ctx->rd_dir_cap, 3 * (size_t)nz + 1) || !ensure(&ctx->rd_err, &ctx->rd_err_cap, 1) ||
         !ensure(&ctx->rd_sum, &ctx->rd_sum_cap, chunks * sizeof(Sum)) ||
-        !ensure(&ctx->rd_first, &ctx->rd_first_cap, chunks) || !ensure(&ctx->rd_entry, &ctx->rd_entry_cap, chunks))
+        !ensure(&ctx->rd_first, &ctx->rd_first_cap, chunks) ||
+        !ensure(&ctx->rd_parts, &ctx->rd_parts_cap, (size_t)((xy - 1) / RD_PART) * nz) || !ensure(&ctx->rd_entry, &ctx->rd_entry_cap, chunks))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     ctx->rd_dir_n = nz;
     return MCG_OK;
@@ -525,7 +615,7 @@ extern "C" mcg_status mcg_rle_decode(mcg_context *ctx, const uint8_t *image, int
     }
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    if ((st = prepare(ctx, nz, p)) != MCG_OK) return st;
+    if ((st = prepare(ctx, xy, nz, p)) != MCG_OK) return st;
     const cudaStream_t s = (cudaStream_t)stream;
     if ((e = cudaMemsetAsync(ctx->rd_err, 0, sizeof(int), s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(ctx->rd_dir, dir.data(), dir.size() * sizeof(long long), cudaMemcpyHostToDevice, s)) !=
@@ -591,7 +681,7 @@ extern "C" mcg_status mcg_rle_decode_file(mcg_context *ctx, const char *path, vo
     cudaError_t e = cudaSuccess;
     if (st == MCG_OK && (e = cudaSetDevice(ctx->device)) != cudaSuccess) st = mcg_cuda_fail(ctx, e);
     const int nz = dims[2];
-    if (st == MCG_OK) st = prepare(ctx, nz, size);
+    if (st == MCG_OK) st = prepare(ctx, xy, nz, size);
     if (st == MCG_OK && !ctx->h_rd_stage) {
         if (cudaMallocHost((void **)&ctx->h_rd_stage, 2 * (size_t)RD_SLAB) != cudaSuccess) {
             ctx->h_rd_stage = nullptr;

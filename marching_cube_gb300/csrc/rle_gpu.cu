@@ -34,10 +34,6 @@ constexpr int RWORDS = RCHUNK / 32;
 constexpr int RWARPS = RT / 32;
 constexpr int kMaxRun = 0x3fff;
 
-__device__ __forceinline__ bool same_voxel(uint32_t a, uint32_t b, bool lossless) {
-    return lossless ? a == b : ((a ^ b) & 0xffffu) == 0u;
-}
-
 // record kind of a record whose first voxel is v (put_run in rle.cpp)
 __device__ __forceinline__ unsigned record_kind(uint32_t v, bool lossless) {
     const int16_t t = (int16_t)(v & 0xffffu);
@@ -57,9 +53,11 @@ struct RleChunk {
 };
 
 // Pass 1.  A warp reads 512 consecutive voxels, 16 bytes a lane at a time, all
-// loads ahead of their use.  Bound: HBM.  One CTA sweeping a slice, a block
-// scan per chunk, took 311 us for 512^3 voxels just to count and 563 us more
-// to write (26 MB); the passes here take 138, 5, 2 and 128 us.
+// loads ahead of their use.  Bound: HBM (the volume once: 79 us for 512^3
+// voxels).  One CTA sweeping a slice, a block scan per chunk, took 311 us for
+// these just to count and 563 us more to write (26 MB); the passes here take
+// 101, 5, 2 and 53 us.  This one took 138 us with the run starts' kinds and
+// words worked out for every 128 voxels, also where no run starts.
 __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
                                                RleChunk *__restrict__ chunks, uint32_t *__restrict__ marks, int vec) {
     constexpr int Q = RCHUNK / RT / 4;  // 16-byte words per lane
@@ -84,6 +82,7 @@ __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol,
         }
     }
     uint32_t before = w0 > 0 && w0 <= xy ? __ldg(sl + w0 - 1) : 0u;
+    const uint32_t differ = lossless ? 0xffffffffu : 0xffffu;
     int bytes = 0, first = INT32_MAX, last = -1;
     uint32_t *out = marks + c * RWORDS + warp * 4 * Q;
 #pragma unroll
@@ -95,22 +94,26 @@ __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol,
         const uint32_t x[5] = {left, v[q].x, v[q].y, v[q].z, v[q].w};
         uint32_t bits = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const bool start = i + k < xy && (i + k == 0 || !same_voxel(x[k + 1], x[k], lossless));
-            if (start) {
-                bits |= 1u << k;
-                bytes += record_kind(x[k + 1], lossless) == 3u ? 6 : 2;
+        for (int k = 0; k < 4; ++k)
+            if ((x[k + 1] ^ x[k]) & differ) bits |= 1u << k;
+        if (i == 0) bits |= 1u;  // a slice starts a run
+        if (i + 4 > xy) bits &= i < xy ? (1u << (xy - i)) - 1u : 0u;
+        uint32_t word = 0;
+        if (__any_sync(0xffffffffu, bits)) {
+            // most 128 voxels have no run start
+            if (bits) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (bits & (1u << k)) bytes += record_kind(x[k + 1], lossless) == 3u ? 6 : 2;
+                first = min(first, i + __ffs(bits) - 1);
+                last = i + 31 - __clz(bits);
             }
+            // eight lanes' bits make a word
+            word = bits << (4 * (lane & 7));
+            word |= __shfl_xor_sync(0xffffffffu, word, 1);
+            word |= __shfl_xor_sync(0xffffffffu, word, 2);
+            word |= __shfl_xor_sync(0xffffffffu, word, 4);
         }
-        if (bits) {
-            first = min(first, i + __ffs(bits) - 1);
-            last = i + 31 - __clz(bits);
-        }
-        // eight lanes' bits make a word
-        uint32_t word = bits << (4 * (lane & 7));
-        word |= __shfl_xor_sync(0xffffffffu, word, 1);
-        word |= __shfl_xor_sync(0xffffffffu, word, 2);
-        word |= __shfl_xor_sync(0xffffffffu, word, 4);
         if ((lane & 7) == 0) out[4 * q + (lane >> 3)] = word;
     }
     bytes = __reduce_add_sync(0xffffffffu, bytes);
@@ -232,30 +235,33 @@ __global__ void __launch_bounds__(RT) rle_slices(const unsigned long long *__res
     if (threadIdx.x == 0) off[nz] = at;
 }
 
-// Pass 3.
+// Pass 3.  Bound: the chain of loads and scans of a chunk, so as many chunks in
+// flight as an SM has threads for: 128 us with 256 threads and room for all of
+// a chunk's records (41 KB), 53 with 128 threads and 9 KB.
+constexpr int ET = RWORDS, EWARPS = ET / 32;  // a thread for each word of marks
+
 struct RleEmit {
-    int pos[RCHUNK + 1];            // record starts (slice index), then the record after the chunk
-    uint16_t img[3 * RCHUNK + 4];   // the records
-    int wn[RWARPS], wb[RWARPS];
+    uint16_t pos[RCHUNK + 1];  // record starts, then the record after the chunk, from the chunk's first voxel
+    uint16_t img[3 * ET];      // ET records at a time
+    int wn[EWARPS], wb[EWARPS];
 };
 
-__global__ void __launch_bounds__(RT) rle_emit(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
+__global__ void __launch_bounds__(ET) rle_emit(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
                                                const RleChunk *__restrict__ chunks, const uint32_t *__restrict__ marks,
                                                const unsigned long long *__restrict__ slice_bytes,
                                                const unsigned long long *__restrict__ slice_off,
                                                uint8_t *__restrict__ img) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    RleEmit &S = *reinterpret_cast<RleEmit *>(smem_raw);
+    __shared__ RleEmit S;
     const bool lossless = lossless_i != 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long c = blockIdx.x;
     const int z = (int)(c / nchunks), c0 = (int)(c - (long long)z * nchunks) * RCHUNK;
+    const uint32_t word = marks[c * RWORDS + tid];
     const RleChunk r = chunks[c];
     const unsigned long long so = slice_off[z];  // even: 40, then 4 and even record bytes a slice
     if (c0 == 0 && tid < 2) reinterpret_cast<uint16_t *>(img + so)[tid] = (uint16_t)(slice_bytes[z] >> (16 * tid));
     if (r.bytes == 0) return;  // no record starts here
     // record starts in order: the split, then the marked voxels
-    const uint32_t word = tid < RWORDS ? marks[c * RWORDS + tid] : 0u;
     int n = __popc(word), incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -267,19 +273,19 @@ __global__ void __launch_bounds__(RT) rle_emit(const uint32_t *__restrict__ vol,
     const int extra = r.split >= 0 ? 1 : 0;
     int at = extra + incl - n, total = extra;
 #pragma unroll
-    for (int w = 0; w < RWARPS; ++w) {
+    for (int w = 0; w < EWARPS; ++w) {
         if (w < warp) at += S.wn[w];
         total += S.wn[w];
     }
-    for (uint32_t m = word; m; m &= m - 1) S.pos[at++] = c0 + 32 * tid + __ffs(m) - 1;
+    for (uint32_t m = word; m; m &= m - 1) S.pos[at++] = (uint16_t)(32 * tid + __ffs(m) - 1);
     if (tid == 0) {
-        if (extra) S.pos[0] = r.split;
-        S.pos[total] = r.next;
+        if (extra) S.pos[0] = (uint16_t)(r.split - c0);
+        S.pos[total] = (uint16_t)(r.next - c0);  // at most a record's voxels past the chunk
     }
     __syncthreads();
-    const uint32_t *sl = vol + (long long)z * xy;
-    int base = 0;  // halfwords before these records
-    for (int j0 = 0; j0 < total; j0 += RT) {
+    const uint32_t *sl = vol + (long long)z * xy + c0;
+    uint16_t *out = reinterpret_cast<uint16_t *>(img + so + 4 + (unsigned int)r.off);
+    for (int j0 = 0; j0 < total; j0 += ET) {
         const int j = j0 + tid;
         uint32_t v = 0;
         int halves = 0, count = 0;
@@ -299,9 +305,9 @@ __global__ void __launch_bounds__(RT) rle_emit(const uint32_t *__restrict__ vol,
         }
         if (lane == 31) S.wb[warp] = sum;
         __syncthreads();
-        int pre = base, all = 0;
+        int pre = 0, all = 0;
 #pragma unroll
-        for (int w = 0; w < RWARPS; ++w) {
+        for (int w = 0; w < EWARPS; ++w) {
             if (w < warp) pre += S.wb[w];
             all += S.wb[w];
         }
@@ -313,11 +319,10 @@ __global__ void __launch_bounds__(RT) rle_emit(const uint32_t *__restrict__ vol,
                 S.img[h + 2] = (uint16_t)(v >> 16);
             }
         }
-        base += all;
         __syncthreads();
+        for (int i = tid; i < all; i += ET) out[i] = S.img[i];
+        out += all;
     }
-    uint16_t *out = reinterpret_cast<uint16_t *>(img + so + 4 + (unsigned int)r.off);
-    for (int h = tid; h < base; h += RT) out[h] = S.img[h];
 }
 
 const char kTagRef[16] = "VOLUME_TSDF_RGB";
@@ -366,9 +371,8 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
         return query ? MCG_OK : MCG_ERR_CAPACITY;
     }
     if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
-    cudaFuncSetAttribute(rle_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RleEmit));
-    rle_emit<<<(unsigned int)total, RT, sizeof(RleEmit), s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks,
-                                                             d_bytes, d_off, ctx->rle_image);
+    rle_emit<<<(unsigned int)total, ET, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks, d_bytes, d_off,
+                                                ctx->rle_image);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     // header (:1303-1310), then the slices

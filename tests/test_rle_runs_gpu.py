@@ -59,3 +59,40 @@ def test_both_ways(mcg, shape, offset, lossless):
         want, _ = mcg.rle_decode_host(image)
         assert np.array_equal(back[offset:offset + n].cpu().numpy().reshape(vol.shape), want)
         assert bool((back[:offset] == 77).all()) and bool((back[offset + n:] == 77).all())
+
+
+@pytest.mark.parametrize("offset", [0, 3])
+@pytest.mark.parametrize("shape", [(2, 256, 256), (2, 257, 255), (3, 256, 257), (2, 300, 500), (3, 1, 200001), (1, 640, 1000)])
+def test_long_chunks_in_parts(mcg, shape, offset):
+    """Slices of one run, of runs that end around multiples of 65536 voxels
+    (where a chunk's parts end), and of short runs then one long run."""
+    nz, ny, nx = shape
+    xy, n = nx * ny, nx * ny * nz
+    rng = np.random.default_rng(nx + offset)
+    for kind in range(3):
+        vol = np.zeros((nz, xy, 2), np.int16)
+        for z in range(nz):
+            if kind == 0:
+                vol[z] = (32766, -32766, 5)[z], 0
+            elif kind == 1:
+                cuts = [c for c in (3 * z, 65535 - z, 65536, 65537 + z, 131072, 131075) if c < xy]
+                for a, b in zip([0] + cuts, cuts + [xy]):
+                    vol[z, a:b, 0] = rng.integers(-1000, 1000)
+            else:
+                at = int(rng.integers(2000, min(xy, 9000)))
+                vol[z, :at, 0] = rng.integers(-3, 3, at)
+                vol[z, at:, 0] = -32766
+                vol[z, xy - 5:, 0] = np.arange(5)
+        vol = vol.reshape(nz, ny, nx, 2)
+        image = bytes(mcg.rle_encode_host(vol, 0.1, 0.2, 0.3, False))
+        back = torch.full((n + 8, 2), 77, dtype=torch.int16, device="cuda")
+        ctx = mcg.default_context()
+        arr = np.frombuffer(image, np.uint8)
+        st = mcg._lib.mcg_rle_decode(ctx.handle, arr.ctypes.data_as(ctypes.c_void_p), arr.size,
+                                     ctypes.c_void_p(back.data_ptr() + 4 * offset), n,
+                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0
+        torch.cuda.synchronize()
+        want, _ = mcg.rle_decode_host(image)
+        assert np.array_equal(back[offset:offset + n].cpu().numpy().reshape(vol.shape), want)
+        assert bool((back[:offset] == 77).all()) and bool((back[offset + n:] == 77).all())
