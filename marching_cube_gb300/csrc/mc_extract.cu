@@ -477,7 +477,12 @@ __device__ __forceinline__ int cached_volume(VolCache &c, const VolDesc *__restr
 // draw in flight meanwhile.  Bound: instructions (about 11 a row), then L2
 // (every voxel is read 1.3 times).  Filling a shared-memory tile by shifted
 // 16-byte words first took 83 us for a 385 x 257 x 321 short2 volume and, with
-// TMA where it applies, 228 us for 64 volumes of 66 M voxels; this 43 and 145.
+// TMA where it applies, 228 us for 64 volumes of 66 M voxels; this 43 and 145,
+// and 43 and 102 with the signs of a short2 brick looked at first (4 operations
+// a row instead of 11; a mixed brick's rows, a quarter of the batch's, are read
+// once more) and three CTAs per SM instead of four, which then only evict each
+// other's lines (four 45 and 110, five 49 and 154, two 39 and 128).  float2
+// keeps the one pass: 30 us for 201 x 175 x 233 voxels against 38.
 struct RowsParams {
     // one volume ...
     const void *vol;
@@ -499,9 +504,59 @@ struct RowsSmem {
     unsigned char ntri[256];
 };
 
+// True where the short2 brick whose first voxel is p has a negative distance
+// and one that is not; FULL: 33 x 9 x 9 voxels are inside the volume, else nx1
+// x ny1 x nz1 of them.  Two operations a voxel row and a vote at the end.
+template <bool FULL>
+__device__ __forceinline__ bool brick_mixed(const short2 *__restrict__ p, long long sy, long long sz, int nx1, int ny1,
+                                            int nz1) {
+    const int lane = threadIdx.x & 31;
+    int e[3], a[BY + 1], b[BY + 1];
+    bool ein[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int r = lane + 32 * j, lz = r / (BY + 1), ly = r - (BY + 1) * lz;
+        ein[j] = r < ROWS && (FULL || (nx1 > BX && ly < ny1 && lz < nz1));
+        e[j] = ein[j] ? p[lz * sz + ly * sy + BX].x : 0;
+    }
+    bool any = false, other = false;
+    auto fetch = [&](int (&w)[BY + 1], int lz) {
+        const short2 *q = p + lz * sz + lane;
+#pragma unroll
+        for (int ly = 0; ly < BY + 1; ++ly) {
+            w[ly] = FULL || (lane < nx1 && ly < ny1 && lz < nz1) ? q->x : 0;
+            q += sy;
+        }
+    };
+    auto test = [&](const int (&w)[BY + 1], int lz) {
+#pragma unroll
+        for (int ly = 0; ly < BY + 1; ++ly) {
+            const bool n = w[ly] < 0;
+            any = any || n;
+            other = other || (!n && (FULL || (lane < nx1 && ly < ny1 && lz < nz1)));
+        }
+    };
+    fetch(a, 0);
+#pragma unroll 1
+    for (int lz = 0; lz < BZ; lz += 2) {
+        fetch(b, lz + 1);
+        test(a, lz);
+        fetch(a, lz + 2);
+        test(b, lz + 1);
+    }
+    test(a, BZ);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        any = any || e[j] < 0;
+        other = other || (ein[j] && e[j] >= 0);
+    }
+    return __any_sync(0xffffffffu, any) && __any_sync(0xffffffffu, other);
+}
+
 // Row masks of the brick whose first voxel is p (this lane's: p[lane]) into row[],
 // the 33rd voxels' into en / ed (row r: bit r % 32 of word r / 32), and whether
-// a voxel inside the volume is negative, or not.  FULL: 33 x 9 x 9 voxels are
+// a voxel inside the volume is negative, or not (both true for a short2 brick,
+// brick_mixed has said so).  FULL: 33 x 9 x 9 voxels are
 // inside; else nx1 x ny1 x nz1 of them, the others read as weight 0.
 template <int VT, bool FULL>
 __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T *__restrict__ p, long long sy, long long sz,
@@ -535,9 +590,11 @@ __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T 
         for (int ly = 0; ly < BY + 1; ++ly) {
             const unsigned int n = __ballot_sync(full, V::neg(w[ly])), d = __ballot_sync(full, V::w0(w[ly]));
             row[lz * (BY + 1) + ly] = make_uint2(n, d);  // (every lane the same)
-            any |= n;
-            if (FULL) every &= n;
-            else if (ly < ny1 && lz < nz1) every &= n | ~xmask;
+            if constexpr (VT == MCG_VOXEL_FLOAT2) {
+                any |= n;
+                if (FULL) every &= n;
+                else if (ly < ny1 && lz < nz1) every &= n | ~xmask;
+            }
         }
     };
     T a[BY + 1], b[BY + 1];
@@ -550,15 +607,18 @@ __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T 
         vote(b, lz + 1);
     }
     vote(a, BZ);
-    pos_any = ~every;
+    neg_any = pos_any = 1u;
+    if constexpr (VT == MCG_VOXEL_FLOAT2) pos_any = ~every;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         en[j] = __ballot_sync(full, V::neg(e[j]));
         ed[j] = __ballot_sync(full, V::w0(e[j]));
-        any |= en[j];
-        pos_any |= __ballot_sync(full, ein[j] && !V::neg(e[j]));
+        if constexpr (VT == MCG_VOXEL_FLOAT2) {
+            any |= en[j];
+            pos_any |= __ballot_sync(full, ein[j] && !V::neg(e[j]));
+        }
     }
-    neg_any = any;
+    if constexpr (VT == MCG_VOXEL_FLOAT2) neg_any = any;
 }
 
 // triangles and occupied cubes of the brick at (x0, y0, z0); whole warp
@@ -571,10 +631,19 @@ __device__ __forceinline__ void count_rows(uint2 *row, const unsigned char *ntri
     const typename Vox<VT>::T *p = vol + lin3(nx, ny, x0, y0, z0);
     const long long sy = nx, sz = (long long)nx * ny;
     unsigned int en[3], ed[3], neg_any, pos_any;
-    if (x0 + BX < nx && y0 + BY < ny && z0 + BZ < nz)
-        load_rows<VT, true>(row, p, sy, sz, 0, 0, 0, en, ed, neg_any, pos_any);
-    else load_rows<VT, false>(row, p, sy, sz, nx - x0, ny - y0, nz - z0, en, ed, neg_any, pos_any);
+    const bool inside = x0 + BX < nx && y0 + BY < ny && z0 + BZ < nz;
     tri = occ = 0;
+    if (inside) {
+        if constexpr (VT == MCG_VOXEL_SHORT2) {
+            if (!brick_mixed<true>(p, sy, sz, 0, 0, 0)) return;
+        }
+        load_rows<VT, true>(row, p, sy, sz, 0, 0, 0, en, ed, neg_any, pos_any);
+    } else {
+        if constexpr (VT == MCG_VOXEL_SHORT2) {
+            if (!brick_mixed<false>(p, sy, sz, nx - x0, ny - y0, nz - z0)) return;
+        }
+        load_rows<VT, false>(row, p, sy, sz, nx - x0, ny - y0, nz - z0, en, ed, neg_any, pos_any);
+    }
     if (!neg_any || !pos_any) return;
     __syncwarp();
     const unsigned int valid = valid_mask(x0, nx);
@@ -608,7 +677,7 @@ __device__ __forceinline__ void count_rows(uint2 *row, const unsigned char *ntri
 }
 
 template <int VT, bool BATCH>
-__global__ void __launch_bounds__(RW_THREADS, VT == MCG_VOXEL_SHORT2 ? 4 : 3) mc_count_rows_kernel(RowsParams p) {
+__global__ void __launch_bounds__(RW_THREADS, 3) mc_count_rows_kernel(RowsParams p) {
     using T = typename Vox<VT>::T;
     __shared__ RowsSmem S;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
