@@ -130,8 +130,7 @@ __device__ __forceinline__ BrickPos slab_pos(long long b, int nbx, int nby, int 
 // into place; the volume's first and last words, partly outside its
 // allocation, are read voxel by voxel.  Rows outside the volume and voxels
 // with x outside [0, nx) are zero.  The stores are plain shared-memory
-// stores (WAIT is kept for the callers' cp.async bookkeeping); the caller's
-// barrier publishes the tile.
+// stores; the caller's barrier publishes the tile.
 template <int VT>
 __device__ __forceinline__ uint4 vol_word(const uint4 *__restrict__ gbase, const typename Vox<VT>::T *__restrict__ vol,
                                           long long k, long long klo, long long khi, int b0, long long N) {
@@ -151,7 +150,7 @@ __device__ __forceinline__ uint4 vol_word(const uint4 *__restrict__ gbase, const
     return make_uint4(u[0], u[1], u[2], u[3]);
 }
 
-template <int VT, int DX, int DY, int DZ, bool WAIT = true>
+template <int VT, int DX, int DY, int DZ>
 __device__ __forceinline__ void fill_tile(typename Vox<VT>::T *tile, const typename Vox<VT>::T *__restrict__ vol,
                                           int nx, int ny, int nz, int ox, int oy, int oz) {
     constexpr int B = Vox<VT>::bytes, VPW = 16 / B, WPR = DX / VPW, NWORDS = WPR * DY * DZ, UPV = B / 4;
@@ -192,7 +191,6 @@ __device__ __forceinline__ void fill_tile(typename Vox<VT>::T *tile, const typen
         }
         dst[i] = out;
     }
-    (void)WAIT;
 }
 
 // ---- normals (cu_kinect_fusion_v1.cu:3146-3225) -----------------------------------

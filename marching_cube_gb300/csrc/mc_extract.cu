@@ -24,17 +24,19 @@
 // A multi-CTA scan (one CTA per chunk of 256 bricks) turns brick counts into
 // 64-bit soup offsets and a list of active bricks (heaviest classes first).
 //
-// Pass 2 (generate) visits only active bricks, with a 2-stage TMA prefetch
-// of the brick + halo (36x10x10 voxels).  The same masks give a compact list
-// of occupied cubes with their vertex offsets; each thread then emits one
-// soup vertex (its cube and edge through a vertex map, or a binary search
-// over the list), computes the fused normal from the tile, and the 28-byte
-// records go out through a per-warp shared-memory stage as full coalesced
-// lines.  The three launches chain with programmatic dependent launch.
+// Pass 2 (generate) visits only active bricks, the tile of the next one (brick
+// + halo, 36x10x10 voxels) fetched by TMA as soon as the last use of this one's
+// is over.  The same masks give the occupied cubes with their vertex offsets
+// and the crossed edges; each crossed edge's record (position, voxel, fused
+// normal) is worked out once and the soup copied out of the records
+// (generate_shared), or, where those do not fit, each thread emits one soup
+// vertex (generate_brick).  The three launches chain with programmatic
+// dependent launch.
 //
 // When TMA cannot describe the volume (x row not a multiple of 16 bytes or an
-// unaligned base) the same kernels fill the tiles by 16-byte words of the
-// volume shifted into place (fill_tile).
+// unaligned base), and for batches, pass 1 is mc_count_rows_kernel, straight
+// from global memory, and generate fills the tiles TMA cannot by 16-byte words
+// of the volume shifted into place (fill_tile).
 //
 // Output order is deterministic: bricks in (bz, by, bx) order, cubes in
 // (z, y, x) order inside a brick, then the table slot -- the reference's
@@ -409,9 +411,9 @@ __global__ void __launch_bounds__(NT)
 // ---- batched extraction: shared definitions ----------------------------------------
 // Bricks of all volumes of a batch form one index space: volume v owns bricks
 // [brick_base, brick_base + nbricks).  A brick's volume is found by binary
-// search over the descriptor table; tiles come by TMA through the volume's
-// own tensor map (global memory) when TMA can describe it, by 16-byte words
-// shifted into place otherwise (fill_tile).  Soup offsets come from one scan over all
+// search over the descriptor table; generate's tiles come by TMA through the
+// volume's own tensor map (global memory) when TMA can describe it, by 16-byte
+// words shifted into place otherwise (fill_tile).  Soup offsets come from one scan over all
 // bricks; a volume's soup starts at the offset of its first brick, i.e. 3x
 // the triangles of the volumes before it.
 struct VolDesc {
@@ -954,8 +956,14 @@ struct GenParams {
 // the 1024^3 volume 1204 us instead of 1104.
 constexpr int SH_VERTS = 1536, SH_RECS = 608, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
 
-template <int VT, int NST>
+//
+// SHARED false: the adjoint's, which goes soup vertex by soup vertex and has no
+// records.  With the records' 24 KB float2 tiles leave room for three CTAs per
+// SM instead of four, and the adjoint of 768^3 voxels of spheres and noise
+// takes 2.21 ms instead of 2.15.
+template <int VT, int NST, bool SHARED = true>
 struct GenSmem {
+    static constexpr int MAPPED = SHARED ? SH_VERTS : BRICK_CUBES;  // soup vertices vmap holds
     static constexpr int STAGE_BYTES = pad128(GTILE * Vox<VT>::bytes);
     unsigned char tiles[NST][STAGE_BYTES];
     unsigned long long neg[ROWS], dead[ROWS];
@@ -968,22 +976,22 @@ struct GenSmem {
             unsigned char occ_ci[BRICK_CUBES];
         };
         struct {  // generate_shared: the records of crossed edges
-            unsigned int rec[SH_RECS * 7];
-            float nrm[SH_RECS * 3];
+            unsigned int rec[SHARED ? SH_RECS * 7 : 1];
+            float nrm[SHARED ? SH_RECS * 3 : 1];
         };
     };
-    unsigned int cubes[SH_CUBES];     // occupied cubes in order: cube | case << 11 | soup vertices before it << 19
-    uint2 slot[SH_SLOTS];             // the edges of a slot that are used (bits 0-31 of 33), its first record
+    unsigned int cubes[SHARED ? SH_CUBES : 1];  // occupied cubes in order: cube | case << 11 | soup vertices before it << 19
+    uint2 slot[SHARED ? SH_SLOTS : 1];  // the edges of a slot that are used (bits 0-31 of 33), its first record
     unsigned int occp[(BY + 2) * (BZ + 2)];  // occupied cubes of cube row (cy, cz) at (cz + 1) * (BY + 2) + cy + 1, zero around
     unsigned int elut[12];            // edge -> slot step | x step << 16
     unsigned int wtot[2][WARPS];
     unsigned short rowcube[CUBE_ROWS];  // occupied cubes before each cube row, and all
     unsigned int ncube;
     unsigned int first[(SH_RECS + 31) / 32];  // bit: the first record of a used slot
-    unsigned short used[SH_SLOTS + 1];  // the used slots, in order
+    unsigned short used[SHARED ? SH_SLOTS + 1 : 1];  // the used slots, in order
     alignas(16) signed char tri[256][16];  // read a row at a time as 16 bytes
     unsigned char nv[256];
-    unsigned short vmap[SH_VERTS + 1];     // soup vertex -> local cube << 4 | edge, when the brick has <= SH_VERTS;
+    unsigned short vmap[MAPPED + 1];       // soup vertex -> local cube << 4 | edge, when the brick has <= MAPPED;
                                            // generate_shared: -> record (one more entry is read, not used)
     long long sbrick[NST];                 // brick id, soup offset and origin of each stage's tile
     unsigned long long svbase[NST];
@@ -1014,7 +1022,7 @@ struct GenOut {
 // Occupied-cube list of a brick whose tile is in shared memory: S.occ_cube /
 // occ_ci / occ_off in (z, y, x) order, S.nocc entries, S.total soup
 // vertices, and S.vmap (each vertex's cube and edge) when the brick has at
-// most SH_VERTS of them.  Called by
+// most MAPPED of them.  Called by
 // every thread (contains __syncthreads); the list is valid after return.
 template <int VT, class Smem>
 __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T *tile, int nx, int ny, int zlim,
@@ -1077,7 +1085,7 @@ __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T
         // index << 4 | edge, the edge of output slot k of triangle j being
         // tri[3j + 2 - k] (cu_marching_cubes_v1.cu:322-333); cube offsets are
         // multiples of 3, so a vertex's slot is its index mod 3
-        if (S.total <= SH_VERTS) {
+        if (S.total <= Smem::MAPPED) {
             const unsigned int nocc = S.nocc;
             for (unsigned int i = tid; i < nocc; i += THREADS) {
                 const unsigned int off = S.occ_off[i], ci = S.occ_ci[i], nvc = S.nv[ci];
@@ -1190,7 +1198,7 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
 
         occupied_list<VT>(S, tile, nx, ny, o.zlim, x0, y0, z0);
         const unsigned int nocc = S.nocc, T_brick = S.total;
-        const bool use_map = T_brick <= SH_VERTS;
+        const bool use_map = T_brick <= Smem::MAPPED;
 
         // emission: one soup vertex per thread, warps take 32 consecutive vertices
         for (unsigned int v0 = warp * 32; v0 < T_brick; v0 += THREADS) {
@@ -1661,7 +1669,7 @@ __device__ __forceinline__ void backward_brick(Smem &S, const typename Vox<VT>::
     const int tid = threadIdx.x;
     occupied_list<VT>(S, tile, nx, ny, zlim, x0, y0, z0);
     const unsigned int nocc = S.nocc, T_brick = S.total;
-    const bool use_map = T_brick <= SH_VERTS;
+    const bool use_map = T_brick <= Smem::MAPPED;
     for (unsigned int v = tid; v < T_brick; v += THREADS) {
         const unsigned long long gv = vbase + v;
         if ((long long)gv >= n_grad) break;
@@ -1708,7 +1716,8 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
     using V = Vox<VT>;
     using T = typename V::T;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    GenSmem<VT, GEN_STAGES> &S = *reinterpret_cast<GenSmem<VT, GEN_STAGES> *>(smem_raw);
+    using Smem = GenSmem<VT, GEN_STAGES, MODE == 0>;
+    Smem &S = *reinterpret_cast<Smem *>(smem_raw);
     const T *__restrict__ vol = static_cast<const T *>(p.vol);
     const int tid = threadIdx.x;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
@@ -2692,7 +2701,7 @@ void launch_classify_x(int G, const CUtensorMap &map, const CUtensorMap &hmap, c
 
 template <int VT, bool TMA, int MODE = 0>
 void launch_generate_t(const CUtensorMap &map, const GenParams &p, const Geometry &g, int sms, cudaStream_t s) {
-    const size_t smem = sizeof(GenSmem<VT, GEN_STAGES>);
+    const size_t smem = sizeof(GenSmem<VT, GEN_STAGES, MODE == 0>);
     static int occ = 0;
     if (!occ) occ = occupancy(mc_generate_kernel<VT, TMA, MODE>, THREADS, smem);
     long long grid = (long long)sms * occ;

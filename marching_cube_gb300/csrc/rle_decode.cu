@@ -4,14 +4,15 @@
 // Only the compressed image crosses the host link: it is copied to the
 // device in slabs of whole slices on a copy stream while earlier slabs
 // expand (from a file: pieces read by host threads into pinned buffers while
-// the GPU copies and expands the pieces before).  One CTA expands one
-// z-slice, 4096 16-bit words at a time:
+// the GPU copies and expands the pieces before).  One CTA expands 4096 16-bit
+// words of a z-slice (and further ones what is beyond each RD_PART voxels):
 //  * every word is a record header, or the first or second word of a
 //    literal; which one follows from the words before it through a
 //    three-state machine (header -> header, or -> literal 1 for kinds 0 and
 //    3; literal 1 -> literal 2 -> header).  Each thread composes the state
-//    maps of its 16 words and a block scan of the compositions (carrying the
-//    state from the chunk before) gives every word its state;
+//    maps of its 16 words and a block scan of the compositions, from the
+//    chunk's entry state (rle_summarize, rle_slice_scan), gives every word its
+//    state;
 //  * a block scan of the run lengths of the headers places each run in the
 //    slice; runs go to shared memory as (start, voxel);
 //  * the chunk's voxels are written by all threads, 16 bytes at a time, each
