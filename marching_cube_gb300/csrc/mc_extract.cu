@@ -687,12 +687,14 @@ __global__ void __launch_bounds__(RW_THREADS, 3) mc_count_rows_kernel(RowsParams
     __syncthreads();
     pdl_wait();
     VolCache vc;
-    unsigned int drawn = 0;
-    if (lane == 0) drawn = atomicAdd(p.ticket, 1u);
+    // the first draw is the warp's number, the others come from the counter (if
+    // there are any: 18 -> 10 us for 57 x 352 x 138 voxels, a brick a warp)
+    const unsigned int warps = gridDim.x * RW_WARPS;
+    unsigned int drawn = blockIdx.x * RW_WARPS + warp;
     for (;;) {
         const long long b0 = (long long)__shfl_sync(0xffffffffu, drawn, 0) * p.draw;
         if (b0 >= p.nbricks) break;
-        if (lane == 0) drawn = atomicAdd(p.ticket, 1u);
+        if (lane == 0) drawn = (long long)warps * p.draw < p.nbricks ? warps + atomicAdd(p.ticket, 1u) : 0xffffffffu;
         for (int k = 0; k < p.draw && b0 + k < p.nbricks; ++k) {
             const long long b = b0 + k;
             unsigned int tri, occ;
