@@ -953,12 +953,12 @@ struct GenParams {
 
 // generate_shared's split: soup vertices and records in hand at a time,
 // occupied cubes per brick, slots (see there).  As many as four CTAs per SM
-// leave room for: with 1280 soup vertices and 512 records the 64-volume batch
+// leave room for (2048 soup vertices and 608 records take 86 us instead of 79
+// for 512^3 voxels): with 1280 soup vertices and 512 records the 64-volume batch
 // takes 267 us instead of 244 at the same occupancy, and at three CTAs per SM
 // the 1024^3 volume 1204 us instead of 1104.
-constexpr int SH_VERTS = 1536, SH_RECS = 608, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
+constexpr int SH_VERTS = 1600, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
 
-//
 // SHARED false: the adjoint's, which goes soup vertex by soup vertex and has no
 // records.  With the records' 24 KB float2 tiles leave room for three CTAs per
 // SM instead of four, and the adjoint of 768^3 voxels of spheres and noise
@@ -1533,21 +1533,24 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
         __syncthreads();
     }
     if (T_brick >= (1u << 13) || (long long)(vbase + T_brick) > o.cap) return false;
+    // soup vertices before layer z: its first cube's
+    auto verts = [&](int z) -> unsigned int {
+        const unsigned int i = z < BZ ? S.rowcube[z * BY] : nocc;
+        return i < nocc ? S.cubes[i] >> 19 : T_brick;
+    };
+    // a layer that is too much by itself is found before the others are done
+    // (these are the heaviest bricks, and the launch waits for the last one)
+    if (T_brick > SH_VERTS && __any_sync(full, lane < BZ && verts(lane + 1) - verts(lane) > (unsigned int)SH_VERTS))
+        return false;
     for (int za = 0, zb = BZ; za < BZ; za = zb, zb = BZ) {
         unsigned int i0 = 0, i1 = nocc, va = 0, nT = T_brick;
         if (T_brick > SH_VERTS) {
-            // the layers from za on that fit; soup vertices before layer z: its first cube's
-            auto verts = [&](int z) -> unsigned int {
-                const unsigned int i = z < BZ ? S.rowcube[z * BY] : nocc;
-                return i < nocc ? S.cubes[i] >> 19 : T_brick;
-            };
+            // the layers from za on that fit
             va = verts(za);
-            while (zb > za && verts(zb) - va > (unsigned int)SH_VERTS) --zb;
-            if (zb == za) return false;  // one layer is too much
+            while (verts(zb) - va > (unsigned int)SH_VERTS) --zb;
             i0 = S.rowcube[za * BY];
             i1 = zb < BZ ? S.rowcube[zb * BY] : nocc;
             nT = verts(zb) - va;
-            if (nT == 0) continue;
             count_slots(za, zb);
             __syncthreads();
             R = number_slots();

@@ -1,5 +1,5 @@
 """The soup from records of crossed edges: bricks around what is taken in
-hand at a time (1536 soup vertices, 608 records, 768 occupied cubes) -- none,
+hand at a time (1600 soup vertices, 640 records, 768 occupied cubes) -- none,
 few, exactly one plane of 1536, several planes in every direction (several
 groups of layers), more than fit (each soup vertex for itself) -- one brick and
 ragged neighbours, a cell whose reciprocal is not used (significand all ones)
@@ -83,3 +83,17 @@ def test_capacity_and_subsets(mcg, keep):
             m = cap // 3 if k == "tri_cube" else cap
             assert torch.equal(out[k][:m], parts[k][:m])
             assert bool((out[k][m:] == 7).all())
+
+
+@pytest.mark.parametrize("upwards", [True, False])
+@pytest.mark.parametrize("n", [50, 63, 64, 65, 66, 67, 68, 90])
+def test_isolated_voxels(mcg, orc, n, upwards):
+    """Isolated negative voxels, 24 soup vertices and 10 records each, around the
+    64 whose records fit, in the lower or the upper layers of the brick."""
+    at = [(z, y, x) for z in (1, 4, 7) for y in (1, 4, 7) for x in range(2, 32, 3)]
+    vol = np.full((9, 9, 33, 2), 1000, np.int16)
+    for z, y, x in (at if upwards else at[::-1])[:n]:
+        vol[z, y, x, 0] = -700
+    o = orc.mc_extract(vol, 0.01)
+    assert len(o["soup"]) == 24 * n
+    assert_same_mesh(gpu_extract(mcg, vol, 0.01), o)
