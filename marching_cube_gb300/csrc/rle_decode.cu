@@ -140,15 +140,17 @@ __device__ __forceinline__ Sum sum_block_scan(const Sum &x, Sum *s_w, Sum *total
 
 struct Dir {
     const long long *off, *len;  // byte range of each slice's records in the image
-    const long long *cbase;      // first chunk of each slice (nz + 1 entries)
-    int nz;
+    const long long *cbase;      // first chunk of each slice (one entry more than slices)
+    int z0, z1;                  // the slab: only its entries, and cbase[z1], are there yet
 };
 
-// slice of chunk c, and its words [c0, c0 + cw) of nw
+// slice of chunk c of the slab, and its words [c0, c0 + cw) of nw
 __device__ __forceinline__ void rd_chunk(const Dir &d, long long c, int *z, long long *c0, int *cw, long long *nw) {
-    // last slice with cbase <= c (cbase[0] <= c): 32 probes a step
+    // the slab's last slice with cbase <= c (cbase[z0] <= c): 32 probes a step.
+    // Entries past the slab may be another image's (a file's directory comes
+    // piece by piece), so they are not looked at.
     const int lane = threadIdx.x & 31;
-    int lo = 0, n = d.nz;
+    int lo = d.z0, n = d.z1 - d.z0;
     while (n > 1) {
         const int step = (n + 31) / 32, i = lane * step;
         const unsigned m = __ballot_sync(0xffffffffu, i < n && d.cbase[lo + i] <= c);
@@ -527,7 +529,7 @@ cudaError_t launch_expand(mcg_context *ctx, const Slab &sl, const long long *cba
                           cudaStream_t s) {
     if (sl.z1 <= sl.z0) return cudaSuccess;
     const int nz = ctx->rd_dir_n;
-    const Dir d{ctx->rd_dir, ctx->rd_dir + nz, ctx->rd_dir + 2 * nz, nz};
+    const Dir d{ctx->rd_dir, ctx->rd_dir + nz, ctx->rd_dir + 2 * nz, sl.z0, sl.z1};
     const long long cf = cbase_host[sl.z0], nc = cbase_host[sl.z1] - cf;
     Sum *sums = reinterpret_cast<Sum *>(ctx->rd_sum);
     unsigned char *entry = ctx->rd_entry;
