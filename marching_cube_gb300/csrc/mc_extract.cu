@@ -1107,14 +1107,13 @@ __device__ __forceinline__ void occupied_list(Smem &S, const typename Vox<VT>::T
 // The soup vertex on the edge from node ga (value f0) to node gb (f1) of the
 // brick at (x0, y0, z0): its position, voxel, that voxel's tsdf and w (also
 // scattered to ver_voxel if given), and its normal.  rcell: mcg_div_reciprocal
-// of the cell, or 0.
-template <int VT>
+// of the cell, or 0.  NEAR: 16-bit distances and mcg_between_nodes.
+template <int VT, bool NEAR>
 __device__ __forceinline__ void make_vertex(const typename Vox<VT>::T *tile,
                                             const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz,
                                             float cell, float rcell, int x0, int y0, int z0, float f0, float f1,
-                                            const int ga[3],
-                                            const int gb[3], bool normals, int16_t *ver_voxel, float P[3], int vox[3],
-                                            short &vt, short &vw, float3 &nrm) {
+                                            const int ga[3], const int gb[3], bool normals, int16_t *ver_voxel,
+                                            float P[3], int vox[3], short &vt, short &vw, float3 &nrm) {
     using V = Vox<VT>;
     using T = typename V::T;
     // getNodeCoo (:243-254) and vertex_interp (:256-264)
@@ -1138,16 +1137,18 @@ __device__ __forceinline__ void make_vertex(const typename Vox<VT>::T *tile,
 #pragma unroll
         for (int d = 0; d < 3; ++d) pf[d] = P[d] / cell;
     }
-    // 16-bit distances: 0 <= t <= 1, so the voxel lies between the one before ga
+    // NEAR: 0 <= t <= 1, so the voxel lies between the one before ga
     // (by rounding) and gb, and the normal's first sample between ga and gb:
     // inside the tile but for a voxel below its origin, inside the volume but
-    // for a last sample past its end.  Floats can give any t.
+    // for a last sample past its end.  Floats can give any t, and other cells
+    // and sides any position, NaN and infinite ones (which convert to 0 and
+    // the largest int) among them.
     bool inside = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         vox[d] = (int)floorf(pf[d] - 0.5f);
-        if (VT == MCG_VOXEL_SHORT2) inside &= vox[d] >= org[d];
-        else inside &= vox[d] >= 0 && vox[d] < dims[d] && vox[d] - org[d] >= 0 && vox[d] - org[d] < tdim[d];
+        if (NEAR) inside &= vox[d] >= org[d];
+        else inside &= vox[d] < dims[d] && mcg_in_tile(vox[d], org[d], tdim[d]);
     }
     if (inside) {
         const T vv = tile[tidx(vox[0] - org[0], vox[1] - org[1], vox[2] - org[2])];
@@ -1168,9 +1169,9 @@ __device__ __forceinline__ void make_vertex(const typename Vox<VT>::T *tile,
         const float fx = pf[0], fy = pf[1], fz = pf[2];
         const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
         const int lx = ix - org[0], ly = iy - org[1], lz = iz - org[2];
-        if (ix + 1 < nx && iy + 1 < ny && iz + 1 < nz &&
-            (VT == MCG_VOXEL_SHORT2 ||
-             (lx >= 0 && ly >= 0 && lz >= 0 && lx + 1 < TX && ly + 1 < TY && lz + 1 < TZ))) {
+        if ((NEAR || (mcg_in_tile(ix, org[0], TX - 1) && mcg_in_tile(iy, org[1], TY - 1) &&
+                      mcg_in_tile(iz, org[2], TZ - 1))) &&
+            ix + 1 < nx && iy + 1 < ny && iz + 1 < nz) {
             const T smp[8] = {tile[tidx(lx, ly, lz)],         tile[tidx(lx + 1, ly, lz)],
                               tile[tidx(lx + 1, ly + 1, lz)], tile[tidx(lx, ly + 1, lz)],
                               tile[tidx(lx, ly, lz + 1)],     tile[tidx(lx + 1, ly, lz + 1)],
@@ -1244,8 +1245,9 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
                     V::f(tile[tidx(lcx + TXO + c_cx(bb), lcy + TYO + c_cy(bb), lcz + TZO + c_cz(bb))]);
                 const int ga[3] = {gx + c_cx(a), gy + c_cy(a), gz + c_cz(a)};
                 const int gb[3] = {gx + c_cx(bb), gy + c_cy(bb), gz + c_cz(bb)};
-                make_vertex<VT>(tile, vol, nx, ny, nz, cell, 0.0f, x0, y0, z0, f0, f1, ga, gb, o.normals != nullptr,
-                                vbase + v < (unsigned long long)o.cap ? o.ver_voxel : nullptr, P, vox, vt, vw, nrm);
+                make_vertex<VT, false>(tile, vol, nx, ny, nz, cell, 0.0f, x0, y0, z0, f0, f1, ga, gb,
+                                       o.normals != nullptr,
+                                       vbase + v < (unsigned long long)o.cap ? o.ver_voxel : nullptr, P, vox, vt, vw, nrm);
             }
             // ---- coalesced stores through the warp stage ----
             const unsigned long long g0 = vbase + v0;  // first record of this warp
@@ -1326,8 +1328,10 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
 // and four CTAs per SM instead of two stages).  Warps wait for barriers more
 // than for anything else: with up to three cubes a thread in step 2, one scan
 // and two barriers instead of those per 256 cubes, 79 and 1061 us.  Returns false (the caller
-// runs generate_brick) where a layer or its records do not fit, or the output
-// ends inside the brick; else tile_done() has been called by every thread
+// runs generate_brick) where a layer or its records do not fit, the output
+// ends inside the brick, or a vertex might lie outside its edge's nodes
+// (mcg_between_nodes: the records' voxels and samples are not tested one by
+// one, which costs 1 % of 512^3 to 1024^3 voxels); else tile_done() has been called by every thread
 // between the last use of the tile and the last copy, so that the next brick's
 // tile is fetched meanwhile.  Called by every thread (contains __syncthreads).
 __device__ __forceinline__ unsigned int shared_elut(int e) {
@@ -1386,6 +1390,8 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
     using V = Vox<VT>;
     const unsigned int full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr bool NEAR = VT == MCG_VOXEL_SHORT2;
+    if (NEAR && !mcg_between_nodes(cell, max(max(nx, ny), nz))) return false;
     // (float distances can make a position infinite)
     const float rcell = VT == MCG_VOXEL_SHORT2 ? mcg_div_reciprocal(cell) : 0.0f;
     if (tid < ROWS) {
@@ -1599,8 +1605,8 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             int vox[3];
             short vt = 0, vw = 0;
             float3 nrm = make_float3(0.f, 0.f, 0.f);
-            make_vertex<VT>(tile, vol, nx, ny, nz, cell, rcell, x0, y0, z0, down ? hi : lo, down ? lo : hi, ga, gb,
-                            o.normals != nullptr, o.ver_voxel, P, vox, vt, vw, nrm);
+            make_vertex<VT, NEAR>(tile, vol, nx, ny, nz, cell, rcell, x0, y0, z0, down ? hi : lo, down ? lo : hi, ga,
+                                  gb, o.normals != nullptr, o.ver_voxel, P, vox, vt, vw, nrm);
             unsigned int *rec = S.rec + 7 * r;
             rec[0] = __float_as_uint(P[0]);
             rec[1] = __float_as_uint(P[1]);
@@ -2330,7 +2336,7 @@ __global__ void __launch_bounds__(FGeo<FG>::NT, MINB) mc_fused_kernel(const __gr
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     vox[d] = (int)floorf(pf[d] - 0.5f);
-                    inside &= vox[d] >= 0 && vox[d] < dims[d] && vox[d] - orgv[d] >= 0 && vox[d] - orgv[d] < tdim[d];
+                    inside &= vox[d] < dims[d] && mcg_in_tile(vox[d], orgv[d], tdim[d]);
                 }
                 if (inside) {
                     const T vv = tile[ftidx<FG>(vox[0] - x0, vox[1] - y0, vox[2] - z0)];
@@ -2351,8 +2357,8 @@ __global__ void __launch_bounds__(FGeo<FG>::NT, MINB) mc_fused_kernel(const __gr
                     const float fx = pf[0], fy = pf[1], fz = pf[2];
                     const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
                     const int lx = ix - x0, ly = iy - y0, lz = iz - z0;
-                    if (ix + 1 < nx && iy + 1 < ny && iz + 1 < nz && lx >= 0 && ly >= 0 && lz >= 0 &&
-                        lx + 1 < FTX && ly + 1 < FTY && lz + 1 < FTZ) {
+                    if (mcg_in_tile(ix, x0, FTX - 1) && mcg_in_tile(iy, y0, FTY - 1) && mcg_in_tile(iz, z0, FTZ - 1) &&
+                        ix + 1 < nx && iy + 1 < ny && iz + 1 < nz) {
                         const T smp[8] = {tile[ftidx<FG>(lx, ly, lz)],         tile[ftidx<FG>(lx + 1, ly, lz)],
                                           tile[ftidx<FG>(lx + 1, ly + 1, lz)], tile[ftidx<FG>(lx, ly + 1, lz)],
                                           tile[ftidx<FG>(lx, ly, lz + 1)],     tile[ftidx<FG>(lx + 1, ly, lz + 1)],

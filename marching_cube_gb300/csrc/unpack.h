@@ -50,3 +50,21 @@ MCG_HD float mcg_div_exact(float a, float b, float y) {
     const float q1 = fmaf(fmaf(-q, b, a), y, q);
     return fmaf(fmaf(-q1, b, a), y, q1);
 }
+
+// Whether a position interpolated between the nodes (i + 0.5) cell and
+// (i + 1.5) cell of a volume whose longest side is `side`, divided by cell,
+// lies between i + 0.25 and i + 1.75: the voxel of a vertex (rounded down, less
+// a half) is then i - 1, i or i + 1 and the first sample of its normal i or
+// i + 1.  Every step of the interpolation is monotonic, so the position stays
+// between the two nodes as rounded, and node and quotient are each off by at
+// most 2^-24 of a coordinate below 2^21, an eighth.  At 2^22 that reaches the
+// next voxel, with a subnormal cell anything, and where (side + 1) cell
+// overflows positions are infinite or NaN (tests/test_between_nodes.py).
+MCG_HD bool mcg_between_nodes(float cell, int side) {
+    return cell > 1e-25f && cell < 1e25f && side <= (1 << 21);
+}
+
+// org <= i < org + n, for any i
+MCG_HD bool mcg_in_tile(int i, int org, int n) {
+    return (unsigned int)i - (unsigned int)org < (unsigned int)n;
+}
