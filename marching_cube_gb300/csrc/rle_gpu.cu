@@ -18,10 +18,15 @@
 //      follows it;  rle_slices: the slices' offsets and the image's size;
 //   3. rle_emit: per chunk with records, from its bits, the voxels at record
 //      starts only; the bytes are laid out in shared memory and leave coalesced.
-// The image then crosses to the host in one copy.
+// The image then crosses to the host in one copy.  Scratch is a bit per voxel
+// (each slice's rounded up to words) and 24 bytes per chunk, of as many slices
+// as fit RSCRATCH, or memory; with more slices, passes 1 and 2 run once more
+// before pass 3.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
+
+#include <algorithm>
 
 #include "mcg_internal.h"
 
@@ -32,6 +37,7 @@ constexpr int RT = 256;            // threads per CTA
 constexpr int RCHUNK = 4096;       // voxels per chunk
 constexpr int RWORDS = RCHUNK / 32;
 constexpr int RWARPS = RT / 32;
+constexpr long long RSCRATCH = 288ll << 20;  // bytes of run-start bits and chunk records at a time: 2^31 voxels'
 constexpr int kMaxRun = 0x3fff;
 
 // record kind of a record whose first voxel is v (put_run in rle.cpp)
@@ -59,7 +65,8 @@ struct RleChunk {
 // 101, 5, 2 and 53 us.  This one took 138 us with the run starts' kinds and
 // words worked out for every 128 voxels, also where no run starts.
 __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
-                                               RleChunk *__restrict__ chunks, uint32_t *__restrict__ marks, int vec) {
+                                               RleChunk *__restrict__ chunks, uint32_t *__restrict__ marks, int cwords,
+                                               int vec) {
     constexpr int Q = RCHUNK / RT / 4;  // 16-byte words per lane
     __shared__ int s_first[RWARPS], s_last[RWARPS], s_bytes[RWARPS];
     const bool lossless = lossless_i != 0;
@@ -84,7 +91,8 @@ __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol,
     uint32_t before = w0 > 0 && w0 <= xy ? __ldg(sl + w0 - 1) : 0u;
     const uint32_t differ = lossless ? 0xffffffffu : 0xffffu;
     int bytes = 0, first = INT32_MAX, last = -1;
-    uint32_t *out = marks + c * RWORDS + warp * 4 * Q;
+    const int word0 = warp * 4 * Q;  // cwords of a chunk's words are kept (those of a slice shorter than a chunk)
+    uint32_t *out = marks + c * cwords;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int i = w0 + 128 * q + 4 * lane;
@@ -114,7 +122,8 @@ __global__ void __launch_bounds__(RT) rle_mark(const uint32_t *__restrict__ vol,
             word |= __shfl_xor_sync(0xffffffffu, word, 2);
             word |= __shfl_xor_sync(0xffffffffu, word, 4);
         }
-        if ((lane & 7) == 0) out[4 * q + (lane >> 3)] = word;
+        const int at = word0 + 4 * q + (lane >> 3);
+        if ((lane & 7) == 0 && at < cwords) out[at] = word;
     }
     bytes = __reduce_add_sync(0xffffffffu, bytes);
     first = __reduce_min_sync(0xffffffffu, first);
@@ -248,7 +257,7 @@ struct RleEmit {
 
 __global__ void __launch_bounds__(ET) rle_emit(const uint32_t *__restrict__ vol, int xy, int nchunks, int lossless_i,
                                                const RleChunk *__restrict__ chunks, const uint32_t *__restrict__ marks,
-                                               const unsigned long long *__restrict__ slice_bytes,
+                                               int cwords, const unsigned long long *__restrict__ slice_bytes,
                                                const unsigned long long *__restrict__ slice_off,
                                                uint8_t *__restrict__ img) {
     __shared__ RleEmit S;
@@ -256,7 +265,7 @@ __global__ void __launch_bounds__(ET) rle_emit(const uint32_t *__restrict__ vol,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long c = blockIdx.x;
     const int z = (int)(c / nchunks), c0 = (int)(c - (long long)z * nchunks) * RCHUNK;
-    const uint32_t word = marks[c * RWORDS + tid];
+    const uint32_t word = tid < cwords ? marks[c * cwords + tid] : 0u;
     const RleChunk r = chunks[c];
     const unsigned long long so = slice_off[z];  // even: 40, then 4 and even record bytes a slice
     if (c0 == 0 && tid < 2) reinterpret_cast<uint16_t *>(img + so)[tid] = (uint16_t)(slice_bytes[z] >> (16 * tid));
@@ -346,22 +355,38 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    const long long nchunks = (xy + RCHUNK - 1) / RCHUNK, total = nchunks * nz;
-    if (total > INT32_MAX) return MCG_ERR_TOO_LARGE;  // one CTA each
-    if (!ensure(&ctx->rle_slices, &ctx->rle_slices_cap, (size_t)2 * nz + 1) ||
-        !ensure(&ctx->rle_chunks, &ctx->rle_chunks_cap, (size_t)total * sizeof(RleChunk)) ||
-        !ensure(&ctx->rle_marks, &ctx->rle_marks_cap, (size_t)total * RWORDS))
+    const long long nchunks = (xy + RCHUNK - 1) / RCHUNK;
+    const int cwords = nchunks == 1 ? (int)((xy + 31) / 32) : RWORDS;  // words of marks per chunk
+    const long long slice_scratch = nchunks * (long long)(sizeof(RleChunk) + 4 * cwords);
+    long long per = std::min<long long>(nz, std::max(1ll, RSCRATCH / slice_scratch));  // slices at a time
+    if (!ensure(&ctx->rle_slices, &ctx->rle_slices_cap, (size_t)2 * nz + 1))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
+    auto scratch = [&]() {  // for `per` slices, fewer where that cannot be had
+        while (!ensure(&ctx->rle_chunks, &ctx->rle_chunks_cap, (size_t)(per * nchunks) * sizeof(RleChunk)) ||
+               !ensure(&ctx->rle_marks, &ctx->rle_marks_cap, (size_t)(per * nchunks * cwords))) {
+            cudaGetLastError();
+            if (per == 1) return false;
+            per = (per + 1) / 2;
+        }
+        return true;
+    };
+    if (!scratch()) return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     unsigned long long *d_bytes = ctx->rle_slices, *d_off = ctx->rle_slices + nz;
-    RleChunk *chunks = reinterpret_cast<RleChunk *>(ctx->rle_chunks);
     const uint32_t *v = static_cast<const uint32_t *>(vol);
     const int vec = ((reinterpret_cast<uintptr_t>(vol) & 15u) == 0 && xy % 4 == 0) ? 1 : 0;
     const int ll = lossless ? 1 : 0;
-    rle_mark<<<(unsigned int)total, RT, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks, vec);
-    rle_place<<<nz, 32, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, d_bytes);
+    // passes 1 and 2 of the slices from z on
+    auto mark = [&](long long z, long long n) {
+        RleChunk *chunks = reinterpret_cast<RleChunk *>(ctx->rle_chunks);
+        rle_mark<<<(unsigned int)(n * nchunks), RT, 0, s>>>(v + z * xy, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks,
+                                                            cwords, vec);
+        rle_place<<<(unsigned int)n, 32, 0, s>>>(v + z * xy, (int)xy, (int)nchunks, ll, chunks, d_bytes + z);
+    };
+    for (long long z = 0; z < nz; z += per) mark(z, std::min(per, nz - z));
     rle_slices<<<1, RT, 0, s>>>(d_bytes, nz, d_off);
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
+    bool again = false;  // the marks are not there any more
     unsigned long long o = 0;
     e = cudaMemcpyAsync(&o, d_off + nz, sizeof(o), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -370,9 +395,26 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
         *size = (int64_t)o;
         return query ? MCG_OK : MCG_ERR_CAPACITY;
     }
-    if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
-    rle_emit<<<(unsigned int)total, ET, 0, s>>>(v, (int)xy, (int)nchunks, ll, chunks, ctx->rle_marks, d_bytes, d_off,
-                                                ctx->rle_image);
+    if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) {
+        // the image before the scratch, then what is left for that
+        cudaGetLastError();
+        cudaFree(ctx->rle_chunks);
+        cudaFree(ctx->rle_marks);
+        ctx->rle_chunks = nullptr;
+        ctx->rle_marks = nullptr;
+        ctx->rle_chunks_cap = ctx->rle_marks_cap = 0;
+        if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o) || !scratch())
+            return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
+        again = true;
+    }
+    for (long long z = 0; z < nz; z += per) {
+        const long long n = std::min(per, nz - z);
+        if (again || per < nz) mark(z, n);
+        rle_emit<<<(unsigned int)(n * nchunks), ET, 0, s>>>(v + z * xy, (int)xy, (int)nchunks, ll,
+                                                            reinterpret_cast<RleChunk *>(ctx->rle_chunks),
+                                                            ctx->rle_marks, cwords, d_bytes + z, d_off + z,
+                                                            ctx->rle_image);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     // header (:1303-1310), then the slices
