@@ -1043,13 +1043,13 @@ mcg_status mcg_integrate_frames(mcg_context *ctx, void *vol, int32_t voxel_type,
     // One frame, or scratch that cannot be had (no memory; inside a stream
     // capture, not sized by an earlier call of the same shapes): frame by frame.
     bool together = most > 1 && nblocks <= (size_t)(UINT32_MAX / 16);
+    const cudaError_t e = cudaSetDevice(ctx->device);
+    if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     if (together && mcg_capturing(s)) {
         together = ctx->depth_scaled_cap >= (size_t)pixels * most && ctx->integ_tiles_cap >= ntiles * most &&
                    ctx->integ_blocks_cap >= nblocks && ctx->integ_masks_cap >= nblocks && ctx->integ_count_cap >= 1;
         ctx->integ_captured = ctx->integ_captured || together;
     } else if (together) {
-        const cudaError_t e = cudaSetDevice(ctx->device);
-        if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
         together = ensure_integ(ctx, &ctx->depth_scaled, &ctx->depth_scaled_cap, (size_t)pixels * most) &&
                    ensure_integ(ctx, &ctx->integ_tiles, &ctx->integ_tiles_cap, ntiles * most) &&
                    ensure_integ(ctx, &ctx->integ_blocks, &ctx->integ_blocks_cap, nblocks) &&
