@@ -780,6 +780,11 @@ __global__ void __launch_bounds__(BW_THREADS) integrate_backward_kernel(IntegBwP
 
 Intr intr_of(const mcg_intrinsic *k) { return Intr{k->fx, k->fy, k->cx, k->cy}; }
 
+// Room for the depth tiles of any image of so many pixels (one column of
+// pixels has most: two tiles for eight), so that a stream capture needs an
+// earlier call of as many pixels only, as for the depths themselves.
+size_t tile_room(long long pixels) { return (size_t)(pixels / 4 + 2); }
+
 // ensure() for integrate's scratch: what a captured graph may refer to is not freed
 template <class T>
 bool ensure_integ(mcg_context *ctx, T **ptr, size_t *cap, size_t n) {
@@ -927,7 +932,7 @@ static mcg_status integrate_impl(mcg_context *ctx, void *vol, int32_t voxel_type
     const long long nblocks = nbx * nby * nbz;
     if (nblocks > (long long)(UINT32_MAX / 16)) return MCG_ERR_TOO_LARGE;  // 32-bit work items
     const dim3 b2(32, TILE_H), g2((w + 31) / 32, (h + TILE_H - 1) / TILE_H);
-    const size_t ntiles = (size_t)2 * g2.x * g2.y;
+    const size_t ntiles = tile_room((long long)w * h);
     // inside a stream capture nothing may be allocated: an earlier call of
     // the same shapes outside the capture has sized every buffer
     if (mcg_capturing(s)) {
@@ -1037,7 +1042,7 @@ mcg_status mcg_integrate_frames(mcg_context *ctx, void *vol, int32_t voxel_type,
     cudaStream_t s = (cudaStream_t)stream;
     const long long pixels = (long long)w * h;
     const size_t nblocks = (size_t)((nx + IB - 1) / IB) * ((ny + IB - 1) / IB) * ((nz + IB - 1) / IB);
-    const size_t ntiles = (size_t)2 * ((w + 31) / 32) * ((h + TILE_H - 1) / TILE_H);
+    const size_t ntiles = tile_room(pixels);
     // frames a pass: 256 MB of ray-length depth at most
     const int most = (int)std::min<long long>({n_frames, FRAMES, std::max(1ll, (64ll << 20) / pixels)});
     // One frame, or scratch that cannot be had (no memory; inside a stream

@@ -75,3 +75,16 @@ def test_captured_frames(mcg, orc, fresh, warm, vtype):
     loop.replay()
     loop.replay()
     assert all(bool((o == 7).all()) for o in other)
+
+
+@pytest.mark.parametrize("warm,image", [((8, 64), (64, 8)), ((3, 300), (300, 3)), ((40, 40), (200, 8))])
+@pytest.mark.parametrize("frames", [FRAMES, 1])
+def test_capture_after_an_image_of_as_many_pixels(mcg, orc, fresh, warm, image, frames):
+    """An earlier call of as many pixels sizes the scratch, whatever their layout."""
+    loop = Loop(mcg, orc, image, torch.int16)
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        mcg._integrate_frames(loop.v, loop.k, loop.pt[:frames], torch.zeros((frames, *warm), device="cuda"), None, False)
+        st.synchronize()
+        loop.capture(st)
+    loop.replay()
