@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(NT)
     if (S.abort && tid == 0) {
         atomicOr(flags, 1u);
         // give loads still in flight a bounded chance to land before exit
-        for (int s = 0; s < CSTAGES; ++s) mbar_wait(&S.bars[s], 0, 100000000ull);
+        for (int s = 0; s < CSTAGES; ++s) mbar_drain(&S.bars[s]);
     }
 }
 
@@ -1875,7 +1875,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
     }
     if (S.abort && tid == 0) {
         atomicOr(&p.totals->flags, 1u);
-        for (int s = 0; s < GEN_STAGES; ++s) mbar_wait(&S.bars[s], 0, 100000000ull);
+        for (int s = 0; s < GEN_STAGES; ++s) mbar_drain(&S.bars[s]);
     }
     // the last CTA out resets the work counter for the next launch over the
     // same list and reports the flags to the host copy
@@ -2436,7 +2436,7 @@ __global__ void __launch_bounds__(FGeo<FG>::NT, MINB) mc_fused_kernel(const __gr
     if (tid == 0) {
         if (S.abort) {
             atomicOr(&p.totals->flags, 1u);
-            mbar_wait(&S.bar, 0, 100000000ull);  // give a load still in flight a bounded chance to land
+            mbar_drain(&S.bar);
         }
         if (my_tris) atomicAdd(&p.totals->triangles, my_tris);
         if (my_occ) atomicAdd(&p.totals->occupied, my_occ);
@@ -2587,7 +2587,7 @@ __global__ void __launch_bounds__(THREADS, 4)
     }
     if (S.abort && tid == 0) {
         atomicOr(&totals->flags, 1u);
-        mbar_wait(&S.bars[0], phase, 100000000ull);
+        mbar_drain(&S.bars[0]);
     }
     // the last CTA out folds the flags into the mapped host copy, where the
     // batch's scan put the count launch's

@@ -317,7 +317,7 @@ __device__ __forceinline__ bool for_each_brick(IdxSmem<VT> &S, const CUtensorMap
     }
     if (TMA && S.abort) {
         if (tid == 0)
-            for (int s = 0; s < ISTAGES; ++s) mbar_wait(&S.bars[s], 0, 100000000ull);
+            for (int s = 0; s < ISTAGES; ++s) mbar_drain(&S.bars[s]);
         return false;
     }
     return true;

@@ -63,6 +63,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
     return true;
 }
 
+// For a CTA that ends because a wait ran out: a bounded chance for a copy still
+// in flight on bar to land, whichever of its phases that completes.  The one
+// before the phase in flight is over, so its wait returns at once.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar) {
+    mbar_wait(bar, 0, 100000000ull);
+    mbar_wait(bar, 1, 100000000ull);
+}
+
 // Asynchronous 4- / 8-byte copies from global to shared memory (cp.async,
 // completion by cp_async_wait_all in the issuing thread).
 __device__ __forceinline__ void cp_async_4(void *dst, const void *src) {
