@@ -957,7 +957,7 @@ struct GenParams {
 // for 512^3 voxels): with 1280 soup vertices and 512 records the 64-volume batch
 // takes 267 us instead of 244 at the same occupancy, and at three CTAs per SM
 // the 1024^3 volume 1204 us instead of 1104.
-constexpr int SH_VERTS = 1600, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
+constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
 
 // SHARED false: the adjoint's, which goes soup vertex by soup vertex and has no
 // records.  With the records' 24 KB float2 tiles leave room for three CTAs per
@@ -982,13 +982,12 @@ struct GenSmem {
             float nrm[SHARED ? SH_RECS * 3 : 1];
         };
     };
-    unsigned int cubes[SHARED ? SH_CUBES : 1];  // occupied cubes in order: cube | case << 11 | soup vertices before it << 19
+    unsigned int cubes[SHARED ? SH_CUBES + 1 : 1];  // occupied cubes in order: cube | case << 11 | soup vertices before it << 19, and all << 19
     uint2 slot[SHARED ? SH_SLOTS : 1];  // the edges of a slot that are used (bits 0-31 of 33), its first record
     unsigned int occp[(BY + 2) * (BZ + 2)];  // occupied cubes of cube row (cy, cz) at (cz + 1) * (BY + 2) + cy + 1, zero around
     unsigned int elut[12];            // edge -> slot step | x step << 16
     unsigned int wtot[2][WARPS];
-    unsigned short rowcube[CUBE_ROWS];  // occupied cubes before each cube row, and all
-    unsigned int ncube;
+    unsigned short rowcube[CUBE_ROWS + 1];  // occupied cubes before each cube row, and all
     unsigned int first[(SH_RECS + 31) / 32];  // bit: the first record of a used slot
     unsigned short used[SHARED ? SH_SLOTS + 1 : 1];  // the used slots, in order
     alignas(16) signed char tri[256][16];  // read a row at a time as 16 bytes
@@ -1319,19 +1318,25 @@ __device__ __forceinline__ void generate_brick(Smem &S, const typename Vox<VT>::
 //   3. one thread a cube: the record number of each of its soup vertices
 //      (S.vmap); one thread a record: position, voxel and normal;
 //   4. the soup is copied out of the records, whole lines at a time.
-// A brick with more than SH_VERTS soup vertices is taken some layers of cubes
-// at a time.  Bound: instructions (a third of them the records', a quarter the
+// A brick with more than SH_VERTS soup vertices or SH_RECS records is taken some
+// layers of cubes at a time, the soup of a layer by itself in parts if need be.
+// Bound: instructions (a third of them the records', a quarter the
 // steps before) and, while copying, the shared-memory pipe.  Working out each
 // soup vertex for itself took 578 warp-instructions per 32 soup vertices, this
 // about 400: 512^3 with 1.2 M triangles 100 -> 82 us, 1024^3 with 19 M 1373 ->
 // 1079 us, 64 volumes with 2.7 M 281 -> 204 us (there also with one tile stage
 // and four CTAs per SM instead of two stages).  Warps wait for barriers more
 // than for anything else: with up to three cubes a thread in step 2, one scan
-// and two barriers instead of those per 256 cubes, 79 and 1061 us.  Returns false (the caller
-// runs generate_brick) where a layer or its records do not fit, the output
-// ends inside the brick, or a vertex might lie outside its edge's nodes
-// (mcg_between_nodes: the records' voxels and samples are not tested one by
-// one, which costs 1 % of 512^3 to 1024^3 voxels); else tile_done() has been called by every thread
+// and two barriers instead of those per 256 cubes, 79 and 1061 us.  Returns false
+// (the caller runs generate_brick) where the cubes, 2^13 soup vertices or a
+// layer's records do not fit, the output ends inside the brick, or a vertex might
+// lie outside its edge's nodes (mcg_between_nodes: the records' voxels and samples
+// are not tested one by one, which costs 1 % of 512^3 to 1024^3 voxels).  With
+// one or two bricks a CTA the launch waits for the heaviest, so few should: one
+// found to have too many records once its first layers were done took 42 us, or
+// a layer of too many soup vertices 32, where the layers, or the parts, take 25
+// (384 x 256 x 320 voxels 49 -> 34 us, all by vertex 43; 256^3 with 3 % of the
+// voxels negative 320 -> 249, by vertex 280).  Else tile_done() has been called by every thread
 // between the last use of the tile and the last copy, so that the next brick's
 // tile is fetched meanwhile.  Called by every thread (contains __syncthreads).
 __device__ __forceinline__ unsigned int shared_elut(int e) {
@@ -1420,10 +1425,10 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
         const int cy = tid & (BY - 1), cz = tid / BY;
         S.occp[(cz + 1) * (BY + 2) + cy + 1] = warp == 0 ? occ[0] : occ[1];
         S.rowcube[tid] = (unsigned short)(warp == 0 ? incl & 0xffffu : (all & 0xffffu) + (incl >> 16));
-        if (tid == 0) S.ncube = (all & 0xffffu) + (all >> 16);
+        if (tid == 0) S.rowcube[CUBE_ROWS] = (unsigned short)((all & 0xffffu) + (all >> 16));
     }
     __syncthreads();
-    const unsigned int nocc = S.ncube;
+    const unsigned int nocc = S.rowcube[CUBE_ROWS];
     if (nocc > SH_CUBES) return false;
     // slots of layers [za, zb): this thread's voxel row; then their numbers
     unsigned long long m[5];
@@ -1535,55 +1540,33 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             if (j < per && i0 + j < nocc) S.cubes[i0 + j] = c[j] | (pre << 19);
             pre += nv[j];
         }
+        if (tid == 0) S.cubes[nocc] = T_brick << 19;
         R = number_slots();
         __syncthreads();
     }
     if (T_brick >= (1u << 13) || (long long)(vbase + T_brick) > o.cap) return false;
     // soup vertices before layer z: its first cube's
-    auto verts = [&](int z) -> unsigned int {
-        const unsigned int i = z < BZ ? S.rowcube[z * BY] : nocc;
-        return i < nocc ? S.cubes[i] >> 19 : T_brick;
-    };
-    // a layer that is too much by itself is found before the others are done
-    // (these are the heaviest bricks, and the launch waits for the last one)
-    if (T_brick > SH_VERTS && __any_sync(full, lane < BZ && verts(lane + 1) - verts(lane) > (unsigned int)SH_VERTS))
-        return false;
+    auto verts = [&](int z) -> unsigned int { return S.cubes[S.rowcube[z * BY]] >> 19; };
+    const bool whole = T_brick <= SH_VERTS && R <= SH_RECS;
     for (int za = 0, zb = BZ; za < BZ; za = zb, zb = BZ) {
-        unsigned int i0 = 0, i1 = nocc, va = 0, nT = T_brick;
-        if (T_brick > SH_VERTS) {
-            // the layers from za on that fit
-            va = verts(za);
-            while (verts(zb) - va > (unsigned int)SH_VERTS) --zb;
-            i0 = S.rowcube[za * BY];
-            i1 = zb < BZ ? S.rowcube[zb * BY] : nocc;
-            nT = verts(zb) - va;
-            count_slots(za, zb);
-            __syncthreads();
-            R = number_slots();
-            __syncthreads();
-        }
-        if (R > SH_RECS) return false;  // uniform
-        // 3. the record of every soup vertex (the last threads first: the
-        // first ones have the records)
-        const unsigned long long g0 = vbase + va;
-        for (unsigned int i = i0 + (THREADS - 1 - tid); i < i1; i += THREADS) {
-            const unsigned int w = S.cubes[i], ci = (w >> 11) & 0xffu, off = (w >> 19) - va;
-            const int x = (int)(w & 31u), cy = (int)(w >> 5) & 7, cz = (int)(w >> 8) & 7;
-            const uint2 *sl = S.slot + 5 * (cz * (BY + 1) + cy);
-            const unsigned int below = (1u << x) - 1u, below1 = below << 1 | 1u;
-            const signed char *tri = S.tri[ci];
-            const unsigned int nvc = S.nv[ci];
-            for (unsigned int q = 0; q < nvc; q += 3) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const unsigned int l = S.elut[tri[q + 2 - k]];
-                    const uint2 v = sl[l & 0xffffu];
-                    S.vmap[off + q + k] = (unsigned short)(v.y + __popc(v.x & (l >> 16 ? below1 : below)));
+        if (!whole) {
+            // the layers from za on whose soup vertices and records fit; one by
+            // itself can have more soup vertices (not many have), which then go
+            // out in parts
+            while (zb > za + 1 && verts(zb) - verts(za) > (unsigned int)SH_VERTS) --zb;
+            for (;;) {
+                if (za || zb < BZ) {
+                    count_slots(za, zb);
+                    __syncthreads();
+                    R = number_slots();
+                    __syncthreads();
                 }
-                if (o.tri_cube) o.tri_cube[(g0 + off + q) / 3] = lin3(nx, ny, x0 + x, y0 + cy, z0 + cz);
+                if (R <= SH_RECS) break;  // (all uniform)
+                if (zb == za + 1) return false;
+                zb = max(za + 1, za + (zb - za) * SH_RECS / R);
             }
         }
-        // and the records
+        // 3. the records
         const unsigned int firsts = lane < (SH_RECS + 31) / 32 ? S.first[lane] : 0u;
         for (int r = tid; r - lane < R; r += THREADS) {
             // its slot: used slots that start up to it; the warp's 32 records are one word of S.first
@@ -1619,45 +1602,75 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             S.nrm[3 * r + 1] = nrm.y;
             S.nrm[3 * r + 2] = nrm.z;
         }
-        __syncthreads();
-        if (zb == BZ) tile_done();
-        // 4. out, 16 bytes a thread from the first 16-byte boundary on.  Bound:
-        // the shared-memory and store pipe; with a word a thread (an entry of
-        // the map, a word of the record and a store for each) this was a
-        // quarter of the launch.
-        auto copy = [&](unsigned int *out, const unsigned int *from, auto words, unsigned int stride, unsigned int first) {
-            constexpr int W = decltype(words)::value;
-            unsigned int *dst = out + g0 * W;
-            const int n = (int)nT * W, lead = (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 3u);
-            const unsigned int rec0 = smem_u32(from) + 4 * first, map0 = smem_u32(S.vmap);
-            for (int i = 4 * tid - lead; i < n; i += 4 * THREADS) {
-                // words i .. i + 3 (i = -lead: from 0 on); they lie in at most two soup vertices
-                const int i0 = max(i, 0);
-                const unsigned int v = W == 7 ? (i0 * 9363u) >> 16 : (i0 * 21846u) >> 16;  // i0 / W
-                const int w = i - W * (int)v;
-                const unsigned int a0 = rec0 + 4 * stride * lds_u16(map0 + 2 * v) + 4 * w;
-                const unsigned int a1 = rec0 + 4 * stride * lds_u16(map0 + 2 * v + 2) + 4 * (w - W);
-                if (i >= 0 && i + 4 <= n) {
-                    uint4 q;
-                    q.x = lds_u32(a0);
-                    q.y = lds_u32((w + 1 < W ? a0 : a1) + 4);
-                    q.z = lds_u32((w + 2 < W ? a0 : a1) + 8);
-                    q.w = lds_u32((w + 3 < W ? a0 : a1) + 12);
-                    *reinterpret_cast<uint4 *>(dst + i) = q;
-                } else {
+        const unsigned int i0 = S.rowcube[za * BY], i1 = S.rowcube[zb * BY];
+        const unsigned int va = verts(za), nT = verts(zb) - va;
+        static_assert(SH_VERTS % 3 == 0, "a part ends with a triangle");
+        unsigned int w0 = 0;
+        do {  // (once also where the last layers are empty: tile_done)
+            const unsigned int nP = min(nT - w0, (unsigned int)SH_VERTS);
+            const unsigned long long g0 = vbase + va + w0;
+            // and the record of every soup vertex (the last threads first: the
+            // first ones have the records)
+            for (unsigned int i = i0 + (THREADS - 1 - tid); i < i1; i += THREADS) {
+                const unsigned int w = S.cubes[i], ci = (w >> 11) & 0xffu, off = (w >> 19) - va - w0;
+                const int x = (int)(w & 31u), cy = (int)(w >> 5) & 7, cz = (int)(w >> 8) & 7;
+                const uint2 *sl = S.slot + 5 * (cz * (BY + 1) + cy);
+                const unsigned int below = (1u << x) - 1u, below1 = below << 1 | 1u;
+                const signed char *tri = S.tri[ci];
+                const unsigned int nvc = S.nv[ci];
+                for (unsigned int q = 0; q < nvc; q += 3) {
+                    const unsigned int at = off + q;  // in the part (those before w0 wrap, in 32 bits)
+                    if (at >= nP) continue;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (i + k >= 0 && i + k < n) dst[i + k] = lds_u32((w + k < W ? a0 : a1) + 4 * k);
+                    for (int k = 0; k < 3; ++k) {
+                        const unsigned int l = S.elut[tri[q + 2 - k]];
+                        const uint2 v = sl[l & 0xffffu];
+                        S.vmap[at + k] = (unsigned short)(v.y + __popc(v.x & (l >> 16 ? below1 : below)));
+                    }
+                    if (o.tri_cube) o.tri_cube[(g0 + at) / 3] = lin3(nx, ny, x0 + x, y0 + cy, z0 + cz);
                 }
             }
-        };
-        const std::integral_constant<int, 7> seven;
-        const std::integral_constant<int, 3> three;
-        if (o.soup) copy(reinterpret_cast<unsigned int *>(o.soup), S.rec, seven, 7, 0);
-        if (o.normals)
-            copy(reinterpret_cast<unsigned int *>(o.normals), reinterpret_cast<const unsigned int *>(S.nrm), three, 3, 0);
-        if (o.vi2vox) copy(reinterpret_cast<unsigned int *>(o.vi2vox), S.rec, three, 7, 3);
-        if (zb < BZ) __syncthreads();  // the next layers' slots and records
+            __syncthreads();
+            if (w0 == 0 && zb == BZ) tile_done();
+            // 4. out, 16 bytes a thread from the first 16-byte boundary on.  Bound:
+            // the shared-memory and store pipe; with a word a thread (an entry of
+            // the map, a word of the record and a store for each) this was a
+            // quarter of the launch.
+            auto copy = [&](unsigned int *out, const unsigned int *from, auto words, unsigned int stride, unsigned int first) {
+                constexpr int W = decltype(words)::value;
+                unsigned int *dst = out + g0 * W;
+                const int n = (int)nP * W, lead = (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 3u);
+                const unsigned int rec0 = smem_u32(from) + 4 * first, map0 = smem_u32(S.vmap);
+                for (int i = 4 * tid - lead; i < n; i += 4 * THREADS) {
+                    // words i .. i + 3 (i = -lead: from 0 on); they lie in at most two soup vertices
+                    const int i0 = max(i, 0);
+                    const unsigned int v = W == 7 ? (i0 * 9363u) >> 16 : (i0 * 21846u) >> 16;  // i0 / W
+                    const int w = i - W * (int)v;
+                    const unsigned int a0 = rec0 + 4 * stride * lds_u16(map0 + 2 * v) + 4 * w;
+                    const unsigned int a1 = rec0 + 4 * stride * lds_u16(map0 + 2 * v + 2) + 4 * (w - W);
+                    if (i >= 0 && i + 4 <= n) {
+                        uint4 q;
+                        q.x = lds_u32(a0);
+                        q.y = lds_u32((w + 1 < W ? a0 : a1) + 4);
+                        q.z = lds_u32((w + 2 < W ? a0 : a1) + 8);
+                        q.w = lds_u32((w + 3 < W ? a0 : a1) + 12);
+                        *reinterpret_cast<uint4 *>(dst + i) = q;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (i + k >= 0 && i + k < n) dst[i + k] = lds_u32((w + k < W ? a0 : a1) + 4 * k);
+                    }
+                }
+            };
+            const std::integral_constant<int, 7> seven;
+            const std::integral_constant<int, 3> three;
+            if (o.soup) copy(reinterpret_cast<unsigned int *>(o.soup), S.rec, seven, 7, 0);
+            if (o.normals)
+                copy(reinterpret_cast<unsigned int *>(o.normals), reinterpret_cast<const unsigned int *>(S.nrm), three, 3, 0);
+            if (o.vi2vox) copy(reinterpret_cast<unsigned int *>(o.vi2vox), S.rec, three, 7, 3);
+            w0 += SH_VERTS;
+            if (w0 < nT || zb < BZ) __syncthreads();  // the next part's map, the next layers' slots and records
+        } while (w0 < nT);
     }
     return true;
 }
