@@ -944,6 +944,7 @@ struct GenParams {
     int16_t *ver_voxel;
     int64_t *tri_cube;
     long long cap;
+    int pick;  // float2: both forward launches were made, the one that records_pay() names does the work
     // adjoint (MODE 1): dL/dP per soup vertex in, dL/df per voxel accumulated
     const float *grad_pos;
     float *grad_f;
@@ -959,10 +960,22 @@ struct GenParams {
 // the 1024^3 volume 1204 us instead of 1104.
 constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
 
-// SHARED false: the adjoint's, which goes soup vertex by soup vertex and has no
-// records.  With the records' 24 KB float2 tiles leave room for three CTAs per
-// SM instead of four, and the adjoint of 768^3 voxels of spheres and noise
-// takes 2.21 ms instead of 2.15.
+// Whether the soup of a float2 volume comes out of records (MODE 0) or is worked
+// out vertex by vertex (MODE 2); the result is the same.  With the records' 26 KB
+// float2 tiles leave room for three CTAs per SM instead of four, so records pay
+// where bricks are as full as a surface makes them, and without normals only
+// where there are few.  Soup vertices a brick, MODE 2 -> MODE 0 in us: without
+// normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 -> 22.5,
+// 915 (1211) 34.8 -> 34.8, 867 (4245) 75 -> 73, 832 (17703) 266 -> 279; with
+// them 34.6 -> 27.0, 34.9 -> 26.2, 42.3 -> 39.2, 94 -> 86, 337 -> 319.  Noise
+// in 256^3 with them: 145 72 -> 95, 485 119 -> 127, 729 154 -> 152, 972 190 ->
+// 179, 1216 222 -> 209, 1458 254 -> 263, 4847 807 -> 882.
+__host__ __device__ inline bool records_pay(long long verts, long long bricks, bool normals) {
+    return verts >= 800 * bricks && verts <= 1300 * bricks && (normals || bricks <= 2048);
+}
+
+// SHARED false: the adjoint's and MODE 2's, which go soup vertex by soup vertex
+// and have no records, four CTAs per SM for float2 too.
 template <int VT, int NST, bool SHARED = true>
 struct GenSmem {
     static constexpr int MAPPED = SHARED ? SH_VERTS : BRICK_CUBES;  // soup vertices vmap holds
@@ -1759,7 +1772,10 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
     }
     __syncthreads();
     pdl_wait();  // the scan's list, offsets and totals
-    const unsigned int nactive = p.totals->active_bricks;
+    unsigned int nactive = p.totals->active_bricks;
+    if (VT == MCG_VOXEL_FLOAT2 && MODE != 1 && p.pick &&
+        records_pay(3 * (long long)p.totals->triangles, nactive, p.normals != nullptr) != (MODE == 0))
+        nactive = 0;
     unsigned int *ticket = &p.totals->gen_ticket;
     // stage st <- brick b (soup offset v): thread 0 records the brick, its
     // offset and origin for the CTA and starts the tile load
@@ -1862,7 +1878,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
                 }
             }
         };
-        if (MODE == 0) {
+        if (MODE != 1) {
             GenOut o;
             o.soup = p.soup;
             o.normals = p.normals;
@@ -1871,8 +1887,11 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
             o.tri_cube = p.tri_cube;
             o.cap = p.cap;
             o.zlim = p.zlim;
-            if (!generate_shared<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o, refill)) {
-                __syncthreads();
+            bool done = false;
+            if constexpr (MODE == 0)
+                done = generate_shared<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o, refill);
+            if (!done) {
+                if (MODE == 0) __syncthreads();
                 generate_brick<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o);
                 __syncthreads();
                 refill();
@@ -2730,9 +2749,20 @@ void launch_generate_t(const CUtensorMap &map, const GenParams &p, const Geometr
     if (!occ) occ = occupancy(mc_generate_kernel<VT, TMA, MODE>, THREADS, smem);
     long long grid = (long long)sms * occ;
     if (grid > g.nbricks) grid = g.nbricks;
-    // MODE 0 follows the scan directly; other launches follow a memset
-    if (MODE == 0) launch_pdl(mc_generate_kernel<VT, TMA, MODE>, (unsigned int)grid, THREADS, smem, s, map, p);
+    // the forward ones follow the scan (or one another) directly, the adjoint a memset
+    if (MODE != 1) launch_pdl(mc_generate_kernel<VT, TMA, MODE>, (unsigned int)grid, THREADS, smem, s, map, p);
     else mc_generate_kernel<VT, TMA, MODE><<<(int)grid, THREADS, smem, s>>>(map, p);
+}
+
+// known: the totals of the count phase, where the host has read them; else both
+// launches are made and the totals on the device decide which does the work (2 us)
+template <bool TMA>
+void launch_generate_float2(const CUtensorMap &map, GenParams p, const Geometry &g, int sms, cudaStream_t s,
+                            const MeshTotals *known) {
+    const bool records = known && records_pay(3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr);
+    p.pick = !known;
+    if (!known || records) launch_generate_t<MCG_VOXEL_FLOAT2, TMA, 0>(map, p, g, sms, s);
+    if (!known || !records) launch_generate_t<MCG_VOXEL_FLOAT2, TMA, 2>(map, p, g, sms, s);
 }
 
 // classify + scan into sc; clears the timeout flag first
@@ -2792,7 +2822,8 @@ cudaError_t launch_count_phase(const mcg_volume *vol, const Geometry &g, const S
 }
 
 cudaError_t launch_generate_phase(const mcg_volume *vol, const Geometry &g, const Scratch &sc,
-                                  const mcg_mesh_out *out, int sms, cudaStream_t s, const mcg_mc_config &cfg) {
+                                  const mcg_mesh_out *out, int sms, cudaStream_t s, const mcg_mc_config &cfg,
+                                  const MeshTotals *known = nullptr) {
     if (out->ver_voxel) {
         cudaError_t e = cudaMemsetAsync(out->ver_voxel, 0, sizeof(int16_t) * (size_t)vol->nx * vol->ny * vol->nz, s);
         if (e != cudaSuccess) return e;
@@ -2820,6 +2851,7 @@ cudaError_t launch_generate_phase(const mcg_volume *vol, const Geometry &g, cons
     p.ver_voxel = out->ver_voxel;
     p.tri_cube = out->tri_cube;
     p.cap = out->capacity_vertices;
+    p.pick = 0;
     p.grad_pos = nullptr;
     p.grad_f = nullptr;
     p.n_grad = 0;
@@ -2831,8 +2863,8 @@ cudaError_t launch_generate_phase(const mcg_volume *vol, const Geometry &g, cons
         if (tma) launch_generate_t<MCG_VOXEL_SHORT2, true>(map, p, g, sms, s);
         else launch_generate_t<MCG_VOXEL_SHORT2, false>(map, p, g, sms, s);
     } else {
-        if (tma) launch_generate_t<MCG_VOXEL_FLOAT2, true>(map, p, g, sms, s);
-        else launch_generate_t<MCG_VOXEL_FLOAT2, false>(map, p, g, sms, s);
+        if (tma) launch_generate_float2<true>(map, p, g, sms, s, known);
+        else launch_generate_float2<false>(map, p, g, sms, s, known);
     }
     return cudaGetLastError();
 }
@@ -3074,7 +3106,9 @@ mcg_status mcg_mc_generate(mcg_context *ctx, const mcg_volume *vol, const mcg_me
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     const Geometry g = geometry_slab(vol->nx, vol->ny, ctx->cls_z0, ctx->cls_z1);
-    e = launch_generate_phase(vol, g, ctx_scratch(ctx), out, ctx->num_sms, s, ctx->mc_cfg);
+    const bool read = !ctx->counts_pending && !mcg_capturing(s);  // the host has waited for the count phase's totals
+    e = launch_generate_phase(vol, g, ctx_scratch(ctx), out, ctx->num_sms, s, ctx->mc_cfg,
+                              read ? ctx->h_totals : nullptr);
     // the totals are re-read so a timeout flagged by generate is reported (the
     // launch writes the flags to the mapped host copy itself)
     if (e == cudaSuccess && !ctx->h_totals_dev)
