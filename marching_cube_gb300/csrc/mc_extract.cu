@@ -960,17 +960,19 @@ struct GenParams {
 // the 1024^3 volume 1204 us instead of 1104.
 constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROWS;
 
-// Whether the soup of a float2 volume comes out of records (MODE 0) or is worked
-// out vertex by vertex (MODE 2); the result is the same.  With the records' 26 KB
-// float2 tiles leave room for three CTAs per SM instead of four, so records pay
+// Whether the soup of a volume comes out of records (MODE 0) or is worked out
+// vertex by vertex (MODE 2); the result is the same.  Nearly empty bricks do not
+// repay the records' steps: noise in 256^3 short2 voxels with normals, soup
+// vertices a brick, MODE 2 -> MODE 0 in us: 52 54 -> 69, 145 71 -> 80, 243 87 ->
+// 90, 340 105 -> 100, 485 127 -> 112.  With the records' 26 KB float2 tiles leave room for three CTAs per SM instead of four, so records pay
 // where bricks are as full as a surface makes them, and without normals only
-// where there are few.  Soup vertices a brick, MODE 2 -> MODE 0 in us: without
-// normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 -> 22.5,
+// where there are few.  Soup vertices a brick as above: without normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 -> 22.5,
 // 915 (1211) 34.8 -> 34.8, 867 (4245) 75 -> 73, 832 (17703) 266 -> 279; with
 // them 34.6 -> 27.0, 34.9 -> 26.2, 42.3 -> 39.2, 94 -> 86, 337 -> 319.  Noise
 // in 256^3 with them: 145 72 -> 95, 485 119 -> 127, 729 154 -> 152, 972 190 ->
 // 179, 1216 222 -> 209, 1458 254 -> 263, 4847 807 -> 882.
-__host__ __device__ inline bool records_pay(long long verts, long long bricks, bool normals) {
+__host__ __device__ inline bool records_pay(int voxel_type, long long verts, long long bricks, bool normals) {
+    if (voxel_type == MCG_VOXEL_SHORT2) return verts >= 256 * bricks;
     return verts >= 800 * bricks && verts <= 1300 * bricks && (normals || bricks <= 2048);
 }
 
@@ -1774,7 +1776,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
     pdl_wait();  // the scan's list, offsets and totals
     unsigned int nactive = p.totals->active_bricks;
     if (VT == MCG_VOXEL_FLOAT2 && MODE != 1 && p.pick &&
-        records_pay(3 * (long long)p.totals->triangles, nactive, p.normals != nullptr) != (MODE == 0))
+        records_pay(VT, 3 * (long long)p.totals->triangles, nactive, p.normals != nullptr) != (MODE == 0))
         nactive = 0;
     unsigned int *ticket = &p.totals->gen_ticket;
     // stage st <- brick b (soup offset v): thread 0 records the brick, its
@@ -2754,15 +2756,17 @@ void launch_generate_t(const CUtensorMap &map, const GenParams &p, const Geometr
     else mc_generate_kernel<VT, TMA, MODE><<<(int)grid, THREADS, smem, s>>>(map, p);
 }
 
-// known: the totals of the count phase, where the host has read them; else both
-// launches are made and the totals on the device decide which does the work (2 us)
-template <bool TMA>
-void launch_generate_float2(const CUtensorMap &map, GenParams p, const Geometry &g, int sms, cudaStream_t s,
-                            const MeshTotals *known) {
-    const bool records = known && records_pay(3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr);
-    p.pick = !known;
-    if (!known || records) launch_generate_t<MCG_VOXEL_FLOAT2, TMA, 0>(map, p, g, sms, s);
-    if (!known || !records) launch_generate_t<MCG_VOXEL_FLOAT2, TMA, 2>(map, p, g, sms, s);
+// known: the totals of the count phase, where the host has read them.  Else
+// short2 soup comes out of records, and for float2 both launches are made and the
+// totals on the device decide which does the work (2 us).
+template <int VT, bool TMA>
+void launch_generate_forward(const CUtensorMap &map, GenParams p, const Geometry &g, int sms, cudaStream_t s,
+                             const MeshTotals *known) {
+    const bool records =
+        !known || records_pay(VT, 3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr);
+    p.pick = !known && VT == MCG_VOXEL_FLOAT2;
+    if (records) launch_generate_t<VT, TMA, 0>(map, p, g, sms, s);
+    if (!records || p.pick) launch_generate_t<VT, TMA, 2>(map, p, g, sms, s);
 }
 
 // classify + scan into sc; clears the timeout flag first
@@ -2860,11 +2864,11 @@ cudaError_t launch_generate_phase(const mcg_volume *vol, const Geometry &g, cons
     const bool tma = encode_volume_map(&map, vol->data, vol->nx, vol->ny, vol->nz, eb, TX, TY, TZ);
     if (!tma) memset(&map, 0, sizeof(map));
     if (vol->voxel_type == MCG_VOXEL_SHORT2) {
-        if (tma) launch_generate_t<MCG_VOXEL_SHORT2, true>(map, p, g, sms, s);
-        else launch_generate_t<MCG_VOXEL_SHORT2, false>(map, p, g, sms, s);
+        if (tma) launch_generate_forward<MCG_VOXEL_SHORT2, true>(map, p, g, sms, s, known);
+        else launch_generate_forward<MCG_VOXEL_SHORT2, false>(map, p, g, sms, s, known);
     } else {
-        if (tma) launch_generate_float2<true>(map, p, g, sms, s, known);
-        else launch_generate_float2<false>(map, p, g, sms, s, known);
+        if (tma) launch_generate_forward<MCG_VOXEL_FLOAT2, true>(map, p, g, sms, s, known);
+        else launch_generate_forward<MCG_VOXEL_FLOAT2, false>(map, p, g, sms, s, known);
     }
     return cudaGetLastError();
 }

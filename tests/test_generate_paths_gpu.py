@@ -1,4 +1,4 @@
-"""Float volumes by records of crossed edges or vertex by vertex, whichever their
+"""Soup by records of crossed edges or vertex by vertex, whichever a volume's
 soup vertices per brick choose: the same soup from a call whose counts the host
 has read, from one call in which the device decides, from a second generate, and
 from a captured graph replayed with volumes on either side.  Oracle: positions,
@@ -91,3 +91,22 @@ def test_graph_of_either(mcg):
         torch.cuda.synchronize()
         assert mcg.counts(ctx)["vertices"] == mesh.num_vertices
         _same(o, mesh, mesh.num_vertices)
+
+
+@pytest.mark.parametrize("dims", [(64, 41, 33), (65, 40, 30), (72, 20, 17)])
+@pytest.mark.parametrize("share", [0.0005, 0.002, 0.005, 0.0053, 0.006, 0.02])
+def test_short_volumes(mcg, orc, dims, share):
+    """256 soup vertices a brick, either side; the host has read the counts or not."""
+    v = _volume(dims, share)
+    vol = np.stack([(v[..., 0] * 30000).astype(np.int16), v[..., 1].astype(np.int16)], axis=-1)
+    vol[..., 0][(vol[..., 0] == 0)] = 7
+    o = orc.mc_extract(vol, 0.01)
+    assert_same_mesh(gpu_extract(mcg, vol, 0.01), o)
+    t = torch.from_numpy(vol).cuda()
+    mesh = mcg.extract(t, 0.01, vi2vox=True, ver_voxel=True, tri_cube=True)
+    out = {k: torch.zeros_like(getattr(mesh, k)) for k in ("soup", "normals", "vi2vox", "ver_voxel", "tri_cube")}
+    mcg.extract_into(t, 0.01, out, mesh.num_vertices, ctx=mcg.Context())
+    assert all(torch.equal(out[k], getattr(mesh, k)) for k in out)
+    for keep in (("soup",), ("normals",), ("soup", "normals", "tri_cube")):
+        part = mcg.extract(t, 0.01, **{k: k in keep for k in out})
+        assert all(torch.equal(getattr(part, k), getattr(mesh, k)) for k in keep)
