@@ -681,9 +681,10 @@ __device__ __forceinline__ void backward_voxel(const IntegBwParams &p, const flo
             ob[f - f0] = o;
             fuse_core(p.is_dynamic, o.s, o.w0, cF, cW, cF, cW);
         }
-        for (; seen; ) {
-            const int k = 31 - __clz(seen);
-            seen &= ~(1u << k);
+        // (a warp's lanes on the same frame: its arrays are interleaved lane by
+        // lane, and its pixels lie together)
+        for (int k = f1 - f0 - 1; k >= 0; --k) {
+            if (!((seen >> k) & 1u)) continue;
             const Obs o = ob[k];
             const float Fp = sF[k], Wp = sW[k];
             float wv = o.w0, mult = 1.0f, d = 0.0f;
@@ -715,13 +716,20 @@ __device__ __forceinline__ void backward_voxel(const IntegBwParams &p, const flo
 
 // Few voxels have a gradient (the band around the surface that the mesh
 // touches), spread thinly over the volume's rows: a CTA collects those of
-// BW_SCAN voxels at a time and works them out BW_THREADS together.  Bound: the
-// work on those voxels (an observation is two divisions and a gather).  One
-// thread a voxel, three observations a frame, took 478 us for 256^3 and ten
-// 320x240 frames.
-constexpr int BW_THREADS = 128, BW_SCAN = 4 * BW_THREADS;
+// ROUNDS voxels a thread at a time and works them out BW_THREADS together.
+// Bound: the work on those voxels (an observation is two divisions and a
+// gather).  256^3 and ten 320x240 frames, gradients at the mesh's voxels: one
+// thread a voxel and three observations a frame 526 us, this 96; at every voxel
+// 3.1 and 1.7 ms.  With each lane at its own next frame in the sweep back these
+// took 94 us and 2.8 ms, and 128^3 with 40 frames 7.5 ms where one thread a
+// voxel takes 1.7 and this 1.3.  Four rounds where they leave a CTA for
+// every place, else one: 64^3 with 40 frames 379 us with four, 201 with one (240
+// with a thread a voxel); 256^3 at the mesh's voxels 96 and 126.
+constexpr int BW_THREADS = 128;
 
+template <int ROUNDS>
 __global__ void __launch_bounds__(BW_THREADS) integrate_backward_kernel(IntegBwParams p) {
+    constexpr int BW_SCAN = ROUNDS * BW_THREADS;
     extern __shared__ float s_pose[];
     __shared__ long long s_at[BW_THREADS + BW_SCAN];
     __shared__ float2 s_g[BW_THREADS + BW_SCAN];
@@ -739,15 +747,15 @@ __global__ void __launch_bounds__(BW_THREADS) integrate_backward_kernel(IntegBwP
         if (p.grad_w0) p.grad_w0[i] = gW;
     };
     for (long long base = (long long)blockIdx.x * BW_SCAN; base < n; base += (long long)gridDim.x * BW_SCAN) {
-        float gF[BW_SCAN / BW_THREADS], gW[BW_SCAN / BW_THREADS];
+        float gF[ROUNDS], gW[ROUNDS];
 #pragma unroll
-        for (int k = 0; k < BW_SCAN / BW_THREADS; ++k) {
+        for (int k = 0; k < ROUNDS; ++k) {
             const long long i = base + k * BW_THREADS + tid;
             gF[k] = i < n ? p.grad_f[i * p.grad_step] : 0.0f;
             gW[k] = i < n && p.grad_w ? p.grad_w[i * p.grad_step] : 0.0f;
         }
 #pragma unroll
-        for (int k = 0; k < BW_SCAN / BW_THREADS; ++k) {
+        for (int k = 0; k < ROUNDS; ++k) {
             const long long i = base + k * BW_THREADS + tid;
             const bool has = gF[k] != 0.0f || gW[k] != 0.0f;
             const unsigned int m = __ballot_sync(0xffffffffu, has);
@@ -1137,8 +1145,12 @@ static mcg_status integrate_backward_impl(mcg_context *ctx, const void *vol0, in
     p.grad_f0 = grad_f0;
     p.grad_w0 = grad_w0;
     const long long n = (long long)nx * ny * nz;
-    const long long grid = std::min((n + BW_SCAN - 1) / BW_SCAN, (long long)ctx->num_sms * 8);
-    integrate_backward_kernel<<<(unsigned int)grid, BW_THREADS, sizeof(float) * 12 * n_frames, s>>>(p);
+    const long long most = (long long)ctx->num_sms * 8;
+    const size_t poses = sizeof(float) * 12 * n_frames;
+    if (n >= most * 4 * BW_THREADS)
+        integrate_backward_kernel<4><<<(unsigned int)most, BW_THREADS, poses, s>>>(p);
+    else
+        integrate_backward_kernel<1><<<(unsigned int)std::min(most, (n + BW_THREADS - 1) / BW_THREADS), BW_THREADS, poses, s>>>(p);
     e = cudaGetLastError();
     return e == cudaSuccess ? MCG_OK : mcg_cuda_fail(ctx, e);
 }
