@@ -944,7 +944,6 @@ struct GenParams {
     int16_t *ver_voxel;
     int64_t *tri_cube;
     long long cap;
-    int pick;  // float2: both forward launches were made, the one that records_pay() names does the work
     // adjoint (MODE 1): dL/dP per soup vertex in, dL/df per voxel accumulated
     const float *grad_pos;
     float *grad_f;
@@ -964,13 +963,20 @@ constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROW
 // vertex by vertex (MODE 2); the result is the same.  Nearly empty bricks do not
 // repay the records' steps: noise in 256^3 short2 voxels with normals, soup
 // vertices a brick, MODE 2 -> MODE 0 in us: 52 54 -> 69, 145 71 -> 80, 243 87 ->
-// 90, 340 105 -> 100, 485 127 -> 112.  With the records' 26 KB float2 tiles leave room for three CTAs per SM instead of four, so records pay
-// where bricks are as full as a surface makes them, and without normals only
-// where there are few.  Soup vertices a brick as above: without normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 -> 22.5,
-// 915 (1211) 34.8 -> 34.8, 867 (4245) 75 -> 73, 832 (17703) 266 -> 279; with
-// them 34.6 -> 27.0, 34.9 -> 26.2, 42.3 -> 39.2, 94 -> 86, 337 -> 319.  Noise
-// in 256^3 with them: 145 72 -> 95, 485 119 -> 127, 729 154 -> 152, 972 190 ->
-// 179, 1216 222 -> 209, 1458 254 -> 263, 4847 807 -> 882.
+// 90, 340 105 -> 100, 485 127 -> 112.  Where only the device knows the counts
+// (one call for both phases, a graph) the MODE 0 launch takes such bricks as MODE
+// 2 does: 192^3, 52 a brick, 44 -> 39 us.  So does a batch's: twelve of 96^3 92 ->
+// 84 us (73 without records, their room being a second tile stage; 729 instead of
+// 585 for 64 volumes of surfaces).  With the records' 26 KB float2 tiles leave
+// room for three CTAs per SM instead of four, so records pay where the host knows
+// that bricks are as full as a surface makes them, and without normals only where
+// there are few (one call for both phases by vertex: 256^3 84 us, with both
+// launches made and the counts choosing 88).  Soup vertices a brick as above:
+// without normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 ->
+// 22.5, 915 (1211) 34.8 -> 34.8, 867 (4245) 75 -> 73, 832 (17703) 266 -> 279; with
+// them 34.6 -> 27.0, 34.9 -> 26.2, 42.3 -> 39.2, 94 -> 86, 337 -> 319.  Noise in
+// 256^3 with them: 145 72 -> 95, 485 119 -> 127, 729 154 -> 152, 972 190 -> 179,
+// 1216 222 -> 209, 1458 254 -> 263, 4847 807 -> 882.
 __host__ __device__ inline bool records_pay(int voxel_type, long long verts, long long bricks, bool normals) {
     if (voxel_type == MCG_VOXEL_SHORT2) return verts >= 256 * bricks;
     return verts >= 800 * bricks && verts <= 1300 * bricks && (normals || bricks <= 2048);
@@ -1016,6 +1022,7 @@ struct GenSmem {
     unsigned int pipe_b;        // refill and its soup offset; pipe_b ~0u = none
     unsigned int wsum[2][2];
     unsigned int nocc, total;
+    int direct;  // MODE 0: vertex by vertex all the same, records do not pay
     int abort;
 };
 
@@ -1774,10 +1781,9 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
     }
     __syncthreads();
     pdl_wait();  // the scan's list, offsets and totals
-    unsigned int nactive = p.totals->active_bricks;
-    if (VT == MCG_VOXEL_FLOAT2 && MODE != 1 && p.pick &&
-        records_pay(VT, 3 * (long long)p.totals->triangles, nactive, p.normals != nullptr) != (MODE == 0))
-        nactive = 0;
+    const unsigned int nactive = p.totals->active_bricks;
+    if (MODE == 0 && tid == 0)
+        S.direct = VT == MCG_VOXEL_SHORT2 && !records_pay(VT, 3 * (long long)p.totals->triangles, nactive, true);
     unsigned int *ticket = &p.totals->gen_ticket;
     // stage st <- brick b (soup offset v): thread 0 records the brick, its
     // offset and origin for the CTA and starts the tile load
@@ -1891,7 +1897,8 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __
             o.zlim = p.zlim;
             bool done = false;
             if constexpr (MODE == 0)
-                done = generate_shared<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o, refill);
+                if (!S.direct)
+                    done = generate_shared<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o, refill);
             if (!done) {
                 if (MODE == 0) __syncthreads();
                 generate_brick<VT>(S, tile, vol, nx, ny, nz, cell, bp.x0, bp.y0, bp.z0, vbase, o);
@@ -2557,6 +2564,7 @@ __global__ void __launch_bounds__(THREADS, 4)
     };
     if (tid == 0) {
         S.abort = 0;
+        S.direct = VT == MCG_VOXEL_SHORT2 && !records_pay(VT, 3 * (long long)totals->triangles, nactive, true);
         mbar_init(&S.bars[0], 1);
         fence_barrier_init();
         S.svol = -1;
@@ -2609,8 +2617,8 @@ __global__ void __launch_bounds__(THREADS, 4)
                 else ptk = 0xffffffffu;  // the list is exhausted: draw no more
             }
         };
-        if (!generate_shared<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x, sp.y, sp.z,
-                                 vbase, o, refill)) {
+        if (S.direct || !generate_shared<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x,
+                                             sp.y, sp.z, vbase, o, refill)) {
             __syncthreads();
             generate_brick<VT>(S, tile, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.cell, sp.x, sp.y, sp.z,
                                vbase, o);
@@ -2756,17 +2764,15 @@ void launch_generate_t(const CUtensorMap &map, const GenParams &p, const Geometr
     else mc_generate_kernel<VT, TMA, MODE><<<(int)grid, THREADS, smem, s>>>(map, p);
 }
 
-// known: the totals of the count phase, where the host has read them.  Else
-// short2 soup comes out of records, and for float2 both launches are made and the
-// totals on the device decide which does the work (2 us).
+// known: the totals of the count phase, where the host has read them.  Else a
+// short2 launch decides by itself, and float2 soup is worked out vertex by vertex.
 template <int VT, bool TMA>
-void launch_generate_forward(const CUtensorMap &map, GenParams p, const Geometry &g, int sms, cudaStream_t s,
+void launch_generate_forward(const CUtensorMap &map, const GenParams &p, const Geometry &g, int sms, cudaStream_t s,
                              const MeshTotals *known) {
-    const bool records =
-        !known || records_pay(VT, 3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr);
-    p.pick = !known && VT == MCG_VOXEL_FLOAT2;
+    const bool records = known ? records_pay(VT, 3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr)
+                               : VT == MCG_VOXEL_SHORT2;
     if (records) launch_generate_t<VT, TMA, 0>(map, p, g, sms, s);
-    if (!records || p.pick) launch_generate_t<VT, TMA, 2>(map, p, g, sms, s);
+    else launch_generate_t<VT, TMA, 2>(map, p, g, sms, s);
 }
 
 // classify + scan into sc; clears the timeout flag first
@@ -2855,7 +2861,6 @@ cudaError_t launch_generate_phase(const mcg_volume *vol, const Geometry &g, cons
     p.ver_voxel = out->ver_voxel;
     p.tri_cube = out->tri_cube;
     p.cap = out->capacity_vertices;
-    p.pick = 0;
     p.grad_pos = nullptr;
     p.grad_f = nullptr;
     p.n_grad = 0;
