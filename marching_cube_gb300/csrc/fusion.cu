@@ -193,7 +193,7 @@ struct IntegParams {
     int tiles_x;
     int nbx, nby;           // blocks of IB^3 voxels per axis
     unsigned int nblocks;
-    unsigned int *list;     // blocks that can hold an updated voxel
+    unsigned int *list;     // blocks that can hold an updated voxel, or null: all
     unsigned int *count;    // how many of them
     // several frames at once: how many (pose_dev, ds, normals and tiles hold
     // them one after another), and per listed block which of them (bits)
@@ -335,6 +335,10 @@ __device__ __forceinline__ void fuse(const IntegParams &p, float sdf, float weig
 // with blocks next to the camera searched, see below); one 320x240 frame into
 // 256^3 float2: 72 -> 20 us.
 constexpr int IB = 8;
+// A volume of so few blocks takes them all: listing them costs a launch and its
+// latency (64^3 and 640x480 23 us, 13 without; 128^3 20-25 and 14-18; 160^3, 8000
+// blocks, 17-19 and 18-25).
+constexpr long long IB_ALL = 4096;
 
 __device__ __forceinline__ bool integ_block_kept(const IntegParams &p, const float *R, const float *t,
                                                  const float *tiles, int x0, int y0, int z0) {
@@ -404,10 +408,26 @@ __device__ __forceinline__ bool integ_block_kept(const IntegParams &p, const flo
     // hundred tiles was most of this launch, 27 us at 512^3)
     const int tu0 = pu0 / TILE_W, tu1 = pu1 / TILE_W, tv0 = pv0 / TILE_H, tv1 = pv1 / TILE_H;
     if ((tu1 - tu0 + 1) * (tv1 - tv0 + 1) > 64) return true;
+    // TILES loads at a time, also across rows (a row's few tiles at a time, one
+    // after another: 160^3 and 640x480 29 us where the view is full, 19 so)
+    constexpr int TILES = 4;
     float zt = 0.0f;
-    for (int ty = tv0; ty <= tv1; ++ty)
-#pragma unroll 4
-        for (int tx = tu0; tx <= tu1; ++tx) zt = fmaxf(zt, tiles[(long long)ty * p.tiles_x + tx]);
+    const int n = (tu1 - tu0 + 1) * (tv1 - tv0 + 1);
+    int tx = tu0;
+    const float *row = tiles + (long long)tv0 * p.tiles_x;
+    for (int i = 0; i < n; i += TILES) {
+        float z[TILES];
+#pragma unroll
+        for (int k = 0; k < TILES; ++k) {
+            z[k] = i + k < n ? row[tx] : 0.0f;
+            if (++tx > tu1) {
+                tx = tu0;
+                row += p.tiles_x;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TILES; ++k) zt = fmaxf(zt, z[k]);
+    }
     if (zt == 0.0f) return false;  // no valid pixel
     const float near = sqrtf(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) - sqrtf(half);
     return !(near > zt + p.min_t + 1e-5f * (size + zt + p.min_t));
@@ -457,10 +477,10 @@ __global__ void __launch_bounds__(256) integrate_kernel(IntegParams p, T *__rest
     constexpr int PASSES = IB * IB / RPP;       // passes per block
     load_pose(p);
     const int lane = threadIdx.x & 31;
-    const unsigned int items = *p.count * PASSES;
+    const unsigned int items = (p.list ? *p.count : p.nblocks) * PASSES;
     const unsigned int warps = gridDim.x * 8u;
     for (unsigned int it = blockIdx.x * 8u + (threadIdx.x >> 5); it < items; it += warps) {
-        const unsigned int b = p.list[it / PASSES];
+        const unsigned int b = p.list ? p.list[it / PASSES] : it / PASSES;
         const unsigned int brow = b / (unsigned int)p.nbx;
         const int r = (int)(it % PASSES) * RPP + lane / LPR;  // row of the block, y fastest
         const int x0 = (int)(b - brow * (unsigned int)p.nbx) * IB + (lane % LPR) * VPL;
@@ -980,7 +1000,8 @@ static mcg_status integrate_impl(mcg_context *ctx, void *vol, int32_t voxel_type
     p.list = ctx->integ_blocks;
     p.count = ctx->integ_count;
     depth_scale_kernel<<<g2, b2, 0, s>>>(p.k, w, h, depth_m, ctx->depth_scaled, ctx->integ_tiles, ctx->integ_count);
-    integrate_blocks_kernel<<<(unsigned int)((nblocks + 255) / 256), 256, 0, s>>>(p);
+    if (nblocks > IB_ALL) integrate_blocks_kernel<<<(unsigned int)((nblocks + 255) / 256), 256, 0, s>>>(p);
+    else p.list = nullptr;
     // one warp per item; the grid holds what the SMs can and strides over more
     const long long most = (long long)ctx->num_sms * 8;
     if (voxel_type == MCG_VOXEL_SHORT2) {
