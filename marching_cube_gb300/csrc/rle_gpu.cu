@@ -38,6 +38,10 @@ constexpr int RCHUNK = 4096;       // voxels per chunk
 constexpr int RWORDS = RCHUNK / 32;
 constexpr int RWARPS = RT / 32;
 constexpr long long RSCRATCH = 288ll << 20;  // bytes of run-start bits and chunk records at a time: 2^31 voxels'
+// Most bytes of an image (at 6 a voxel) whose records are written before its size
+// has been read: encoding 32^3 voxels takes 67 us so, 79 with the wait between the
+// launches; 96^3 146 and 151.
+constexpr long long RAHEAD = 8ll << 20;
 constexpr int kMaxRun = 0x3fff;
 
 // record kind of a record whose first voxel is v (put_run in rle.cpp)
@@ -387,6 +391,27 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
     e = cudaGetLastError();
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     bool again = false;  // the marks are not there any more
+    auto emit = [&]() {
+        for (long long z = 0; z < nz; z += per) {
+            const long long n = std::min(per, nz - z);
+            if (again || per < nz) mark(z, n);
+            rle_emit<<<(unsigned int)(n * nchunks), ET, 0, s>>>(v + z * xy, (int)xy, (int)nchunks, ll,
+                                                                reinterpret_cast<RleChunk *>(ctx->rle_chunks),
+                                                                ctx->rle_marks, cwords, d_bytes + z, d_off + z,
+                                                                ctx->rle_image);
+        }
+    };
+    // a small volume's records are written before its size is known
+    bool ahead = !query && per == nz && mcg_rle_bound(nx, ny, nz) <= RAHEAD;
+    if (ahead && !ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)mcg_rle_bound(nx, ny, nz))) {
+        cudaGetLastError();
+        ahead = false;
+    }
+    if (ahead) {
+        emit();
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
+    }
     unsigned long long o = 0;
     e = cudaMemcpyAsync(&o, d_off + nz, sizeof(o), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -395,28 +420,23 @@ extern "C" mcg_status mcg_rle_encode(mcg_context *ctx, const void *vol, int32_t 
         *size = (int64_t)o;
         return query ? MCG_OK : MCG_ERR_CAPACITY;
     }
-    if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) {
-        // the image before the scratch, then what is left for that
-        cudaGetLastError();
-        cudaFree(ctx->rle_chunks);
-        cudaFree(ctx->rle_marks);
-        ctx->rle_chunks = nullptr;
-        ctx->rle_marks = nullptr;
-        ctx->rle_chunks_cap = ctx->rle_marks_cap = 0;
-        if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o) || !scratch())
-            return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
-        again = true;
+    if (!ahead) {
+        if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o)) {
+            // the image before the scratch, then what is left for that
+            cudaGetLastError();
+            cudaFree(ctx->rle_chunks);
+            cudaFree(ctx->rle_marks);
+            ctx->rle_chunks = nullptr;
+            ctx->rle_marks = nullptr;
+            ctx->rle_chunks_cap = ctx->rle_marks_cap = 0;
+            if (!ensure(&ctx->rle_image, &ctx->rle_image_cap, (size_t)o) || !scratch())
+                return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
+            again = true;
+        }
+        emit();
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     }
-    for (long long z = 0; z < nz; z += per) {
-        const long long n = std::min(per, nz - z);
-        if (again || per < nz) mark(z, n);
-        rle_emit<<<(unsigned int)(n * nchunks), ET, 0, s>>>(v + z * xy, (int)xy, (int)nchunks, ll,
-                                                            reinterpret_cast<RleChunk *>(ctx->rle_chunks),
-                                                            ctx->rle_marks, cwords, d_bytes + z, d_off + z,
-                                                            ctx->rle_image);
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
     // header (:1303-1310), then the slices
     memcpy(image, lossless ? kTagLossless : kTagRef, 16);
     const int32_t dims[3] = {nx, ny, nz};
