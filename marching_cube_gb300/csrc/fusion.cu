@@ -342,7 +342,7 @@ constexpr long long IB_ALL = 4096;
 
 __device__ __forceinline__ bool integ_block_kept(const IntegParams &p, const float *R, const float *t,
                                                  const float *tiles, int x0, int y0, int z0) {
-    const int x1 = min(x0 + IB, p.nx) - 1, y1 = min(y0 + IB, p.ny) - 1, z1 = min(z0 + IB, p.nz) - 1;
+    const int x1 = x0 + min(IB, p.nx - x0) - 1, y1 = y0 + min(IB, p.ny - y0) - 1, z1 = z0 + min(IB, p.nz - z0) - 1;
     const float lo[3] = {p.ray_x[x0], (float)y0 * p.grid_s, (float)z0 * p.grid_s};
     const float hi[3] = {p.ray_x[x1], (float)y1 * p.grid_s, (float)z1 * p.grid_s};
     float c[3], hf[3], mag[3];
@@ -477,10 +477,11 @@ __global__ void __launch_bounds__(256) integrate_kernel(IntegParams p, T *__rest
     constexpr int PASSES = IB * IB / RPP;       // passes per block
     load_pose(p);
     const int lane = threadIdx.x & 31;
-    const unsigned int items = (p.list ? *p.count : p.nblocks) * PASSES;
+    // (64-bit: a volume can have 2^30 blocks)
+    const unsigned long long items = (unsigned long long)(p.list ? *p.count : p.nblocks) * PASSES;
     const unsigned int warps = gridDim.x * 8u;
-    for (unsigned int it = blockIdx.x * 8u + (threadIdx.x >> 5); it < items; it += warps) {
-        const unsigned int b = p.list ? p.list[it / PASSES] : it / PASSES;
+    for (unsigned long long it = blockIdx.x * 8u + (threadIdx.x >> 5); it < items; it += warps) {
+        const unsigned int b = p.list ? p.list[it / PASSES] : (unsigned int)(it / PASSES);
         const unsigned int brow = b / (unsigned int)p.nbx;
         const int r = (int)(it % PASSES) * RPP + lane / LPR;  // row of the block, y fastest
         const int x0 = (int)(b - brow * (unsigned int)p.nbx) * IB + (lane % LPR) * VPL;
@@ -806,6 +807,8 @@ __global__ void __launch_bounds__(BW_THREADS) integrate_backward_kernel(IntegBwP
     if (tid < s_n) work(tid);
 }
 
+long long blocks_of(int n) { return ((long long)n + IB - 1) / IB; }
+
 Intr intr_of(const mcg_intrinsic *k) { return Intr{k->fx, k->fy, k->cx, k->cy}; }
 
 // Room for the depth tiles of any image of so many pixels (one column of
@@ -956,9 +959,9 @@ static mcg_status integrate_impl(mcg_context *ctx, void *vol, int32_t voxel_type
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return mcg_cuda_fail(ctx, e);
-    const long long nbx = (nx + IB - 1) / IB, nby = (ny + IB - 1) / IB, nbz = (nz + IB - 1) / IB;
+    const long long nbx = blocks_of(nx), nby = blocks_of(ny), nbz = blocks_of(nz);
     const long long nblocks = nbx * nby * nbz;
-    if (nblocks > (long long)(UINT32_MAX / 16)) return MCG_ERR_TOO_LARGE;  // 32-bit work items
+    if (nblocks > (long long)UINT32_MAX) return MCG_ERR_TOO_LARGE;  // (a terabyte of voxels at least)
     const dim3 b2(32, TILE_H), g2((w + 31) / 32, (h + TILE_H - 1) / TILE_H);
     const size_t ntiles = tile_room((long long)w * h);
     // inside a stream capture nothing may be allocated: an earlier call of
@@ -1036,9 +1039,9 @@ static mcg_status integrate_pass(mcg_context *ctx, void *vol, int32_t voxel_type
     p.is_dynamic = is_dynamic ? 1 : 0;
     p.tiles = ctx->integ_tiles;
     p.tiles_x = 2 * (int)g2.x;
-    p.nbx = (nx + IB - 1) / IB;
-    p.nby = (ny + IB - 1) / IB;
-    const long long nblocks = (long long)p.nbx * p.nby * ((nz + IB - 1) / IB);
+    p.nbx = (int)blocks_of(nx);
+    p.nby = (int)blocks_of(ny);
+    const long long nblocks = p.nbx * (p.nby * blocks_of(nz));
     p.nblocks = (unsigned int)nblocks;
     p.list = ctx->integ_blocks;
     p.count = ctx->integ_count;
@@ -1070,7 +1073,7 @@ mcg_status mcg_integrate_frames(mcg_context *ctx, void *vol, int32_t voxel_type,
     if (!(min_t > 0.0f) || !(max_t > 0.0f) || !(grid_s > 0.0f)) return MCG_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const long long pixels = (long long)w * h;
-    const size_t nblocks = (size_t)((nx + IB - 1) / IB) * ((ny + IB - 1) / IB) * ((nz + IB - 1) / IB);
+    const size_t nblocks = (size_t)(blocks_of(nx) * blocks_of(ny) * blocks_of(nz));
     const size_t ntiles = tile_room(pixels);
     // frames a pass: 256 MB of ray-length depth at most
     const int most = (int)std::min<long long>({n_frames, FRAMES, std::max(1ll, (64ll << 20) / pixels)});
