@@ -483,8 +483,14 @@ __device__ __forceinline__ int cached_volume(VolCache &c, const VolDesc *__restr
 // and 43 and 102 with the signs of a short2 brick looked at first (4 operations
 // a row instead of 11; a mixed brick's rows, a quarter of the batch's, are read
 // once more) and three CTAs per SM instead of four, which then only evict each
-// other's lines (four 45 and 110, five 49 and 154, two 39 and 128).  float2
-// keeps the one pass: 30 us for 201 x 175 x 233 voxels against 38.
+// other's lines (four 45 and 110, five 49 and 154, two 39 and 128).  A warp does
+// not look at them after a brick with triangles, nor where it has one brick only
+// and the second reading would be all of the time: counting twelve 96^3 volumes
+// of noise in every brick 55 -> 45 us (45 by TMA; 55 also where every brick is
+// looked at), 64 of 128^3 178 -> 151 (161 by TMA), 35 x 200 x 200 voxels 33 -> 26
+// (28 by tiles filled first).  float2 keeps the one pass: 30 us for 201 x 175 x
+// 233 voxels against 38; its batches take this way, too, TMA or not: 64 of 128^3
+// 184 us (262 by TMA), 16 empty ones of 160^3 97 (110) with generate.
 struct RowsParams {
     // one volume ...
     const void *vol;
@@ -497,6 +503,7 @@ struct RowsParams {
     uint32_t *brick_tris, *chunk;
     unsigned int *ticket;
     int draw;  // consecutive bricks drawn at a time
+    int look;  // short2: the signs of a warp's first brick first
 };
 
 constexpr int RW_THREADS = 256, RW_WARPS = RW_THREADS / 32;
@@ -555,17 +562,30 @@ __device__ __forceinline__ bool brick_mixed(const short2 *__restrict__ p, long l
     return __any_sync(0xffffffffu, any) && __any_sync(0xffffffffu, other);
 }
 
+// A voxel as load_rows holds it: short2 as the word that was loaded (its
+// halves taken apart row by row, a brick's rows took 8 us instead of 4).
+template <int VT>
+struct RowVox : Vox<VT> {};
+template <>
+struct RowVox<MCG_VOXEL_SHORT2> {
+    using T = unsigned int;
+    static __device__ __forceinline__ T fill() { return 0u; }
+    static __device__ __forceinline__ bool neg(T v) { return v & 0x8000u; }
+    static __device__ __forceinline__ bool w0(T v) { return v < 0x10000u; }
+};
+
 // Row masks of the brick whose first voxel is p (this lane's: p[lane]) into row[],
 // the 33rd voxels' into en / ed (row r: bit r % 32 of word r / 32), and whether
-// a voxel inside the volume is negative, or not (both true for a short2 brick,
-// brick_mixed has said so).  FULL: 33 x 9 x 9 voxels are
-// inside; else nx1 x ny1 x nz1 of them, the others read as weight 0.
+// a voxel inside the volume is negative, or not (both true for a short2 brick:
+// brick_mixed has said so, or its cubes do).  FULL: 33 x 9 x 9 voxels are inside;
+// else nx1 x ny1 x nz1 of them, the others read as weight 0.
 template <int VT, bool FULL>
 __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T *__restrict__ p, long long sy, long long sz,
                                           int nx1, int ny1, int nz1, unsigned int en[3], unsigned int ed[3],
                                           unsigned int &neg_any, unsigned int &pos_any) {
-    using V = Vox<VT>;
+    using V = RowVox<VT>;
     using T = typename V::T;
+    const T *vox = reinterpret_cast<const T *>(p);
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int xmask = FULL || nx1 >= 32 ? full : (1u << nx1) - 1u;
@@ -575,11 +595,11 @@ __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T 
     for (int j = 0; j < 3; ++j) {
         const int r = lane + 32 * j, lz = r / (BY + 1), ly = r - (BY + 1) * lz;
         ein[j] = r < ROWS && (FULL || (nx1 > BX && ly < ny1 && lz < nz1));
-        e[j] = ein[j] ? p[lz * sz + ly * sy + BX] : V::fill();
+        e[j] = ein[j] ? vox[lz * sz + ly * sy + BX] : V::fill();
     }
     // planes of nine rows, the next one's loads out before this one's votes
     auto fetch = [&](T (&w)[BY + 1], int lz) {
-        const T *q = p + lz * sz + lane;
+        const T *q = vox + lz * sz + lane;
 #pragma unroll
         for (int ly = 0; ly < BY + 1; ++ly) {
             w[ly] = FULL || (lane < nx1 && ly < ny1 && lz < nz1) ? *q : V::fill();
@@ -627,7 +647,8 @@ __device__ __forceinline__ void load_rows(uint2 *row, const typename Vox<VT>::T 
 template <int VT>
 __device__ __forceinline__ void count_rows(uint2 *row, const unsigned char *ntri,
                                            const typename Vox<VT>::T *__restrict__ vol, int nx, int ny, int nz,
-                                           int zlim, int x0, int y0, int z0, unsigned int &tri, unsigned int &occ) {
+                                           int zlim, int x0, int y0, int z0, bool look, unsigned int &tri,
+                                           unsigned int &occ) {
     const unsigned int full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const typename Vox<VT>::T *p = vol + lin3(nx, ny, x0, y0, z0);
@@ -637,12 +658,12 @@ __device__ __forceinline__ void count_rows(uint2 *row, const unsigned char *ntri
     tri = occ = 0;
     if (inside) {
         if constexpr (VT == MCG_VOXEL_SHORT2) {
-            if (!brick_mixed<true>(p, sy, sz, 0, 0, 0)) return;
+            if (look && !brick_mixed<true>(p, sy, sz, 0, 0, 0)) return;
         }
         load_rows<VT, true>(row, p, sy, sz, 0, 0, 0, en, ed, neg_any, pos_any);
     } else {
         if constexpr (VT == MCG_VOXEL_SHORT2) {
-            if (!brick_mixed<false>(p, sy, sz, nx - x0, ny - y0, nz - z0)) return;
+            if (look && !brick_mixed<false>(p, sy, sz, nx - x0, ny - y0, nz - z0)) return;
         }
         load_rows<VT, false>(row, p, sy, sz, nx - x0, ny - y0, nz - z0, en, ed, neg_any, pos_any);
     }
@@ -691,6 +712,7 @@ __global__ void __launch_bounds__(RW_THREADS, 3) mc_count_rows_kernel(RowsParams
     // there are any: 18 -> 10 us for 57 x 352 x 138 voxels, a brick a warp)
     const unsigned int warps = gridDim.x * RW_WARPS;
     unsigned int drawn = blockIdx.x * RW_WARPS + warp;
+    bool look = p.look;
     for (;;) {
         const long long b0 = (long long)__shfl_sync(0xffffffffu, drawn, 0) * p.draw;
         if (b0 >= p.nbricks) break;
@@ -704,13 +726,14 @@ __global__ void __launch_bounds__(RW_THREADS, 3) mc_count_rows_kernel(RowsParams
                 const VolDesc &d = p.vols[v];
                 const BrickPos bp = brick_pos((unsigned int)(b - vc.base), d.nbx, d.nby);
                 count_rows<VT>(S.row[warp], S.ntri, static_cast<const T *>(d.data), d.nx, d.ny, d.nz, d.nz - 1, bp.x0,
-                               bp.y0, bp.z0, tri, occ);
+                               bp.y0, bp.z0, look, tri, occ);
             } else {
                 const unsigned int q = (unsigned int)b / (unsigned int)p.nbx, z = q / (unsigned int)p.nby;
                 count_rows<VT>(S.row[warp], S.ntri, static_cast<const T *>(p.vol), p.nx, p.ny, p.nz, p.zlim,
                                (int)((unsigned int)b - q * (unsigned int)p.nbx) * BX,
-                               (int)(q - z * (unsigned int)p.nby) * BY, (int)z * BZ + p.zbase, tri, occ);
+                               (int)(q - z * (unsigned int)p.nby) * BY, (int)z * BZ + p.zbase, look, tri, occ);
             }
+            look = tri == 0;  // one with triangles is not often followed by one on one side
             if (lane == 0) {
                 p.brick_tris[b] = tri;
                 if (tri) {
@@ -965,9 +988,9 @@ constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROW
 // vertices a brick, MODE 2 -> MODE 0 in us: 52 54 -> 69, 145 71 -> 80, 243 87 ->
 // 90, 340 105 -> 100, 485 127 -> 112.  Where only the device knows the counts
 // (one call for both phases, a graph) the MODE 0 launch takes such bricks as MODE
-// 2 does: 192^3, 52 a brick, 44 -> 39 us.  So does a batch's: twelve of 96^3 92 ->
-// 84 us (73 without records, their room being a second tile stage; 729 instead of
-// 585 for 64 volumes of surfaces).  With the records' 26 KB float2 tiles leave
+// 2 does: 192^3, 52 a brick, 44 -> 39 us.  So does a batch's: twelve of 96^3 8 us
+// less (4 us more than without records, whose room is a second tile stage's: 729
+// instead of 585 us for 64 volumes of surfaces).  With the records' 26 KB float2 tiles leave
 // room for three CTAs per SM instead of four, so records pay where the host knows
 // that bricks are as full as a surface makes them, and without normals only where
 // there are few (one call for both phases by vertex: 256^3 84 us, with both
@@ -2715,6 +2738,7 @@ void launch_count_rows(RowsParams p, int sms, cudaStream_t s) {
     const long long grid = std::min<long long>((long long)sms * occ, (p.nbricks + RW_WARPS - 1) / RW_WARPS);
     // four bricks a draw where every warp still gets several draws
     p.draw = p.nbricks >= grid * RW_WARPS * 16 ? 4 : 1;
+    p.look = p.nbricks > grid * RW_WARPS;
     if (BATCH) mc_count_rows_kernel<VT, BATCH><<<(unsigned int)grid, RW_THREADS, 0, s>>>(p);
     else launch_pdl(mc_count_rows_kernel<VT, BATCH>, (unsigned int)grid, RW_THREADS, 0, s, p);
 }
