@@ -1174,7 +1174,8 @@ static mcg_status integrate_backward_impl(mcg_context *ctx, const void *vol0, in
     if (n >= most * 4 * BW_THREADS)
         integrate_backward_kernel<4><<<(unsigned int)most, BW_THREADS, poses, s>>>(p);
     else
-        integrate_backward_kernel<1><<<(unsigned int)std::min(most, (n + BW_THREADS - 1) / BW_THREADS), BW_THREADS, poses, s>>>(p);
+        integrate_backward_kernel<1>
+            <<<(unsigned int)std::min(most, (n + BW_THREADS - 1) / BW_THREADS), BW_THREADS, poses, s>>>(p);
     e = cudaGetLastError();
     return e == cudaSuccess ? MCG_OK : mcg_cuda_fail(ctx, e);
 }

@@ -75,7 +75,8 @@ constexpr int GTILE = TX * TY * TZ;
 // tile stages and minimum resident CTAs per SM of the single-volume generate
 // launch.  One stage measured faster than two at 4 CTAs/SM (a brick's work
 // hides most of its next tile's load, and the smaller footprint lets the next
-// launch's count CTAs start beside the drained ones); 5 CTAs/SM spill.
+// launch's count CTAs start beside the drained ones); 5 CTAs/SM spill.  Float2
+// launches with records hold three: their tiles and the records fill an SM.
 #ifndef MCG_GEN_STAGES
 #define MCG_GEN_STAGES 1
 #endif
@@ -1026,9 +1027,11 @@ struct GenSmem {
             float nrm[SHARED ? SH_RECS * 3 : 1];
         };
     };
-    unsigned int cubes[SHARED ? SH_CUBES + 1 : 1];  // occupied cubes in order: cube | case << 11 | soup vertices before it << 19, and all << 19
+    // occupied cubes in order: cube | case << 11 | soup vertices before it << 19, and all << 19
+    unsigned int cubes[SHARED ? SH_CUBES + 1 : 1];
     uint2 slot[SHARED ? SH_SLOTS : 1];  // the edges of a slot that are used (bits 0-31 of 33), its first record
-    unsigned int occp[(BY + 2) * (BZ + 2)];  // occupied cubes of cube row (cy, cz) at (cz + 1) * (BY + 2) + cy + 1, zero around
+    // occupied cubes of cube row (cy, cz) at (cz + 1) * (BY + 2) + cy + 1, zero around
+    unsigned int occp[(BY + 2) * (BZ + 2)];
     unsigned int elut[12];            // edge -> slot step | x step << 16
     unsigned int wtot[2][WARPS];
     unsigned short rowcube[CUBE_ROWS + 1];  // occupied cubes before each cube row, and all
@@ -1622,7 +1625,8 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             const int s = S.used[slots - 1], row = s / 5, kind = s - 5 * row;
             const uint2 sl = S.slot[s];
             const int lz = row / (BY + 1), ly = row - (BY + 1) * lz;
-            const int j = r - (int)sl.y, x = j < __popc(sl.x) ? select_bit(sl.x, (unsigned int)j) : 32, dx = kind < 2, dy = kind == 2 || kind == 3, dz = kind == 4;
+            const int j = r - (int)sl.y, x = j < __popc(sl.x) ? select_bit(sl.x, (unsigned int)j) : 32;
+            const int dx = kind < 2, dy = kind == 2 || kind == 3, dz = kind == 4;
             const bool down = kind == 1 || kind == 3;
             const int t = tidx(x + TXO, ly + TYO, lz + TZO);
             const float lo = V::f(tile[t]), hi = V::f(tile[t + dx + dy * TX + dz * (TX * TY)]);
@@ -1681,7 +1685,8 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             // the shared-memory and store pipe; with a word a thread (an entry of
             // the map, a word of the record and a store for each) this was a
             // quarter of the launch.
-            auto copy = [&](unsigned int *out, const unsigned int *from, auto words, unsigned int stride, unsigned int first) {
+            auto copy = [&](unsigned int *out, const unsigned int *from, auto words, unsigned int stride,
+                            unsigned int first) {
                 constexpr int W = decltype(words)::value;
                 unsigned int *dst = out + g0 * W;
                 const int n = (int)nP * W, lead = (int)((reinterpret_cast<uintptr_t>(dst) >> 2) & 3u);
@@ -1711,7 +1716,8 @@ __device__ __forceinline__ bool generate_shared(Smem &S, const typename Vox<VT>:
             const std::integral_constant<int, 3> three;
             if (o.soup) copy(reinterpret_cast<unsigned int *>(o.soup), S.rec, seven, 7, 0);
             if (o.normals)
-                copy(reinterpret_cast<unsigned int *>(o.normals), reinterpret_cast<const unsigned int *>(S.nrm), three, 3, 0);
+                copy(reinterpret_cast<unsigned int *>(o.normals), reinterpret_cast<const unsigned int *>(S.nrm), three,
+                     3, 0);
             if (o.vi2vox) copy(reinterpret_cast<unsigned int *>(o.vi2vox), S.rec, three, 7, 3);
             w0 += SH_VERTS;
             if (w0 < nT || zb < BZ) __syncthreads();  // the next part's map, the next layers' slots and records
@@ -1781,7 +1787,8 @@ __device__ __forceinline__ void backward_brick(Smem &S, const typename Vox<VT>::
 }
 
 template <int VT, bool TMA, int MODE>
-__global__ void __launch_bounds__(THREADS, GEN_MINB) mc_generate_kernel(const __grid_constant__ CUtensorMap map, GenParams p) {
+__global__ void __launch_bounds__(THREADS, GEN_MINB)
+    mc_generate_kernel(const __grid_constant__ CUtensorMap map, GenParams p) {
     using V = Vox<VT>;
     using T = typename V::T;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -3317,7 +3324,7 @@ __global__ void mc_batch_reset_kernel(MeshTotals *totals, unsigned long long *__
 namespace mcg {
 namespace {
 
-// Device table layout: [VolDesc x nvol][pad to 64][classify maps x nvol][generate maps x nvol]
+// Device table layout: [VolDesc x nvol][pad to 64][generate maps x nvol]
 size_t btab_desc_bytes(int nvol) { return ((sizeof(VolDesc) * (size_t)nvol + 63) / 64) * 64; }
 size_t btab_bytes(int nvol) { return btab_desc_bytes(nvol) + sizeof(CUtensorMap) * (size_t)nvol; }
 
@@ -3451,7 +3458,7 @@ MeshTotals *batch_host(mcg_context *ctx) {
 }
 
 template <int VT>
-void launch_classify_multi(mcg_context *ctx, int nvol, long long nbricks, cudaStream_t s) {
+void launch_count_multi(mcg_context *ctx, int nvol, long long nbricks, cudaStream_t s) {
     RowsParams p = {};
     p.vols = reinterpret_cast<const VolDesc *>(ctx->d_btab);
     p.nvol = nvol;
@@ -3532,8 +3539,8 @@ cudaError_t launch_batch_count(mcg_context *ctx, int32_t vtype, int32_t nvol, lo
     if (rg < 1) rg = 1;
     if (rg > 4LL * ctx->num_sms) rg = 4LL * ctx->num_sms;
     mc_batch_reset_kernel<<<(unsigned int)rg, 256, 0, s>>>(ctx->d_totals, ctx->d_vol_sums, nvol, ctx->brick_occ, cw);
-    if (vtype == MCG_VOXEL_SHORT2) launch_classify_multi<MCG_VOXEL_SHORT2>(ctx, nvol, nbricks, s);
-    else launch_classify_multi<MCG_VOXEL_FLOAT2>(ctx, nvol, nbricks, s);
+    if (vtype == MCG_VOXEL_SHORT2) launch_count_multi<MCG_VOXEL_SHORT2>(ctx, nvol, nbricks, s);
+    else launch_count_multi<MCG_VOXEL_FLOAT2>(ctx, nvol, nbricks, s);
     MeshTotals *host = batch_host(ctx);
     const ScanBatch bt{reinterpret_cast<const VolDesc *>(ctx->d_btab), nvol, ctx->d_vol_sums,
                        reinterpret_cast<BatchBrick *>(ctx->batch_list), host ? ctx->h_vol_sums_dev : nullptr};

@@ -554,7 +554,8 @@ mcg_status prepare(mcg_context *ctx, int64_t xy, int nz, int64_t size) {
         !ensure(&ctx->rd_dir, &ctx->rd_dir_cap, 3 * (size_t)nz + 1) || !ensure(&ctx->rd_err, &ctx->rd_err_cap, 1) ||
         !ensure(&ctx->rd_sum, &ctx->rd_sum_cap, chunks * sizeof(Sum)) ||
         !ensure(&ctx->rd_first, &ctx->rd_first_cap, chunks) ||
-        !ensure(&ctx->rd_parts, &ctx->rd_parts_cap, (size_t)((xy - 1) / RD_PART) * nz) || !ensure(&ctx->rd_entry, &ctx->rd_entry_cap, chunks))
+        !ensure(&ctx->rd_parts, &ctx->rd_parts_cap, (size_t)((xy - 1) / RD_PART) * nz) ||
+        !ensure(&ctx->rd_entry, &ctx->rd_entry_cap, chunks))
         return mcg_cuda_fail(ctx, cudaErrorMemoryAllocation);
     ctx->rd_dir_n = nz;
     return MCG_OK;
