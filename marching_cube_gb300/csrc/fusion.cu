@@ -691,21 +691,21 @@ __device__ __forceinline__ void backward_voxel(const IntegBwParams &p, const flo
         // the segment forward, its observations and (F, W) before each kept
         float sF[BW_SEG], sW[BW_SEG];
         Obs ob[BW_SEG];
-        unsigned int seen = 0;
+        int seen = 0;
         float cF = ckF[sg], cW = ckW[sg];
         for (int f = f0; f < f1; ++f) {
             Obs o;
             if (!bw_observe(p, s_pose + 12 * f, f, px, py, pz, o)) continue;
-            seen |= 1u << (f - f0);
-            sF[f - f0] = cF;
-            sW[f - f0] = cW;
-            ob[f - f0] = o;
+            o.pix += f * ((long long)p.w * p.h);
+            sF[seen] = cF;
+            sW[seen] = cW;
+            ob[seen++] = o;
             fuse_core(p.is_dynamic, o.s, o.w0, cF, cW, cF, cW);
         }
-        // (a warp's lanes on the same frame: its arrays are interleaved lane by
-        // lane, and its pixels lie together)
+        // (a warp's lanes at the same place of their arrays, which are interleaved
+        // lane by lane)
         for (int k = f1 - f0 - 1; k >= 0; --k) {
-            if (!((seen >> k) & 1u)) continue;
+            if (k >= seen) continue;
             const Obs o = ob[k];
             const float Fp = sF[k], Wp = sW[k];
             float wv = o.w0, mult = 1.0f, d = 0.0f;
@@ -728,7 +728,7 @@ __device__ __forceinline__ void backward_voxel(const IntegBwParams &p, const flo
                 gw0 = gw * mult;
             }
             const float gz = gs * o.dsdz - gw0 * o.w0 / o.z;
-            atomicAdd(p.grad_depth + (f0 + k) * (long long)p.w * p.h + o.pix, gz * o.c);
+            atomicAdd(p.grad_depth + o.pix, gz * o.c);
             gF = gFp;
             gW = gWp;
         }
@@ -740,12 +740,13 @@ __device__ __forceinline__ void backward_voxel(const IntegBwParams &p, const flo
 // ROUNDS voxels a thread at a time and works them out BW_THREADS together.
 // Bound: the work on those voxels (an observation is two divisions and a
 // gather).  256^3 and ten 320x240 frames, gradients at the mesh's voxels: one
-// thread a voxel and three observations a frame 526 us, this 96; at every voxel
-// 3.1 and 1.7 ms.  With each lane at its own next frame in the sweep back these
-// took 94 us and 2.8 ms, and 128^3 with 40 frames 7.5 ms where one thread a
-// voxel takes 1.7 and this 1.3.  Four rounds where they leave a CTA for
-// every place, else one: 64^3 with 40 frames 379 us with four, 201 with one (240
-// with a thread a voxel); 256^3 at the mesh's voxels 96 and 126.
+// thread a voxel and three observations a frame 526 us, this 83; at every voxel
+// 3.1 and 1.6 ms.  With observations kept by frame and each lane going back over
+// its own these took 94 us and 2.8 ms, and 128^3 with 40 frames 7.5 ms where one
+// thread a voxel takes 1.7 and this 1.3; with all lanes on the same frame 97 us
+// and 1.7 ms.  Four rounds where they leave a CTA for every place, else one: 64^3
+// with 40 frames 379 us with four, 199 with one (240 with a thread a voxel); 256^3
+// at the mesh's voxels 96 and 126.
 constexpr int BW_THREADS = 128;
 
 template <int ROUNDS>
