@@ -989,21 +989,25 @@ constexpr int SH_VERTS = 1599, SH_RECS = 640, SH_CUBES = 768, SH_SLOTS = 5 * ROW
 // vertices a brick, MODE 2 -> MODE 0 in us: 52 54 -> 69, 145 71 -> 80, 243 87 ->
 // 90, 340 105 -> 100, 485 127 -> 112.  Where only the device knows the counts
 // (one call for both phases, a graph) the MODE 0 launch takes such bricks as MODE
-// 2 does: 192^3, 52 a brick, 44 -> 39 us.  So does a batch's: twelve of 96^3 8 us
+// 2 does: 192^3, 52 a brick, 44 -> 39 us; float2, 145 a brick, 64 -> 61 (53 with
+// MODE 2's fourth CTA).  So does a batch's: twelve of 96^3 8 us
 // less (4 us more than without records, whose room is a second tile stage's: 729
-// instead of 585 us for 64 volumes of surfaces).  With the records' 26 KB float2 tiles leave
-// room for three CTAs per SM instead of four, so records pay where the host knows
-// that bricks are as full as a surface makes them, and without normals only where
-// there are few (one call for both phases by vertex: 256^3 84 us, with both
-// launches made and the counts choosing 88).  Soup vertices a brick as above:
-// without normals 1119 (128^3, 202 bricks) 28.7 -> 23.3, 968 (501 bricks) 28.6 ->
-// 22.5, 915 (1211) 34.8 -> 34.8, 867 (4245) 75 -> 73, 832 (17703) 266 -> 279; with
-// them 34.6 -> 27.0, 34.9 -> 26.2, 42.3 -> 39.2, 94 -> 86, 337 -> 319.  Noise in
-// 256^3 with them: 145 72 -> 95, 485 119 -> 127, 729 154 -> 152, 972 190 -> 179,
-// 1216 222 -> 209, 1458 254 -> 263, 4847 807 -> 882.
-__host__ __device__ inline bool records_pay(int voxel_type, long long verts, long long bricks, bool normals) {
-    if (voxel_type == MCG_VOXEL_SHORT2) return verts >= 256 * bricks;
-    return verts >= 800 * bricks && verts <= 1300 * bricks && (normals || bricks <= 2048);
+// instead of 585 us for 64 volumes of surfaces).
+__host__ __device__ inline bool few_vertices(long long verts, long long bricks) { return verts < 256 * bricks; }
+
+// The same where the host has read the counts.  With the records' 26 KB float2
+// tiles leave room for three CTAs per SM instead of four, so records pay where
+// bricks are as full as a surface makes them, and without normals only where there
+// are few.  Float2, MODE 2 -> MODE 0 in us with normals / without: spheres, 683
+// soup vertices a brick (131 x 129 x 133) 75 -> 58 / 64 -> 52, 766 (128^3) 60 -> 53
+// / 53 -> 48, 755 (256^3) 105 -> 94 / 91 -> 85, 758 (320^3, 2515 bricks) 136 -> 131
+// / 120 -> 120, 753 (512^3) 327 -> 322 / 298 -> 304; a fused 256^3, 916, 101 -> 109 / 90
+// -> 98, 385 x 257 x 321, 924, 133 -> 126 / 118 -> 117; noise in 192^3, 145 75 -> 85
+// / 67 -> 77, 484 99 -> 101 / 84 -> 90, 727 116 -> 114 / 97 -> 100, 967 131 -> 126 /
+// 109 -> 109, 1451 162 -> 167 / 130 -> 144, 4833 413 -> 440 / 313 -> 343.
+inline bool records_pay(int voxel_type, long long verts, long long bricks, bool normals) {
+    if (voxel_type == MCG_VOXEL_SHORT2) return !few_vertices(verts, bricks);
+    return verts >= 640 * bricks && verts <= 1300 * bricks && (normals || bricks <= 2048);
 }
 
 // SHARED false: the adjoint's and MODE 2's, which go soup vertex by soup vertex
@@ -1048,7 +1052,7 @@ struct GenSmem {
     unsigned int pipe_b;        // refill and its soup offset; pipe_b ~0u = none
     unsigned int wsum[2][2];
     unsigned int nocc, total;
-    int direct;  // MODE 0: vertex by vertex all the same, records do not pay
+    int direct;  // MODE 0: vertex by vertex all the same (few_vertices)
     int abort;
 };
 
@@ -1812,8 +1816,7 @@ __global__ void __launch_bounds__(THREADS, GEN_MINB)
     __syncthreads();
     pdl_wait();  // the scan's list, offsets and totals
     const unsigned int nactive = p.totals->active_bricks;
-    if (MODE == 0 && tid == 0)
-        S.direct = VT == MCG_VOXEL_SHORT2 && !records_pay(VT, 3 * (long long)p.totals->triangles, nactive, true);
+    if (MODE == 0 && tid == 0) S.direct = few_vertices(3 * (long long)p.totals->triangles, nactive);
     unsigned int *ticket = &p.totals->gen_ticket;
     // stage st <- brick b (soup offset v): thread 0 records the brick, its
     // offset and origin for the CTA and starts the tile load
@@ -2594,7 +2597,7 @@ __global__ void __launch_bounds__(THREADS, 4)
     };
     if (tid == 0) {
         S.abort = 0;
-        S.direct = VT == MCG_VOXEL_SHORT2 && !records_pay(VT, 3 * (long long)totals->triangles, nactive, true);
+        S.direct = VT == MCG_VOXEL_SHORT2 && few_vertices(3 * (long long)totals->triangles, nactive);
         mbar_init(&S.bars[0], 1);
         fence_barrier_init();
         S.svol = -1;
@@ -2795,13 +2798,13 @@ void launch_generate_t(const CUtensorMap &map, const GenParams &p, const Geometr
     else mc_generate_kernel<VT, TMA, MODE><<<(int)grid, THREADS, smem, s>>>(map, p);
 }
 
-// known: the totals of the count phase, where the host has read them.  Else a
-// short2 launch decides by itself, and float2 soup is worked out vertex by vertex.
+// known: the totals of the count phase, where the host has read them.  Else the
+// launch with records looks at them itself.
 template <int VT, bool TMA>
 void launch_generate_forward(const CUtensorMap &map, const GenParams &p, const Geometry &g, int sms, cudaStream_t s,
                              const MeshTotals *known) {
-    const bool records = known ? records_pay(VT, 3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr)
-                               : VT == MCG_VOXEL_SHORT2;
+    const bool records =
+        !known || records_pay(VT, 3 * (long long)known->triangles, known->active_bricks, p.normals != nullptr);
     if (records) launch_generate_t<VT, TMA, 0>(map, p, g, sms, s);
     else launch_generate_t<VT, TMA, 2>(map, p, g, sms, s);
 }
