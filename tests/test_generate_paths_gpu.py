@@ -14,7 +14,7 @@ from mc_util import assert_same_mesh, gpu_extract
 
 pytestmark = pytest.mark.gpu
 
-# share of negative voxels -> about 48500 times that many soup vertices a brick: the rule's ends are 800 and 1300
+# share of negative voxels -> about 48500 times that many soup vertices a brick: the rules' ends are 256, 640 and 1300
 SHARES = [0.0, 0.001, 0.01, 0.015, 0.0165, 0.02, 0.025, 0.0268, 0.03, 0.05, 0.1, 0.5]
 
 
